@@ -12,6 +12,18 @@ struct AttnParams {
   int causal;
 };
 
+// fp32 GEMM on the tensor cores (three bf16 parts per operand); strides in elements: A(m,k), B(k,n), C(m,n), O(m,n) and two
+// batch dimensions each.  Sets *handled = 1 when it took the call.
+struct F32Gemm {
+  const void *a, *b, *c;
+  void* o;
+  int64_t M, N, K, b0, b1;
+  int64_t a_b0, a_b1, a_m, a_k, b_b0, b_b1, b_k, b_n, c_b0, c_b1, c_m, c_n, o_b0, o_b1, o_m, o_n;
+  int dt_c, has_c;
+  float alpha, beta;
+};
+int gemm_f32_split(const F32Gemm& g, int* handled);
+
 int matmul_f32_dispatch(const kd_matmul_cfg* cfg, const kd_tensor* a, const kd_tensor* b, const kd_tensor* c,
                         const kd_tensor* out);
 // Tensor-core GEMM; sets *handled = 1 when it took the call (bf16 operands in a supported layout).

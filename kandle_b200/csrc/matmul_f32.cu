@@ -1,7 +1,7 @@
 // Key `matmul`: general strided batched GEMM with fp32 accumulation on the CUDA cores.
 //
-// This is the exact-fp32 path (tcgen05 has no fp32 input format; tf32 would break the fp32
-// parity bound), and the fallback for operand layouts the tensor-core path does not take.  It
+// fp32 operands with K contiguous go to the tensor cores in three bf16 parts (gemm_f32_split.cu); this is the path for
+// every other layout, for short K, and for mixed types.  It
 // accepts everything MatmulDispatchResult can describe
 // (packages/core/src/dispatch/matmulOps.ts:32-125): transpose flags, 4-D element strides with
 // broadcast batch dims, alpha/beta/C -- a superset of the reference shader, which only honours
@@ -147,6 +147,13 @@ int matmul_f32_dispatch(const kd_matmul_cfg* cfg, const kd_tensor* a, const kd_t
     KD_TRY(tensor_ptr(c, &pc));
   }
   if (p.M == 0 || p.N == 0 || p.b0 * p.b1 == 0) return KD_OK;
+  if (p.dt_a == KD_F32 && p.dt_b == KD_F32 && p.dt_o == KD_F32) {
+    const F32Gemm g{pa, pb, pc, po, p.M, p.N, p.K, p.b0, p.b1, p.a_b0, p.a_b1, p.a_m, p.a_k, p.b_b0, p.b_b1, p.b_k, p.b_n,
+                    p.c_b0, p.c_b1, p.c_m, p.c_n, p.o_b0, p.o_b1, p.o_m, p.o_n, p.dt_c, p.has_c, p.alpha, p.beta};
+    int handled = 0;
+    KD_TRY(gemm_f32_split(g, &handled));
+    if (handled) return KD_OK;
+  }
   const int64_t gx = (p.N + BN - 1) / BN, gy = (p.M + BM - 1) / BM, gz = p.b0 * p.b1;
   KD_REQUIRE(gy <= 65535 && gz <= 65535, "matmul: grid too large (M tiles %lld, batch %lld)", (long long)gy, (long long)gz);
   dim3 grid((unsigned)gx, (unsigned)gy, (unsigned)gz);

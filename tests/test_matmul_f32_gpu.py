@@ -1,0 +1,68 @@
+"""fp32 matmul on the tensor cores (gemm_f32_split.cu) against float64: edges of its 128 x 64/128 x 64 tiles, K split over
+a cluster, batches, alpha / beta / C, and numbers outside the range of the split."""
+import numpy as np
+import pytest
+
+from kandle_b200 import core
+from kandle_b200.core import Tensor
+
+pytestmark = pytest.mark.gpu
+
+
+def _bound(a, b):
+    """Every product and partial sum rounds at 2^-24 of at most sum |a||b|: four roundings' worth for the dropped terms
+    (2^-26 each), the sums inside a k-block and the sums over k-blocks, which grow slower than their number."""
+    return 4 * 2.0 ** -24 * (np.abs(a).astype(np.float64) @ np.abs(b).astype(np.float64).T)
+
+
+def _rand(shape, seed):
+    return np.random.default_rng(seed).standard_normal(shape).astype(np.float32)
+
+
+# one row to several tiles, N and K beside multiples of 64 and 128, K of one block, split tiles (few tiles, deep K)
+@pytest.mark.parametrize("m,n,k", [(1, 1, 64), (1, 130, 68), (127, 64, 64), (128, 128, 128), (129, 65, 132), (300, 257, 100), (64, 1024, 1024),
+                                   (130, 192, 196), (512, 1024, 320), (97, 3072, 1024), (128, 300, 4096), (260, 20000, 72)])
+def test_matmul_f32_tiles(backend, m, n, k):
+    a, b = _rand((m, k), 1), _rand((n, k), 2)
+    got = core.matmul(Tensor(a), Tensor(b), transposeB=True).dataAsync()
+    err = np.abs(got - a.astype(np.float64) @ b.astype(np.float64).T)
+    assert (err <= _bound(a, b)).all(), (err / _bound(a, b)).max()
+
+
+def test_matmul_f32_batches_views_and_scalars(backend):
+    a, b, c = _rand((2, 3, 70, 136), 3), _rand((3, 90, 136), 4), _rand((90,), 5)
+    # rows of a wider buffer, a broadcast batch, C broadcast over rows
+    wide = Tensor(np.concatenate([a, a], axis=-1))
+    view = wide.slice(":, :, :, 136:272")
+    got = core.matmul(view, Tensor(b), transposeB=True, alpha=0.5).dataAsync()
+    ref = 0.5 * (a.astype(np.float64) @ b.astype(np.float64).transpose(0, 2, 1))
+    assert np.abs(got - ref).max() <= 1e-6 * np.abs(ref).max() * 2
+    got = core.linear(Tensor(a[0, 0]), Tensor(b[0]), Tensor(c)).dataAsync()
+    ref = a[0, 0].astype(np.float64) @ b[0].astype(np.float64).T + c
+    assert np.abs(got - ref).max() <= 1e-6 * np.abs(ref).max() * 2
+
+
+@pytest.mark.parametrize("m,n,k", [(130, 70, 128), (130, 300, 1024)])
+@pytest.mark.parametrize("value", [np.inf, -np.inf, np.nan, 3e38, -3.4e38, 0.0])
+def test_matmul_f32_values_without_a_split(backend, m, n, k, value):
+    a, b = _rand((m, k), 6), _rand((n, k), 7)
+    a[3, 5] = value
+    b[n - 1, k - 1] = value
+    got = core.matmul(Tensor(a), Tensor(b), transposeB=True).dataAsync()
+    with np.errstate(all="ignore"):
+        exact = a.astype(np.float64) @ b.astype(np.float64).T
+        ref = exact.astype(np.float32)
+    assert np.array_equal(np.isnan(got), np.isnan(ref))
+    assert np.array_equal(got[np.isinf(ref)], ref[np.isinf(ref)])
+    ok = np.isfinite(ref)
+    ok[3, n - 1] = False      # two huge terms: whether their sum overflows on the way depends on its order
+    a[~np.isfinite(a)], b[~np.isfinite(b)] = 0, 0
+    assert (np.abs(got[ok] - exact[ok]) <= 16 * _bound(a, b)[ok]).all()       # (plain fused multiply-adds: more roundings)
+
+
+@pytest.mark.parametrize("scale", [1e-31, 1e-36, 1e-40])
+def test_matmul_f32_tiny_operand(backend, scale):
+    a, b = _rand((70, 256), 8) * np.float32(scale), _rand((130, 256), 9) * np.float32(1e20)
+    got = core.matmul(Tensor(a), Tensor(b), transposeB=True).dataAsync()
+    exact = a.astype(np.float64) @ b.astype(np.float64).T
+    assert (np.abs(got - exact) <= 16 * _bound(a, b)).all()
