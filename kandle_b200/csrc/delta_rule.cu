@@ -24,6 +24,8 @@
 // A CTA is eight consumer warps (one or more heads) and eight helper warps.  The helpers prepare the
 // next block of tokens (convolution, silu, unit norms, decays, step sizes) in shared memory while the
 // consumers walk through the current one.
+// That form needs a head for every SM: one sequence of 8192 tokens and 16 heads took 5.67 ms, 64 CTAs walking 1300 cycles
+// a token.  Calls with few heads take delta_prepare_kernel and recurrence_kernel instead (recurrence.cuh): 1.55 ms.
 // Bound: fp32 pipe in prefill (3.25 dim vdim multiply-adds per head and token), HBM in decode
 // (the state is read and written once per token: 8 dim vdim bytes per head and sequence).
 #include "common.cuh"
@@ -477,6 +479,190 @@ delta_rule_kernel(const T* __restrict__ proj, const T* __restrict__ hist, int64_
   if (active) state_store<LPC>(s, srow, p.dv_pad);
 }
 
+// One warp: the record of four tokens of a head, and their value columns.
+template <typename T, int LPC>
+__global__ void __launch_bounds__(128)
+delta_prepare_kernel(const T* __restrict__ proj, const T* __restrict__ hist, int64_t hist_b, int64_t hist_ld, DeltaParams p, RecStream r) {
+  constexpr bool FAST = sizeof(T) == 2;
+  constexpr int DK = 16 * LPC;                 // padded key channels
+  constexpr int CH = DK > 128 ? DK / 128 : 1;  // passes over the key channels
+  constexpr int REC = rec_floats(true, DK);
+  pdl_wait();
+  pdl_trigger();
+  const int lane = threadIdx.x & 31;
+  const int64_t item = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+  if (item >= (int64_t)r.units * r.groups) return;
+  // (heads side by side: neighbouring warps read neighbouring columns)
+  const unsigned row_of = (unsigned)item / p.H;
+  const int h = (int)((unsigned)item - row_of * p.H), b = (int)(row_of / r.groups), grp = (int)(row_of - b * r.groups), unit = b * p.H + h;
+  const int t = r.t0 + grp * 4;
+  const int hk = h / (p.H / p.Hk);
+  const T* seq = proj + (int64_t)b * p.S * p.ld;
+  const T* hb = hist + (int64_t)b * hist_b;
+  const int kc = p.Hk * p.dim;             // history channels: q, k, v side by side
+  const ConvSource<T> cq{seq + p.q_col + hk * p.dim, hb + hk * p.dim, p.ld, hist_ld, p.conv_q + (int64_t)hk * p.dim * p.taps, p.taps, t, p.S, p.dim, p.vec_q != 0};
+  const ConvSource<T> ck{seq + p.k_col + hk * p.dim, hb + kc + hk * p.dim, p.ld, hist_ld, p.conv_k + (int64_t)hk * p.dim * p.taps, p.taps, t, p.S, p.dim, p.vec_q != 0};
+  const int at = h * p.vdim;
+  const ConvSource<T> cv{seq + p.v_col + at, hb + 2 * kc + at, p.ld, hist_ld, p.conv_v + (int64_t)at * p.taps, p.taps, t, p.S,
+                         p.vdim, p.vec_v != 0};
+  const int c0 = lane * 4;
+  Raw4<T> raw[7];
+  float g[CH][4][4];
+  const float* a = p.a + ((int64_t)b * p.S + t) * p.ld_a + (p.head_decay ? h : h * p.dim);
+  float ah[4] = {0.f, 0.f, 0.f, 0.f};
+  if (p.head_decay) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) ah[q] = a[(t + q < p.S ? q : 0) * p.ld_a];
+  } else
+#pragma unroll
+  for (int i = 0; i < CH; ++i) {
+    const int c = i * 128 + c0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const float* ar = a + (t + q < p.S ? q : 0) * p.ld_a;
+      if (p.vec_a) {
+        const float4 f = *reinterpret_cast<const float4*>(ar + (c < p.dim ? c : 0));
+        g[i][q][0] = f.x; g[i][q][1] = f.y; g[i][q][2] = f.z; g[i][q][3] = f.w;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) g[i][q][e] = c + e < p.dim ? ar[c + e] : 0.f;
+      }
+    }
+  }
+  if (CH == 1 && ck.vec) conv_fetch<T>(ck, c0, raw);
+  // decays
+  const float rate = p.neg_rate[h];
+  float least = 1.f;
+  if (p.head_decay) {
+    const float bias = __ldg(p.dt_bias + h);
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      ah[q] = t + q < p.S ? dr_decay<FAST>(rate, ah[q] + bias) : 1.f;
+      least = fminf(least, ah[q]);
+#pragma unroll
+      for (int i = 0; i < CH; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) g[i][q][e] = i * 128 + c0 + e < p.dim ? ah[q] : 1.f;
+    }
+  } else
+#pragma unroll
+  for (int i = 0; i < CH; ++i) {
+    const int c = i * 128 + c0;
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const bool in = c + e < p.dim;
+      const float bias = in ? __ldg(p.dt_bias + h * p.dim + c + e) : 0.f;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        g[i][q][e] = in && t + q < p.S ? dr_decay<FAST>(rate, g[i][q][e] + bias) : 1.f;
+        least = fminf(least, g[i][q][e]);
+      }
+    }
+  }
+  bool flagged = __any_sync(0xffffffffu, least < REC_SMALL_DECAY);
+  // P: running products of the decays (flagged groups: one, the decays go beside the record)
+  float* rec = r.rec + ((int64_t)unit * r.groups + grp) * REC;
+  if (flagged) {
+    float* direct = r.direct + ((int64_t)unit * r.groups + grp) * 4 * DK;
+#pragma unroll
+    for (int i = 0; i < CH; ++i) {
+      const int c = i * 128 + c0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        if (c < DK) *reinterpret_cast<float4*>(direct + q * DK + c) = make_float4(g[i][q][0], g[i][q][1], g[i][q][2], g[i][q][3]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) g[i][q][e] = 1.f;
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < CH; ++i) {
+    const int c = i * 128 + c0;
+#pragma unroll
+    for (int q = 1; q < 4; ++q)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) g[i][q][e] *= g[i][q - 1][e];
+    if (c < DK) *reinterpret_cast<float4*>(rec + 12 * DK + c) = make_float4(g[i][3][0], g[i][3][1], g[i][3][2], g[i][3][3]);
+  }
+  float y[CH][4][4], kr[CH][4][4], kw[CH][4][4], inv[4];
+  // k: read side k P, write side k / P
+  if (CH == 1 && ck.vec) {
+    conv_finish<T, FAST>(ck, c0, raw, y[0]);
+    conv_fetch<T>(cq, c0, raw);
+  } else {
+    for (int i = 0; i < CH; ++i) conv_slow<T, FAST>(ck, i * 128 + c0, y[i]);
+  }
+  unit_scale<false, CH>(y, 1.0f, inv);
+#pragma unroll
+  for (int i = 0; i < CH; ++i) {
+    const int c = i * 128 + c0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float kk = y[i][q][e] * inv[q];
+        kr[i][q][e] = kk * g[i][q][e];
+        kw[i][q][e] = kk / g[i][q][e];
+      }
+      if (c < DK) {
+        *reinterpret_cast<float4*>(rec + q * DK + c) = make_float4(kr[i][q][0], kr[i][q][1], kr[i][q][2], kr[i][q][3]);
+        *reinterpret_cast<float4*>(rec + (8 + q) * DK + c) = make_float4(kw[i][q][0], kw[i][q][1], kw[i][q][2], kw[i][q][3]);
+      }
+    }
+  }
+  if (CH == 1 && cq.vec) {
+    conv_finish<T, FAST>(cq, c0, raw, y[0]);
+  } else {
+    for (int i = 0; i < CH; ++i) conv_slow<T, FAST>(cq, i * 128 + c0, y[i]);
+  }
+  if (cv.vec) conv_fetch<T>(cv, c0, raw);
+  unit_scale<false, CH>(y, p.q_scale, inv);
+#pragma unroll
+  for (int i = 0; i < CH; ++i) {
+    const int c = i * 128 + c0;
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e) y[i][q][e] *= inv[q] * g[i][q][e];
+      if (c < DK) *reinterpret_cast<float4*>(rec + (4 + q) * DK + c) = make_float4(y[i][q][0], y[i][q][1], y[i][q][2], y[i][q][3]);
+    }
+  }
+  float m[16];
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      float x = 0.f;
+#pragma unroll
+      for (int i = 0; i < CH; ++i)
+#pragma unroll
+        for (int e = 0; e < 4; ++e) x = s <= a ? fmaf(y[i][a][e], kw[i][s][e], x) : fmaf(kr[i][s][e], kw[i][a][e], x);
+      m[a * 4 + s] = x;
+    }
+  lanes_sum<16, 32>(lane, m);
+  if ((lane & 1) == 0) rec[REC + REC_M + (lane >> 1)] = m[0];
+  if (lane < 4) {
+    rec[REC + REC_BETA + lane] = t + lane < p.S ? rec_sigmoid<FAST>(rec_f<T>(seq[(int64_t)(t + lane) * p.ld + p.b_col + h])) : 0.f;
+    rec[REC + REC_FLAG + lane] = flagged ? 1.f : 0.f;
+  }
+#pragma unroll 1
+  for (int c = c0; c < r.tiles * r.dvc; c += 128) {
+    if (cv.vec) {
+      if (c != c0) conv_fetch<T>(cv, c, raw);
+      conv_finish<T, FAST>(cv, c, raw, y[0]);
+    } else {
+      conv_slow<T, FAST>(cv, c, y[0]);
+    }
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const int tile = (c + e) / r.dvc, at_tile = (c + e) - tile * r.dvc;
+      if (tile < r.tiles)
+        *reinterpret_cast<float4*>(r.v + ((((int64_t)unit * r.tiles + tile) * r.groups + grp) * r.dvc + at_tile) * 4) =
+            make_float4(y[0][0][e], y[0][1][e], y[0][2][e], y[0][3][e]);
+    }
+  }
+}
+
 // ----------------------------------------------------------------------------- one token (decode)
 // The state of a head is read and written once: HBM-bound.  256 threads per (head, 64 value columns): warp r
 // holds rows r RPW .. of the state, a lane four columns of every second one; all loads are issued before anything
@@ -701,7 +887,22 @@ static int f32_vec(const kd_tensor* t, int64_t n, const char* what, const float*
 }
 
 template <typename T, int LPC>
+static int launch_delta_few(const void* proj, const void* hist, int64_t hist_b, int64_t hist_ld, const DeltaParams& p, int* handled) {
+  RecStream r{};
+  r.units = p.B * p.H; r.H = p.H; r.S = p.S; r.vdim = p.vdim; r.dk_pad = p.dk_pad; r.dv_pad = p.dv_pad;
+  r.state = p.state; r.o = p.o;
+  return launch_recurrence<16 * LPC, true>(r, handled, [&](const RecStream& part) {
+    const int64_t items = (int64_t)part.units * part.groups;
+    KD_CUDA_CHECK(launch_ex(delta_prepare_kernel<T, LPC>, dim3((unsigned)((items + 3) / 4)), dim3(128), 0, (const T*)proj, (const T*)hist, hist_b, hist_ld, p, part));
+    return after_launch("delta_prepare_kernel");
+  });
+}
+
+template <typename T, int LPC>
 static int launch_delta(const void* proj, const void* hist, int64_t hist_b, int64_t hist_ld, DeltaParams p) {
+  int handled = 0;
+  KD_TRY((launch_delta_few<T, LPC>(proj, hist, hist_b, hist_ld, p, &handled)));
+  if (handled) return KD_OK;
   constexpr int CPW = 8 * (32 / LPC), DK = 16 * LPC;
   const int units = p.B * p.H;
   p.wpu = (p.vdim + CPW - 1) / CPW;

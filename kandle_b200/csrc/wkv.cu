@@ -12,6 +12,8 @@
 // its read and its write.  Two tokens' outputs are summed over a group's lanes together.
 // Eight consumer warps (208 registers a thread) and four helper warps (88); a helper warp prepares four tokens of a
 // head in as many lanes as the head has quads of channels, so a warp takes two groups of tokens of a 64-channel head.
+// Calls with few heads take wkv_prepare_kernel and recurrence_kernel (recurrence.cuh): 8192 tokens of 32 heads in 1.23 ms,
+// 3.49 ms with one CTA a head.
 // Bound: fp32 pipe in prefill (2.25 dim^2 multiply-adds per head and token), HBM in decode (the state is read and
 // written once per token: 8 dim^2 bytes per head and sequence).
 #include "common.cuh"
@@ -413,6 +415,172 @@ wkv_kernel(const T* __restrict__ r_in, const T* __restrict__ k_in, const T* __re
   if (active) state_store<LPC>(s, srow, p.dv_pad);
 }
 
+// The records of GPI groups of four tokens a warp, and their value columns.
+template <typename T, int LPC>
+__global__ void __launch_bounds__(128)
+wkv_prepare_kernel(const T* __restrict__ r_in, const T* __restrict__ k_in, const T* __restrict__ v_in, WkvParams p, RecStream r) {
+  constexpr bool FAST = sizeof(T) == 2;
+  constexpr int DK = 16 * LPC;                 // padded key channels
+  constexpr int CH = DK > 128 ? DK / 128 : 1;  // passes over the key channels
+  constexpr int LANES = DK < 128 ? DK / 4 : 32, GPI = 32 / LANES;      // lanes that share a token's channels
+  constexpr int REC = rec_floats(false, DK);
+  pdl_wait();
+  pdl_trigger();
+  const int lane = threadIdx.x & 31;
+  const int sub = lane / LANES, c0 = (lane % LANES) * 4;
+  const unsigned mine = LANES == 32 ? 0xffffffffu : ((1u << LANES) - 1u) << (sub * LANES);
+  // (heads side by side: neighbouring warps read neighbouring columns)
+  const int64_t items = (int64_t)r.units * r.groups, own = ((int64_t)blockIdx.x * 4 + (threadIdx.x >> 5)) * GPI + sub, item = own < items ? own : items - 1;
+  const unsigned row_of = (unsigned)item / p.H;
+  const int h = (int)((unsigned)item - row_of * p.H), b = (int)(row_of / r.groups), grp = (int)(row_of - b * r.groups), unit = b * p.H + h;
+  const int t = r.t0 + grp * 4;
+  // (all lanes take part in the sums; those of a group past the end or without a group store nothing)
+  const bool stores = own < (int64_t)r.units * r.groups;
+  const int64_t row = (int64_t)b * p.S + (t < p.S ? t : 0);
+  const int left = p.S - t;                // tokens of this group that exist
+  const int at = h * p.dim, nv = p.dim;
+  float g[CH][4][4], bonus[4] = {0.f, 0.f, 0.f, 0.f}, least = 1.f;
+  Raw4<T> rraw[CH][4], kraw[CH][4], v0[4];
+  if (p.vec) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int64_t rq = row + (q < left ? q : 0);
+#pragma unroll
+      for (int i = 0; i < CH; ++i) {
+        const int cc = at + (i * 128 + c0 < p.dim ? i * 128 + c0 : 0);
+        const float4 f = *reinterpret_cast<const float4*>(p.logits + rq * p.ld_w + cc);
+        g[i][q][0] = f.x; g[i][q][1] = f.y; g[i][q][2] = f.z; g[i][q][3] = f.w;
+        rraw[i][q].load(r_in + rq * p.ld + cc);
+        kraw[i][q].load(k_in + rq * p.ld + cc);
+      }
+      v0[q].load(v_in + rq * p.ld + at + (c0 < nv ? c0 : 0));
+    }
+  } else {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int64_t rq = row + (q < left ? q : 0);
+#pragma unroll
+      for (int i = 0; i < CH; ++i) {
+        float rr[4], kk[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const int c = i * 128 + c0 + e, cc = at + (c < p.dim ? c : 0);
+          g[i][q][e] = p.logits[rq * p.ld_w + cc];
+          rr[e] = rec_f<T>(r_in[rq * p.ld + cc]);
+          kk[e] = rec_f<T>(k_in[rq * p.ld + cc]);
+        }
+        rraw[i][q].set(rr);
+        kraw[i][q].set(kk);
+      }
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < CH; ++i) {
+    const int c = i * 128 + c0;
+    float w0[4], u[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      w0[e] = c + e < p.dim ? __ldg(p.w0 + at + c + e) : 0.f;
+      u[e] = c + e < p.dim ? __ldg(p.u + at + c + e) : 0.f;
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float rr[4], kk[4];
+      rraw[i][q].get(rr);
+      kraw[i][q].get(kk);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const bool use = c + e < p.dim && q < left;
+        g[i][q][e] = use ? double_exp_decay<FAST>(g[i][q][e] + w0[e]) : 1.f;
+        least = fminf(least, g[i][q][e]);
+        bonus[q] = use ? fmaf(rr[e] * u[e], kk[e], bonus[q]) : bonus[q];
+      }
+    }
+  }
+  const bool flagged = (__ballot_sync(0xffffffffu, least < REC_SMALL_DECAY) & mine) != 0;
+  // P: product of the decays of the tokens before (flagged groups: one, the decays go beside the record)
+  float* rec = r.rec + ((int64_t)unit * r.groups + grp) * REC;
+  float rd[CH][4][4], kw[CH][4][4];
+#pragma unroll
+  for (int i = 0; i < CH; ++i) {
+    const int c = i * 128 + c0;
+    if (flagged && stores) {
+      float* direct = r.direct + ((int64_t)unit * r.groups + grp) * 4 * DK;
+#pragma unroll
+      for (int q = 0; q < 4; ++q) *reinterpret_cast<float4*>(direct + q * DK + c) = make_float4(g[i][q][0], g[i][q][1], g[i][q][2], g[i][q][3]);
+    }
+    float P[4] = {1.f, 1.f, 1.f, 1.f};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      float rr[4], kk[4];
+      rraw[i][q].get(rr);
+      kraw[i][q].get(kk);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const bool use = c + e < p.dim && q < left;
+        rd[i][q][e] = use ? rr[e] * P[e] : 0.f;
+        P[e] *= flagged ? 1.f : g[i][q][e];
+        kw[i][q][e] = !use ? 0.f : FAST ? kk[e] * rcpf(P[e]) : kk[e] / P[e];
+      }
+      if (stores) {
+        *reinterpret_cast<float4*>(rec + q * DK + c) = make_float4(rd[i][q][0], rd[i][q][1], rd[i][q][2], rd[i][q][3]);
+        *reinterpret_cast<float4*>(rec + (4 + q) * DK + c) = make_float4(kw[i][q][0], kw[i][q][1], kw[i][q][2], kw[i][q][3]);
+      }
+    }
+    if (stores) *reinterpret_cast<float4*>(rec + 8 * DK + c) = make_float4(P[0], P[1], P[2], P[3]);
+  }
+  float m[16];
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int s = 0; s < 4; ++s) {
+      float x = 0.f;
+      if (s < a) {
+#pragma unroll
+        for (int i = 0; i < CH; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) x = fmaf(rd[i][a][e], kw[i][s][e], x);
+      }
+      m[a * 4 + s] = s == a ? bonus[a] : x;      // (every lane's share; the bonus is summed with the rest)
+    }
+  lanes_sum<16, LANES>(lane % LANES, m);
+  if (stores) {
+    constexpr int OWN = 16 / LANES > 1 ? 16 / LANES : 1, REP = LANES > 16 ? LANES / 16 : 1;
+    if (lane % REP == 0) {
+#pragma unroll
+      for (int i = 0; i < OWN; ++i) rec[REC + REC_M + (lane % LANES) * OWN / REP + i] = m[i];
+    }
+    if (c0 == 0) *reinterpret_cast<float4*>(rec + REC + REC_FLAG) = flagged ? make_float4(1.f, 1.f, 1.f, 1.f) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 1
+    for (int c = c0; c < r.tiles * r.dvc; c += LANES * 4) {
+      float y[4][4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) y[q][e] = 0.f;
+        if (q < left) {
+          const T* src = v_in + (row + q) * p.ld + at + c;
+          if (p.vec) {
+            if (c < nv) {
+              if (c != c0) v0[q].load(src);
+              v0[q].get(y[q]);
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < 4; ++e) if (c + e < nv) y[q][e] = rec_f<T>(src[e]);
+          }
+        }
+      }
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int tile = (c + e) / r.dvc, at_tile = (c + e) - tile * r.dvc;
+        if (tile < r.tiles)
+          *reinterpret_cast<float4*>(r.v + ((((int64_t)unit * r.tiles + tile) * r.groups + grp) * r.dvc + at_tile) * 4) = make_float4(y[0][e], y[1][e], y[2][e], y[3][e]);
+      }
+    }
+  }
+}
+
 // One token: 256 threads per (head, 64 columns), as delta_step_kernel; the state is read and written once.
 template <typename T, int RPW>
 __global__ void __launch_bounds__(256, RPW <= 16 ? 3 : 2)
@@ -476,7 +644,23 @@ wkv_step_kernel(const T* __restrict__ r_in, const T* __restrict__ k_in, const T*
 }
 
 template <typename T, int LPC>
+static int launch_wkv_few(const void* r, const void* k, const void* v, const WkvParams& p, int* handled) {
+  RecStream rs{};
+  rs.units = p.B * p.H; rs.H = p.H; rs.S = p.S; rs.vdim = p.dim; rs.dk_pad = p.dk_pad; rs.dv_pad = p.dv_pad;
+  rs.state = p.state; rs.o = p.o;
+  return launch_recurrence<16 * LPC, false>(rs, handled, [&](const RecStream& part) {
+    constexpr int PER = 4 * (LPC < 8 ? 8 / LPC : 1);
+    const int64_t items = (int64_t)part.units * part.groups;
+    KD_CUDA_CHECK(launch_ex(wkv_prepare_kernel<T, LPC>, dim3((unsigned)((items + PER - 1) / PER)), dim3(128), 0, (const T*)r, (const T*)k, (const T*)v, p, part));
+    return after_launch("wkv_prepare_kernel");
+  });
+}
+
+template <typename T, int LPC>
 static int launch_wkv(const void* r, const void* k, const void* v, WkvParams p) {
+  int handled = 0;
+  KD_TRY((launch_wkv_few<T, LPC>(r, k, v, p, &handled)));
+  if (handled) return KD_OK;
   constexpr int CPW = 8 * (32 / LPC), DK = 16 * LPC, TB = wkv_tokens<LPC>();
   const int units = p.B * p.H;
   p.wpu = (p.dim + CPW - 1) / CPW;

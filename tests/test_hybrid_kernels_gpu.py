@@ -306,6 +306,14 @@ def test_delta_rule_decays_from_one_to_zero(backend, dtype, a_mean, a_sd, rate_s
         _delta_case(1, 50, 3, 3, 40, 24, 4, dtype, cuts, a_mean, a_sd, rate_sd)
 
 
+@pytest.mark.parametrize("S", [31, 32, 33, 39])
+def test_delta_rule_few_heads_take_records(backend, S):
+    """The line between the forms, ragged last groups, and a prompt of several portions of records."""
+    _delta_case(3, S, 5, 5, 128, 72, 4, "bfloat16", [S])
+    if S == 39:
+        _delta_case(1, 1551, 16, 16, 128, 128, 4, "bfloat16", [1551], a_mean=-3.0)
+
+
 def test_delta_rule_many_heads_share_a_block(backend):
     """Enough heads for several per block, in a batch: bf16 and fp32 agree with the plain form for every one."""
     _delta_case(20, 19, 16, 8, 64, 64, 4, "bfloat16", [18, 1])

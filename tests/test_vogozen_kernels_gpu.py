@@ -367,6 +367,14 @@ def test_wkv_decays_from_one_to_zero(backend, dtype, w_mean, w_sd):
         _wkv_case(1, 50, 3, 40, dtype, cuts, w_mean, w_sd)
 
 
+@pytest.mark.parametrize("S", [31, 32, 33, 39])
+def test_wkv_few_heads_take_records(backend, S):
+    """The line between the forms, ragged last groups, and a prompt of several portions of records."""
+    _wkv_case(3, S, 5, 64, "bfloat16", [S])
+    if S == 39:
+        _wkv_case(1, 1901, 32, 64, "bfloat16", [1901], w_mean=-3.0)
+
+
 def test_wkv_many_heads_share_a_block(backend):
     _wkv_case(20, 19, 16, 64, "bfloat16", [18, 1])
     _wkv_case(12, 19, 32, 32, "float32", [2, 17])
