@@ -152,7 +152,7 @@ class CudaTensorHandle:
         h = self
         tmp = None
         if not (self.isContiguous()):
-            tmp = CudaBackend.instance().createTensorHandle(self.shape, self.dtype)
+            tmp = CudaBackend.instance().createTensorHandle(self.shape, self.dtype, clear=False)
             lib.call("kd_copy", ctypes.byref(tmp.c()), ctypes.byref(self.c()))
             h = tmp
         code, esz, npdt = DTYPES[self.dtype]
@@ -217,8 +217,10 @@ class CudaBackend:
         return cls._instance
 
     # createTensorHandle(shape, dtype, data?)  |  createTensorHandle({shape,dtype,storage?,...})
+    # New storage is zero-initialised.  clear=False leaves out that pass over memory for outputs of which the operator
+    # that follows writes every element.
     def createTensorHandle(self, shape, dtype: str | None = None, data=None, *, storage: CudaStorage | None = None,
-                           strides=None, offset: int = 0, memoryFormat: str = "contiguous") -> CudaTensorHandle:
+                           strides=None, offset: int = 0, memoryFormat: str = "contiguous", clear: bool = True) -> CudaTensorHandle:
         if isinstance(shape, dict):
             o = shape
             return self.createTensorHandle(o["shape"], o["dtype"], o.get("data"), storage=o.get("storage"),
@@ -232,7 +234,7 @@ class CudaBackend:
             return CudaTensorHandle(storage, shape, dtype, strides, offset, memoryFormat)
         code, esz, npdt = DTYPES[dtype]
         n = int(math.prod(shape))
-        st = CudaStorage(max(n * esz, 1), zero=(data is None))  # new storage is zero-initialised
+        st = CudaStorage(max(n * esz, 1), zero=clear and data is None)
         h = CudaTensorHandle(st, shape, dtype, None, 0, memoryFormat)
         if data is not None:
             self.upload(h, data)

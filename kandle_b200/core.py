@@ -275,6 +275,12 @@ def _new(shape, dtype) -> CudaTensorHandle:
     return _backend().createTensorHandle(tuple(shape), dtype)
 
 
+def _output(shape, dtype) -> CudaTensorHandle:
+    """Storage for an operator that writes every element of it: not cleared first (the clears were 3.9 of 33.5 ms of a
+    Whisper encoder pass over 64 clips, and half of the launches of the fp32 modules)."""
+    return _backend().createTensorHandle(tuple(shape), dtype, clear=False)
+
+
 def _binary(key: str, a: Tensor, b, scalars=None) -> Tensor:
     if not isinstance(b, Tensor):
         if key == "mul":
@@ -286,7 +292,7 @@ def _binary(key: str, a: Tensor, b, scalars=None) -> Tensor:
         else:
             b = Tensor(np.asarray(b, dtype=np.float32).reshape(()), dtype="float32")
     shape = _broadcast_shape(a.shape, b.shape)
-    out = _new(shape, _promote(a.dtype, b.dtype))
+    out = _output(shape, _promote(a.dtype, b.dtype))
     _kernel(key)(TensorIterator([a._handle, b._handle], [out], scalars or {}))
     return Tensor(_handle=out)
 
@@ -294,7 +300,7 @@ def _binary(key: str, a: Tensor, b, scalars=None) -> Tensor:
 def _unary(key: str, a: Tensor, scalars=None) -> Tensor:
     # neg / abs keep an integer dtype; the transcendental keys promote integers to float32
     keep = a.dtype in _FLOAT_RANK or key in ("neg", "abs")
-    out = _new(a.shape, a.dtype if keep else "float32")
+    out = _output(a.shape, a.dtype if keep else "float32")
     _kernel(key)(TensorIterator([a._handle], [out], scalars or {}))
     return Tensor(_handle=out)
 
@@ -353,7 +359,7 @@ def sigmoid(a: Tensor) -> Tensor:
 
 
 def _copy_like(key: str, a: Tensor, dtype: str) -> Tensor:
-    out = _new(a.shape, dtype)
+    out = _output(a.shape, dtype)
     _kernel(key)(TensorIterator([a._handle], [out]))
     return Tensor(_handle=out)
 
@@ -377,19 +383,19 @@ def copy_(dst: Tensor, src: Tensor) -> Tensor:
 
 
 def zeros(shape, dtype: str = "float32") -> Tensor:
-    out = _new(shape, dtype)
+    out = _output(shape, dtype)
     _kernel("zeros")(TensorIterator([], [out]))
     return Tensor(_handle=out)
 
 
 def ones(shape, dtype: str = "float32") -> Tensor:
-    out = _new(shape, dtype)
+    out = _output(shape, dtype)
     _kernel("ones")(TensorIterator([], [out]))
     return Tensor(_handle=out)
 
 
 def full(shape, value: float, dtype: str = "float32") -> Tensor:
-    out = _new(shape, dtype)
+    out = _output(shape, dtype)
     _kernel("full")(TensorIterator([], [out], {"fillValue": value}))
     return Tensor(_handle=out)
 
@@ -406,7 +412,7 @@ def manualSeed(seed: int) -> None:
 
 def randn(shape, dtype: str = "float32") -> Tensor:
     """N(0,1) numbers from the device generator (packages/core/src/generated/internal/randn.ts)."""
-    out = _new(shape, dtype)
+    out = _output(shape, dtype)
     _kernel("randn")(TensorIterator([], [out]))
     return Tensor(_handle=out)
 
@@ -415,7 +421,7 @@ def arange(start, end=None, step=1, dtype: str = "int32") -> Tensor:
     if end is None:
         start, end = 0, start
     n = max(0, int(math.ceil((end - start) / step)))
-    out = _new((n,), dtype)
+    out = _output((n,), dtype)
     _kernel("arange")(TensorIterator([], [out], {"start": start, "step": step}))
     return Tensor(_handle=out)
 
@@ -430,7 +436,7 @@ def cat(tensors: Sequence[Tensor], dim: int = 0) -> Tensor:
     dtype = first.dtype
     for t in tensors[1:]:
         dtype = _promote(dtype, t.dtype)
-    out = Tensor(_handle=_new(shape, dtype))
+    out = Tensor(_handle=_output(shape, dtype))
     pos = 0
     for t in tensors:
         items = [slice(None)] * first.ndim
@@ -468,7 +474,7 @@ def argmax(a: Tensor, dim: int = -1, keepdim: bool = False) -> Tensor:
         moved = a.permute(dims)
         src = moved
     out_shape = src.shape[:-1]
-    out = _new(out_shape, "int64")
+    out = (_output if src.shape[-1] else _new)(out_shape, "int64")
     _kernel("argmax")(TensorIterator([src._handle], [out], {"dim": dim}))
     if moved is not None:
         moved.dispose()
@@ -497,7 +503,7 @@ def matmul(a: Tensor, b: Tensor, *, transposeA: bool = False, transposeB: bool =
     if K != K2:
         raise ValueError(f"matmul: inner dimensions do not match ({K} vs {K2}); shapes {a.shape} @ {b.shape}")
     batch = _broadcast_shape(av.shape[:-2], bv.shape[:-2])
-    out = _new(batch + (M, N), _promote(a.dtype, b.dtype))
+    out = (_output if K else _new)(batch + (M, N), _promote(a.dtype, b.dtype))
     variant = "mm" if not batch else "bmm"
     cfg = MatmulDispatchResult(variant, out, M, K, N, batch, transposeA, transposeB, alpha, beta,
                                inputC._handle if inputC is not None else None)
@@ -594,7 +600,7 @@ def scaledDotProductAttention(q: Tensor, k: Tensor, v: Tensor, attnMask: Tensor 
         raise ValueError("isCausal=true cannot be used with attnMask")
     fa = _backend().operators.find("flash_attention")
     if attnMask is None and fa is not None:
-        out = _new(q.shape, q.dtype)
+        out = _output(q.shape, q.dtype)
         fa(q._handle, k._handle, v._handle, out, float(scale), bool(isCausal))
         return Tensor(_handle=out)
     scores = matmul(q, k, transposeB=True, alpha=scale)

@@ -151,7 +151,7 @@ def _alloc_like(x, out):
     from .backend import CudaBackend
     if out is not None:
         return out
-    return CudaBackend.instance().createTensorHandle(x.shape, x.dtype)
+    return CudaBackend.instance().createTensorHandle(x.shape, x.dtype, clear=False)
 
 
 def _rms_norm(inputs, params):
@@ -189,7 +189,7 @@ def _flash_attention(q, k, v, out, scale: float, isCausal: bool) -> None:
 
 def _conv1d(cfg: ConvDispatchResult, inp, weight, bias=None):
     from .backend import CudaBackend
-    out = CudaBackend.instance().createTensorHandle(cfg.outputShape, cfg.dtype)
+    out = CudaBackend.instance().createTensorHandle(cfg.outputShape, cfg.dtype, clear=0 in inp.shape or 0 in weight.shape)
     lib.call("kd_conv1d", _ref(inp), _ref(weight), _ref(bias), int(cfg.stride), int(cfg.padding), _ref(out))
     return out
 

@@ -82,7 +82,7 @@ class WhisperEncoderEngine:
     def _block(self, blk, x: Tensor) -> Tensor:
         B, T, E = x.shape
         H, D = self.H, self.D
-        e = lambda *shape: core.empty(shape, "bfloat16")  # noqa: E731
+        e = lambda *shape: Tensor(_handle=core._output(shape, "bfloat16"))  # noqa: E731
         mha = blk.self_attn
         y = blk.self_attn_layer_norm(x)
         qkv = e(B, T, 3 * E)
@@ -121,9 +121,9 @@ class WhisperEncoderEngine:
             raise ValueError(f"{T} frames exceed the encoder context of {enc.config.nAudioCtx}")
         mt = mel.permute([0, 2, 1])
         mel_t = core.contiguous(mt)                # [B, L, nMels]
-        h1 = core.empty((B, L, E), "bfloat16")
+        h1 = Tensor(_handle=core._output((B, L, E), "bfloat16"))
         lib.call("kd_conv1d_tokens_bf16", _r(mel_t), _r(self.w1), _r(enc.conv1.bias), None, KD_ACT_GELU, 3, 1, 1, _r(h1))
-        x = core.empty((B, T, E), "bfloat16")
+        x = Tensor(_handle=core._output((B, T, E), "bfloat16"))
         pos = self._positions(B, T)
         lib.call("kd_conv1d_tokens_bf16", _r(h1), _r(self.w2), _r(enc.conv2.bias), _r(pos), KD_ACT_GELU, 3, 2, 1, _r(x))
         for t in (mt, mel_t, h1):
