@@ -39,6 +39,23 @@ def test_sdpa_shapes_and_tails(backend, oracle, causal, b, hq, hkv, sq, skv, d):
     close(out.dataAsync(), oracle.sdpa(q, k, v, is_causal=causal))
 
 
+@pytest.mark.parametrize("d", [64, 128])
+@pytest.mark.parametrize("sq, skv", [(16, 16), (31, 31), (32, 64), (65, 65), (97, 128), (160, 96)])
+@pytest.mark.parametrize("heads", [2, 40])
+def test_sdpa_register_tiles(backend, oracle, heads, sq, skv, d):
+    """Edges of the row and key tiles with 16 and with 32 rows a block; infinities among masked values stay out of the sums
+    of rows that see none of their 32-key block."""
+    q, k, v = synth.normal("q", (1, heads, sq, d)), synth.normal("k", (1, heads // 2, skv, d)), synth.normal("v", (1, heads // 2, skv, d))
+    for causal in (False, True):
+        close(core.scaledDotProductAttention(Tensor(q), Tensor(k), Tensor(v), None, 0.0, causal).dataAsync(), oracle.sdpa(q, k, v, is_causal=causal))
+    if min(sq, skv) > 32:
+        v[:, :, 32:] = np.inf
+        got = core.scaledDotProductAttention(Tensor(q), Tensor(k), Tensor(v), None, 0.0, True).dataAsync()
+        v[:, :, 32:] = 0
+        close(got[:, :, :32], oracle.sdpa(q, k, v, is_causal=True)[:, :, :32])
+        assert not np.isfinite(got[:, :, 32:]).any()
+
+
 def test_sdpa_3d_and_strided_inputs(backend, oracle):
     q, k, v = synth.normal("q", (6, 20, 64)), synth.normal("k", (6, 20, 64)), synth.normal("v", (6, 20, 64))
     out = core.scaledDotProductAttention(Tensor(q), Tensor(k), Tensor(v))
