@@ -190,6 +190,33 @@ def test_binary_broadcast_and_alpha(backend, oracle):
         core.add(Tensor(a), Tensor(synth.normal("z", (7,))))
 
 
+@pytest.mark.parametrize("inner", [3, 4, 6, 8, 36])
+@pytest.mark.parametrize("da, db", [("float32", "float32"), ("bfloat16", "float32"), ("float16", "bfloat16")])
+def test_pointwise_orders_and_strides(backend, inner, da, db):
+    """Every way the operands' rows can lie: merged and permuted dimensions, broadcast rows and numbers, offsets that leave
+    the 16-byte grid, mixed types; against numpy element by element."""
+    x, y = Tensor(synth.normal("x", (2, 3, 5, inner + 4)), dtype=da), Tensor(synth.normal("y", (2, 3, 5, inner + 4)), dtype=db)
+    xs, ys = x.dataAsync(), y.dataAsync()
+    out = lambda a, b: core.add(a, b, 0.5)  # noqa: E731
+    rounded = {"float32": lambda r: r, "bfloat16": lib.round_to_bf16, "float16": lambda r: r.astype(np.float16).astype(np.float32)}
+    for off in (0, 1, 4):
+        for order in ([0, 1, 2, 3], [0, 2, 1, 3], [2, 1, 0, 3], [3, 0, 2, 1]):
+            cut = f"..., {off}:{off + inner}"
+            a, b = x.slice(cut).permute(order), y.slice(cut).permute(order)
+            na, nb = (v[..., off:off + inner].transpose(order).astype(np.float32) for v in (xs, ys))
+            for b2, nb2 in ((b, nb), (b.slice([slice(0, 1)] * 3 + [slice(None)]), nb[:1, :1, :1]), (b.slice([slice(None)] * 3 + [slice(0, 1)]), nb[..., :1])):
+                got = out(a, b2)
+                want = rounded[got.dtype](na + np.float32(0.5) * nb2)
+                assert np.abs(got.dataAsync() - want).max() <= (1e-6 if got.dtype == "float32" else 0), (off, order)
+            assert np.array_equal(core.contiguous(a).dataAsync(), na)
+            assert np.array_equal(core.cast(a, db).dataAsync(), rounded[db](na))
+            dst = core.zeros((2, 3, 5, inner + 4), db)
+            core.copy_(dst.slice(cut).permute(order), a)
+            want = np.zeros((2, 3, 5, inner + 4), np.float32)
+            want[..., off:off + inner] = rounded[db](xs[..., off:off + inner].astype(np.float32))
+            assert np.array_equal(dst.dataAsync(), want)
+
+
 def test_views_copy_cat_cast(backend):
     x = synth.normal("x", (2, 3, 4, 6))
     t = Tensor(x)
