@@ -10,6 +10,8 @@
 //               mbarrier complete_tx; loads are plain tiled loads (no cluster multicast).
 //   warp 1      one elected thread issues tcgen05.mma (M=128, N=BLOCK_N, K=16 x4 per stage) into a
 //               TMEM accumulator; tcgen05.commit releases the smem stage / publishes the tile.
+//   Few rows: a cluster of 2 or 4 CTAs shares a tile, each a range of k-blocks; the first adds the others' sums to its own
+//   and has the epilogue (choose_tile).
 //   warps 2-5   epilogue: tcgen05.ld the 128xBLOCK_N fp32 tile (one row per thread), apply the
 //               fused epilogue, convert and store.  Two TMEM accumulators let the epilogue of tile
 //               i overlap the mainloop of tile i+1.
@@ -115,6 +117,7 @@ struct GemmParams {
   // (group_off null) group_rows rows each
   const int* group_off;
   int groups, group_rows;
+  int splits;             // CTAs of a cluster that share a tile, each with a range of k-blocks (then a CTA has one tile)
   float glu_limit;        // epi == 4: clamped GLU, see clamped_glu_f; epi == 5: GELU(gate) * up
 };
 
@@ -168,7 +171,20 @@ __device__ __forceinline__ float tanh_f(float x) {
   return fmaf(-2.0f, r, 1.0f);
 }
 
-template <int BLOCK_N, int STAGES>
+// Barrier of a cluster (every thread of every CTA passes it twice, whatever its role and whether or not a wait gave up).
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ float4 ld_peer_f4(uint32_t addr, uint32_t rank) {
+  uint32_t remote;
+  float4 v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(addr), "r"(rank));
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "r"(remote) : "memory");
+  return v;
+}
+
+// SHARED: the CTAs of a cluster share a tile (an instantiation of its own: the plain one took 0.6 us longer with it inside)
+template <int BLOCK_N, int STAGES, bool SHARED>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, GemmParams p) {
   constexpr int A_BYTES = GEMM_BM * GEMM_BK * 2;
@@ -232,6 +248,9 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     num_m_tiles = group_tile[p.groups];
   }
   const int total_tiles = num_m_tiles * p.num_n_tiles;
+  const int rank = SHARED ? (int)(blockIdx.x % p.splits) : 0, first = SHARED ? (int)(blockIdx.x / p.splits) : (int)blockIdx.x;
+  const int step = SHARED ? (int)(gridDim.x / p.splits) : (int)gridDim.x;
+  const int kb_begin = SHARED ? num_k_blocks * rank / p.splits : 0, kb_end = SHARED ? num_k_blocks * (rank + 1) / p.splits : num_k_blocks;
   // first A row, end of the valid rows and first W row of tile row m_tile
   auto locate = [&](int m_tile, int& row0, int& row_end, int& w_row) {
     if (p.groups == 0) { row0 = m_tile * GEMM_BM; row_end = p.M; w_row = 0; return; }
@@ -250,11 +269,11 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
+      for (int tile = first; ok && tile < total_tiles; tile += step) {
         const int m_tile = tile / p.num_n_tiles, n_tile = tile - m_tile * p.num_n_tiles;
         int row0, row_end, w_row;
         locate(m_tile, row0, row_end, w_row);
-        for (int kb = 0; kb < num_k_blocks; ++kb) {
+        for (int kb = kb_begin; kb < kb_end; ++kb) {
           if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.err, 201)) { ok = false; break; }
           uint8_t* sa = smem + stage * STAGE_BYTES;
           mbar_arrive_expect_tx(&full[stage], STAGE_BYTES);
@@ -271,11 +290,11 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
+      for (int tile = first; ok && tile < total_tiles; tile += step) {
         if (!mbar_wait(&tmem_empty[acc], acc_phase ^ 1, abort_flag, p.err, 202)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BLOCK_N);
-        for (int kb = 0; kb < num_k_blocks; ++kb) {
+        for (int kb = kb_begin; kb < kb_end; ++kb) {
           if (!mbar_wait(&full[stage], phase, abort_flag, p.err, 203)) { ok = false; break; }
           tc_fence_after();
           const uint32_t a_addr = smem_u32(smem + stage * STAGE_BYTES);
@@ -284,7 +303,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
           for (int k = 0; k < GEMM_BK / 16; ++k) {
             const uint64_t adesc = make_smem_desc_sw128(a_addr + k * 32, 16, 1024);
             const uint64_t bdesc = make_smem_desc_sw128(b_addr + k * 32, 16, 1024);
-            umma_ss(d_tmem, adesc, bdesc, IDESC, (kb | k) != 0 ? 1u : 0u);
+            umma_ss(d_tmem, adesc, bdesc, IDESC, ((kb - kb_begin) | k) != 0 ? 1u : 0u);
           }
           umma_commit(&empty[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
@@ -299,19 +318,62 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     const int q = warp & 3;  // TMEM lane quarter this warp may access
     int acc = 0;
     uint32_t acc_phase = 0;
-    for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x) {
+    for (int tile = first; tile < total_tiles; tile += step) {
       const int m_tile = tile / p.num_n_tiles, n_tile = tile - m_tile * p.num_n_tiles;
       int row0, row_end, w_row;
       locate(m_tile, row0, row_end, w_row);
       bool ok = mbar_wait(&tmem_full[acc], acc_phase, abort_flag, p.err, 204);
       ok = __all_sync(0xffffffffu, ok);
-      if (!ok) break;
+      if (!SHARED && !ok) break;
       tc_fence_after();
+      if constexpr (SHARED) {
+        // The others leave their sums in the stages that no copy or product uses any more, rows side by side in pieces of
+        // four columns; the first adds them to its own in tensor memory, in the order of the k ranges.
+        const uint32_t t_own = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BLOCK_N);
+        uint8_t* mine = smem + (q * 32 + lane) * 16;
+        uint32_t x[32];
+        if (ok && rank > 0) {
+#pragma unroll 1
+          for (int c = 0; c < BLOCK_N; c += 32) {
+            tmem_ld_32x32(t_own + c, x);
+            tmem_wait_ld();
+#pragma unroll
+            for (int j = 0; j < 8; ++j) *reinterpret_cast<uint4*>(mine + (c / 4 + j) * (GEMM_BM * 16)) = make_uint4(x[j * 4], x[j * 4 + 1], x[j * 4 + 2], x[j * 4 + 3]);
+          }
+        }
+        __syncwarp();
+        cluster_sync();
+        if (ok && rank == 0) {
+          const uint32_t at = smem_u32(mine);
+#pragma unroll 1
+          for (int c = 0; c < BLOCK_N; c += 32) {
+            tmem_ld_32x32(t_own + c, x);
+            tmem_wait_ld();
+            for (int r = 1; r < p.splits; ++r) {
+              float4 v[8];
+#pragma unroll
+              for (int j = 0; j < 8; ++j) v[j] = ld_peer_f4(at + (c / 4 + j) * (GEMM_BM * 16), (uint32_t)r);
+#pragma unroll
+              for (int j = 0; j < 8; ++j) {
+                x[j * 4] = __float_as_uint(__uint_as_float(x[j * 4]) + v[j].x);
+                x[j * 4 + 1] = __float_as_uint(__uint_as_float(x[j * 4 + 1]) + v[j].y);
+                x[j * 4 + 2] = __float_as_uint(__uint_as_float(x[j * 4 + 2]) + v[j].z);
+                x[j * 4 + 3] = __float_as_uint(__uint_as_float(x[j * 4 + 3]) + v[j].w);
+              }
+            }
+            tmem_st_32x32(t_own + c, x);
+          }
+          tmem_wait_st();
+        }
+        __syncwarp();
+        cluster_sync();      // (the first may still be reading the others' shared memory)
+        if (rank > 0 || !ok) break;
+      }
       const int row = row0 + q * 32 + lane;
       const bool row_ok = row < row_end;
       bool released = false;   // accumulator already handed back inside the branch
       const uint32_t t_row = tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * BLOCK_N);
-      if (BLOCK_N == 256 && p.epi == 3) {
+      if ((BLOCK_N == 256 || (BLOCK_N == 128 && SHARED)) && p.epi == 3) {
         // q/k-norm + RoPE + cache write (see fused.cu for the stand-alone kernel and the reference
         // operators it replaces).  A thread owns one token row; a head is 128 consecutive columns,
         // so the norm and both members of every rotation pair (i, i+64) are thread-local.
@@ -592,6 +654,11 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     }
   }
 
+  if (SHARED && warp < 2) {
+    __syncwarp();
+    cluster_sync();
+    cluster_sync();
+  }
   // teardown: every role falls through to here, also after an aborted wait
   tc_fence_before();
   __syncthreads();
@@ -608,17 +675,60 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams&
   constexpr int SMEM = STAGES * STAGE_BYTES + 1024 + 256;
   static bool configured[64] = {false};   // per device: kd_shutdown + kd_init may move the library to another GPU
   if (!configured[ctx().device & 63]) {
-    KD_CUDA_CHECK(cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<BLOCK_N, STAGES>,
-                                       cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+    KD_CUDA_CHECK(cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<BLOCK_N, STAGES, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+    if (BLOCK_N < 256)
+      KD_CUDA_CHECK(cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<BLOCK_N, STAGES, BLOCK_N < 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
     configured[ctx().device & 63] = true;
   }
   // (grouped: every group may end in a partial tile, and groups without rows have none)
   p.num_m_tiles = (p.M + GEMM_BM - 1) / GEMM_BM + (p.groups ? (p.groups < p.M ? p.groups : p.M) : 0);
   p.num_n_tiles = (p.N + BLOCK_N - 1) / BLOCK_N;
   const int64_t total = (int64_t)p.num_m_tiles * p.num_n_tiles;
+  // (choose_tile shares no 256-wide tile; the epilogue over heads is in this instantiation, or the plain one would grow)
+  if (BLOCK_N < 256 && (p.splits > 1 || p.epi == 3)) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)(total * p.splits));
+    cfg.blockDim = dim3(GEMM_THREADS);
+    cfg.dynamicSmemBytes = SMEM;
+    cfg.stream = ctx().stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)p.splits;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = ctx().pdl ? 2 : 1;
+    KD_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gemm_bf16_tcgen05_kernel<BLOCK_N, STAGES, BLOCK_N < 256>, ta, tb, p));
+    return after_launch("gemm_bf16_tcgen05_kernel");
+  }
+  p.splits = 1;
   const int grid = total < ctx().sm_count ? (int)total : ctx().sm_count;
-  KD_CUDA_CHECK(launch_ex(gemm_bf16_tcgen05_kernel<BLOCK_N, STAGES>, dim3(grid), dim3(GEMM_THREADS), (size_t)SMEM, ta, tb, p));
+  KD_CUDA_CHECK(launch_ex(gemm_bf16_tcgen05_kernel<BLOCK_N, STAGES, false>, dim3(grid), dim3(GEMM_THREADS), (size_t)SMEM, ta, tb, p));
   return after_launch("gemm_bf16_tcgen05_kernel");
+}
+
+// Tile width and number of CTAs that share a tile (p.splits) where 256-wide tiles would leave more than half of the GPU idle;
+// widths from `narrowest` on.  An SM takes a k-block in the time of its copies from L2 (about 83 GB/s: 0.28, 0.38, 0.57 us
+// for 64-, 128- and 256-wide tiles); a shared tile costs two barriers of the cluster and the others' sums.  Measured, one CTA
+// and the chosen number a tile, 97 rows: N = 1024, K = 2048 16.3, 12.4 us; N = 1024, K = 3072 20.6, 14.5; N = 768, K = 3072
+// 18.6, 12.5; N = K = 768 8.4, 10.4 (not shared).  Above two rows of tiles it gave little or nothing (700 rows: 16.5, 18.5).
+static int choose_tile(GemmParams& p, int narrowest) {
+  const int64_t m_tiles = (p.M + GEMM_BM - 1) / GEMM_BM, kbs = (p.K + GEMM_BK - 1) / GEMM_BK, sms = ctx().sm_count;
+  double best = 1e30;
+  int bn = 256;
+  p.splits = 1;
+  for (int w = narrowest; w <= 256; w *= 2) {
+    const int64_t tiles = m_tiles * ((p.N + w - 1) / w);
+    const double block = w == 64 ? 0.28 : w == 128 ? 0.38 : 0.57, wide = w == 64 ? 0.0 : 0.8;
+    for (int s = 1; s <= (w == 256 || m_tiles > 2 ? 1 : 4); s *= 2) {
+      // (a CTA of a shared tile has one tile; clusters of four do not fill every SM)
+      if (s > 1 && (tiles * s > (s == 4 ? sms - sms / 8 : sms) || kbs < 2 * s)) break;
+      const double cost = (double)((tiles * s + sms - 1) / sms) * ((kbs + s - 1) / s) * block + (s > 1 ? 1.5 + 0.75 * s + (s - 1) * wide : 0.0);
+      if (cost < best) { best = cost; bn = w; p.splits = s; }
+    }
+  }
+  return bn;
 }
 
 // out[M, N or N/2] = epilogue(A[M,K] * W[N,K]^T).  Pointers are device pointers; ld* in elements.
@@ -659,17 +769,11 @@ int gemm_bf16_bias_act(const void* A, int64_t lda, const void* W, int64_t ldw, v
   p.err = ctx().error_flag;
   CUtensorMap ta, tb;
   KD_TRY(make_tmap_bf16_2d(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, GEMM_BM, GEMM_BK));
-  // wide tiles, unless they would leave most of the GPU idle (a few rows, or a narrow output)
   const int64_t wide = (int64_t)((M + GEMM_BM - 1) / GEMM_BM) * ((N + 255) / 256);
-  if (epi == 2 || (N >= 256 && wide * 2 > ctx().sm_count)) {
-    KD_TRY(make_tmap_bf16_2d(&tb, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, 256, GEMM_BK));
-    return launch_gemm<256, 4>(ta, tb, p);
-  }
-  if (N > 64 && wide * 4 > ctx().sm_count) {
-    KD_TRY(make_tmap_bf16_2d(&tb, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, 128, GEMM_BK));
-    return launch_gemm<128, 6>(ta, tb, p);
-  }
-  KD_TRY(make_tmap_bf16_2d(&tb, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, 64, GEMM_BK));
+  const int bn = N >= 256 && wide * 2 > ctx().sm_count ? 256 : choose_tile(p, 64);
+  KD_TRY(make_tmap_bf16_2d(&tb, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, bn, GEMM_BK));
+  if (bn == 256) return launch_gemm<256, 4>(ta, tb, p);
+  if (bn == 128) return launch_gemm<128, 6>(ta, tb, p);
   return launch_gemm<64, 8>(ta, tb, p);
 }
 
@@ -715,8 +819,10 @@ int gemm_bf16_qkv_rope(const void* A, int64_t lda, const void* W, int64_t ldw, i
   p.kc_b = kc_b; p.kc_h = kc_h; p.kc_s = kc_s;
   CUtensorMap ta, tb;
   KD_TRY(make_tmap_bf16_2d(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, GEMM_BM, GEMM_BK));
-  KD_TRY(make_tmap_bf16_2d(&tb, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, 256, GEMM_BK));
-  return launch_gemm<256, 4>(ta, tb, p);
+  const int64_t wide = (int64_t)((M + GEMM_BM - 1) / GEMM_BM) * ((N + 255) / 256);
+  const int bn = wide * 2 > ctx().sm_count ? 256 : choose_tile(p, 128);      // (a head of 128 columns lies in one tile)
+  KD_TRY(make_tmap_bf16_2d(&tb, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, bn, GEMM_BK));
+  return bn == 256 ? launch_gemm<256, 4>(ta, tb, p) : launch_gemm<128, 6>(ta, tb, p);
 }
 
 // ----------------------------------------------------------------------------- skinny (decode) GEMM

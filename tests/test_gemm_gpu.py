@@ -42,6 +42,19 @@ def test_linear_bf16_matches_oracle(backend, oracle, m, n, k):
     assert np.abs(got32 - ref).max() <= 1e-4 * np.abs(ref).max()     # fp32 output: accumulation order only
 
 
+@pytest.mark.parametrize("m", [2, 128, 129, 384])
+@pytest.mark.parametrize("n,k", [(64, 192), (200, 520), (1024, 3072), (4096, 1024), (768, 136)])
+def test_linear_bf16_few_rows_share_k(backend, oracle, m, n, k):
+    """One, two and four blocks to a tile, ranges of unequal length, remainders in every dimension."""
+    x, w = lib.round_to_bf16(synth.normal("x", (m, k))), lib.round_to_bf16(synth.normal("w", (n, k), 0.05))
+    ref = oracle.linear(x, w)
+    got = _linear_bf16(x, w, out_dtype="float32")
+    assert np.abs(got - ref).max() <= 1e-4 * np.abs(ref).max()       # accumulation order only
+    assert np.array_equal(got, _linear_bf16(x, w, out_dtype="float32"))
+    r = lib.round_to_bf16(synth.normal("r", (m, n)))
+    bf16_close(_linear_bf16(x, w, r, 1), oracle.add(r, ref))
+
+
 def test_linear_bf16_residual_epilogue(backend, oracle):
     x, w = lib.round_to_bf16(synth.normal("x", (200, 2048))), lib.round_to_bf16(synth.normal("w", (1024, 2048), 0.02))
     r = lib.round_to_bf16(synth.normal("r", (200, 1024)))
