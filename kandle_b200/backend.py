@@ -14,6 +14,7 @@ from __future__ import annotations
 import ctypes
 import itertools
 import math
+import struct
 from typing import Callable, Sequence
 
 import numpy as np
@@ -22,6 +23,11 @@ from . import lib
 from .lib import DTYPES, KandleCudaError, kd_matmul_cfg, kd_tensor
 
 _ids = itertools.count(1)
+
+# A kd_tensor as bytes, written in one step: filling the structure's arrays element by element took most of a call's time.
+_TENSOR = struct.Struct(f"=Qqii{lib.KD_MAX_DIMS}q{lib.KD_MAX_DIMS}q")
+assert _TENSOR.size == ctypes.sizeof(kd_tensor)
+_PAD = [(0,) * (lib.KD_MAX_DIMS - n) for n in range(lib.KD_MAX_DIMS + 1)]
 
 
 def contiguous_strides(shape: Sequence[int]) -> tuple[int, ...]:
@@ -77,24 +83,25 @@ class CudaStorage:
 
 class CudaTensorHandle:
     """ITensorHandle (packages/types/src/tensor.ts:6-55): metadata + a share of a storage.
-    Strides and offset are in elements."""
+    Strides and offset are in elements.  The metadata of a handle never changes; a view is a new handle."""
 
     device = "cuda"
 
     def __init__(self, storage: CudaStorage, shape, dtype: str, strides=None, offset: int = 0,
                  memoryFormat: str = "contiguous"):
         self.storage = storage
-        self.shape = tuple(int(s) for s in shape)
+        self.shape = tuple(map(int, shape))
         if len(self.shape) > lib.KD_MAX_DIMS:
             raise ValueError(f"rank {len(self.shape)} exceeds {lib.KD_MAX_DIMS}")
         if dtype not in DTYPES:
             raise ValueError(f"unsupported dtype {dtype!r}")
         self.dtype = dtype
-        self.strides = tuple(int(s) for s in strides) if strides is not None else contiguous_strides(self.shape)
+        self.strides = tuple(map(int, strides)) if strides is not None else contiguous_strides(self.shape)
         self.offset = int(offset)
         self.memoryFormat = memoryFormat
         self.id = next(_ids)
         self._disposed = False
+        self._c = None
 
     # --- metadata
     @property
@@ -134,15 +141,11 @@ class CudaTensorHandle:
     def c(self) -> kd_tensor:
         if self._disposed or self.storage.isDisposed:
             raise RuntimeError("tensor handle used after dispose()")
-        t = kd_tensor()
-        t.storage = self.storage.handle
-        t.offset = self.offset
-        t.dtype = DTYPES[self.dtype][0]
-        t.ndim = len(self.shape)
-        for i, (s, st) in enumerate(zip(self.shape, self.strides)):
-            t.shape[i] = s
-            t.strides[i] = st
-        return t
+        if self._c is None:
+            shape, strides = self.shape, self.strides
+            self._c = kd_tensor.from_buffer_copy(_TENSOR.pack(self.storage.handle, self.offset, DTYPES[self.dtype][0], len(shape),
+                                                              *shape, *_PAD[len(shape)], *strides, *_PAD[len(strides)]))
+        return self._c
 
     # --- readback
     def dataAsync(self) -> np.ndarray:
@@ -228,7 +231,7 @@ class CudaBackend:
                                            memoryFormat=o.get("memoryFormat", "contiguous"))
         if dtype not in DTYPES:
             raise ValueError(f"unsupported dtype {dtype!r}")
-        shape = tuple(int(s) for s in shape)
+        shape = tuple(map(int, shape))
         if storage is not None:
             storage.incRef()
             return CudaTensorHandle(storage, shape, dtype, strides, offset, memoryFormat)
