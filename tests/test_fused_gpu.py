@@ -161,6 +161,17 @@ def test_swiglu(backend, oracle, partials):
     close_bf16(out.dataAsync(), oracle.mul(oracle.unary("silu", g), u))
 
 
+@pytest.mark.parametrize("rows", [1023, 1024, 1031])
+@pytest.mark.parametrize("n", [8, 264, 1024, 1032, 2560, 2568, 4096])
+@pytest.mark.parametrize("skip", [0, 4])
+def test_add_rmsnorm_of_fp32_rows(backend, oracle, n, rows, skip):
+    """The forms for few rows, for many, and for rows that do not start on 32 bytes."""
+    flat, w = synth.normal("x", (rows * n + skip,)), lib.round_to_bf16(synth.normal("w", (n,), 0.1, 1.0))
+    norm, whole = core.empty((rows, n), "bfloat16"), Tensor(flat)
+    lib.call("kd_add_rmsnorm", _r(whole.slice([slice(skip, None)]).view(rows, n)), None, _r(bf(w)), ctypes.c_float(1e-6), None, _r(norm))
+    close_bf16(norm.dataAsync(), oracle.rms_norm(flat[skip:].reshape(rows, n), w, 1e-6))
+
+
 @pytest.mark.parametrize("rows", [5, 1500])
 @pytest.mark.parametrize("n", [1024, 2560, 64])
 @pytest.mark.parametrize("mode", ["plain", "residual", "partials"])
