@@ -1,3 +1,4 @@
+import gc
 import os
 import sys
 
@@ -24,3 +25,11 @@ def oracle():
     from oracle import oracle as orc
     orc.build()
     return orc
+
+
+@pytest.fixture(autouse=True)
+def _garbage_first(request):
+    """Tests that account device memory start without garbage of earlier ones: an exception's traceback keeps its frames'
+    tensors until the cycle is collected, which may otherwise happen between two readings."""
+    if any(word in request.node.name for word in ("refcount", "alloc")):
+        gc.collect()

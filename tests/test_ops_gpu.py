@@ -146,6 +146,15 @@ def test_layer_norm(backend, oracle, rows, n):
     close(core.layerNorm(Tensor(x), (n,), Tensor(w), Tensor(b), 1e-5).dataAsync(), oracle.layer_norm(x, w, b, 1e-5))
 
 
+@pytest.mark.parametrize("rows, n", [(3, 8), (70, 512), (70, 520), (70, 768), (70, 776), (40, 1032), (40, 2048), (19100, 264), (19100, 768)])
+def test_norms_of_bf16_rows(backend, oracle, rows, n):
+    """Every vector count a lane, and enough rows for several to a warp."""
+    x, w, b = (lib.round_to_bf16(synth.normal(k, s)) for k, s in (("x", (rows, n)), ("w", (n,)), ("b", (n,))))
+    tx, tw, tb = (Tensor(v, dtype="bfloat16") for v in (x, w, b))
+    close(core.layerNorm(tx, (n,), tw, tb, 1e-5).dataAsync(), oracle.layer_norm(x, w, b, 1e-5), 4e-3)
+    close(core.rmsNorm(tx, (n,), tw, 1e-6).dataAsync(), oracle.rms_norm(x, w, 1e-6), 4e-3)
+
+
 @pytest.mark.parametrize("rows,n", [(9, 333), (2, 151936), (64, 77)])
 def test_softmax(backend, oracle, rows, n):
     x = synth.normal("x", (rows, n), 4.0)
