@@ -93,7 +93,9 @@ template <int REGS>
 __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS)); }
 template <int REGS>
 __device__ __forceinline__ void regs_inc() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS)); }
+// Barrier of a cluster.  It wants its warps converged: one lane alone issues the products, rows past the output store nothing.
 __device__ __forceinline__ void cluster_arrive_wait() {
+  __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 __device__ __forceinline__ float4 ld_cluster_f4(uint32_t addr, uint32_t rank) {
