@@ -256,7 +256,8 @@ __global__ void __launch_bounds__(FS_THREADS, 1) gemm_f32_split_kernel(SplitPara
     for (; ok && tile < p.total; tile += step, ++ordinal) {
       uint32_t small = 0xffffffffu;
       for (int kb = 0; kb < num_kb; ++kb) {
-        if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.err, 221)) { ok = false; break; }
+        ok = __all_sync(0xffffffffu, mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.err, 221));
+        if (!ok) break;
         if (kb * FS_BK > k_last) {
 #pragma unroll
           for (int i = 0; i < A_PASSES + B_PASSES; ++i) buf[i] = make_float4(0.f, 0.f, 0.f, 0.f);

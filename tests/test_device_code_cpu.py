@@ -20,3 +20,16 @@ def test_aligned_cluster_barriers_follow_a_reconvergence(name):
     code = _code(os.path.join(CSRC, name))
     for m in re.finditer(r'asm volatile\(\s*"barrier\.cluster\.arrive[^"]*\.aligned', code):
         assert re.search(r"__syncwarp\(\);\s*$", code[:m.start()]), f"{name}: line {code[:m.start()].count(chr(10)) + 1}"
+
+
+@pytest.mark.parametrize("name", ["gemm_f32_split.cu", "recurrence.cuh"])
+def test_whole_warps_give_up_together(name):
+    """A wait that runs out for some lanes only would leave the others at the warp's next full-mask instruction.  Waits of
+    whole warps are combined; the rest belong to one lane (`issue`, the copying warp's `lane == 0`)."""
+    lines = _code(os.path.join(CSRC, name)).split("\n")
+    for i, line in enumerate(lines):
+        if "mbar_wait(" in line and "__all_sync(0xffffffffu" not in line:
+            before = "\n".join(lines[:i])
+            alone = max(before.rfind("auto issue = [&]()"), before.rfind("if (lane == 0) {"))
+            warp_role = max(before.rfind("regs_inc<"), before.rfind("const int j = lane % LPC"))
+            assert alone > warp_role, f"{name}: {line.strip()}"
