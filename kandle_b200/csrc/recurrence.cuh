@@ -248,12 +248,11 @@ recurrence_kernel(RecStream p) {
         sm100::bulk_load(dst + REC_STAGE_GROUPS * REC, v + (int64_t)g * p.dvc * 4, (uint32_t)(n * p.dvc * 16), &full[stage]);
         if (++stage == p.stages) { stage = 0; phase ^= 1; }
       }
-      // A CTA does not end before its copies: the consumers wait for every stage; where they gave up, this does.
-      if (*abort_flag)
-        for (int s = 0; s < p.stages; ++s) {
-          const long long since = clock64();
-          while (!sm100::mbar_try_wait(&full[s], s < stage ? phase : phase ^ 1) && clock64() - since < 1000000) {}
-        }
+      // A CTA does not end before its copies: consumers that give up, now or later, leave the wait for them to this warp.
+      for (int s = 0; s < p.stages; ++s) {
+        const long long since = clock64();
+        while (!sm100::mbar_try_wait(&full[s], s < stage ? phase : phase ^ 1) && clock64() - since < 1000000) {}
+      }
     }
     return;
   }

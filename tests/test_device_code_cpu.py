@@ -33,3 +33,11 @@ def test_whole_warps_give_up_together(name):
             alone = max(before.rfind("auto issue = [&]()"), before.rfind("if (lane == 0) {"))
             warp_role = max(before.rfind("regs_inc<"), before.rfind("const int j = lane % LPC"))
             assert alone > warp_role, f"{name}: {line.strip()}"
+
+
+def test_the_copying_warp_outlives_its_copies():
+    """recurrence_kernel: consumers may give up after the copying warp's last request, so its wait for what is in flight
+    may not hang on the abort flag of that moment."""
+    code = _code(os.path.join(CSRC, "recurrence.cuh"))
+    role = code[code.index("if (warp == consumers) {"):code.index("const int j = lane % LPC")]
+    assert "mbar_try_wait(&full[s]" in role and "abort_flag)\n" not in role[role.rindex("bulk_load"):]
