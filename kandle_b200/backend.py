@@ -83,7 +83,7 @@ class CudaStorage:
 
 class CudaTensorHandle:
     """ITensorHandle (packages/types/src/tensor.ts:6-55): metadata + a share of a storage.
-    Strides and offset are in elements.  The metadata of a handle never changes; a view is a new handle."""
+    Strides and offset are in elements."""
 
     device = "cuda"
 
@@ -101,7 +101,7 @@ class CudaTensorHandle:
         self.memoryFormat = memoryFormat
         self.id = next(_ids)
         self._disposed = False
-        self._c = None
+        self._packed_for = self._packed = None
 
     # --- metadata
     @property
@@ -141,11 +141,13 @@ class CudaTensorHandle:
     def c(self) -> kd_tensor:
         if self._disposed or self.storage.isDisposed:
             raise RuntimeError("tensor handle used after dispose()")
-        if self._c is None:
+        now = (self.storage.handle, self.offset, self.dtype, self.shape, self.strides)
+        if now != self._packed_for:      # the bytes are kept with what they were packed from
             shape, strides = self.shape, self.strides
-            self._c = kd_tensor.from_buffer_copy(_TENSOR.pack(self.storage.handle, self.offset, DTYPES[self.dtype][0], len(shape),
-                                                              *shape, *_PAD[len(shape)], *strides, *_PAD[len(strides)]))
-        return self._c
+            self._packed = _TENSOR.pack(self.storage.handle, self.offset, DTYPES[self.dtype][0], len(shape),
+                                        *shape, *_PAD[len(shape)], *strides, *_PAD[len(strides)])
+            self._packed_for = now
+        return kd_tensor.from_buffer_copy(self._packed)      # the caller's own
 
     # --- readback
     def dataAsync(self) -> np.ndarray:

@@ -112,3 +112,17 @@ def test_select_and_integer_index_raise_like_the_reference():
     with pytest.raises(IndexError):
         t.slice(":, 7, :")
     assert t.slice(":, -5, 1:3").shape == (4, 2)
+
+
+def test_descriptors_belong_to_their_caller():
+    """A descriptor that a caller writes to leaves the handle alone, and one made after the handle's metadata changed
+    shows the change."""
+    import types
+    from kandle_b200.backend import CudaTensorHandle
+    h = CudaTensorHandle(types.SimpleNamespace(handle=7, isDisposed=False, decRef=lambda: None), (2, 3), "float32")
+    t = h.c()
+    t.shape[0], t.offset = 99, 5
+    again = h.c()
+    assert (again.storage, again.offset, again.ndim, list(again.shape[:3]), list(again.strides[:2])) == (7, 0, 2, [2, 3, 0], [3, 1])
+    h.offset, h.shape = 4, (1, 3)
+    assert (h.c().offset, h.c().shape[0], again.offset) == (4, 1, 0)
