@@ -13,7 +13,8 @@
 // Range: a split needs room below it.  Numbers with 2^-100 <= |x| < 2^127, and zero, split exactly.  The converting warps
 // keep the least of a tile; a tile with a smaller one, and 32 rows with a sum that is not finite (so does every infinity,
 // NaN or number from 2^127 on end), are computed again by their accumulating warps with plain fused multiply-adds, in the
-// order of matmul_f32_kernel.
+// order of matmul_f32_kernel.  One such number costs its tiles, a denormal weight every row of tiles: 512 x 3072 x 1024 takes
+// 38 us, 356 with every tile computed again (matmul_f32_kernel 367); 2048 x 4096 x 4096 463 and 5512 us (7510).
 //
 // Structure (one persistent CTA per SM, 640 threads):
 //   warps 0-7    global fp32 -> registers (next k-block in flight) -> three bf16 planes per operand in shared memory,
@@ -22,8 +23,8 @@
 //   warp 16      one thread issues 24 tcgen05.mma per k-block (M=128, N=BN, K=16).
 //                (warps 17-19 idle: registers move between groups of four warps)
 // Bound: the split, about 35 instructions per 4 numbers of either operand and 1.8 us per 128 x 128 x 64 block, against
-// 0.8 us of MMA.  2048 x 4096 x 4096 takes 465 us = 148 TFLOP/s; matmul_f32_kernel reaches about 5.  A tile too few SMs
-// share K: a cluster of 2 or 4 CTAs, each a range of k-blocks, adds its sums up through shared memory in a fixed order.
+// 0.8 us of MMA.  2048 x 4096 x 4096 takes 463 us = 148 TFLOP/s; matmul_f32_kernel reaches about 9.  Where the tiles
+// are too few for the SMs, K is shared: a cluster of 2 or 4 CTAs, each a range of k-blocks, adds its sums up through shared memory in a fixed order.
 #include "common.cuh"
 #include "kernels.cuh"
 #include "sm100.cuh"
@@ -342,36 +343,53 @@ __global__ void __launch_bounds__(FS_THREADS, 1) gemm_f32_split_kernel(SplitPara
       if (lane == 0) mbar_arrive(&rest_empty[parity]);
       int z, m0, n0;
       locate(tile, z, m0, n0);
-      const int row = m0 + q * 32 + lane, col0 = n0 + half * COLS;
-      // Where a row's sums go: the output, or (split tiles) this CTA's share in the stages that no copy or product uses any
-      // more; 16-byte pieces of a row trade places so that eight rows meet eight bank groups.
-      uint8_t* mine = smem + (q * 32 + lane) * (BN * 4);
-      auto put = [&](int c, const float (&v)[4]) {
-        if (p.splits > 1) *reinterpret_cast<float4*>(mine + ((((half * COLS + c) >> 2) ^ (lane & 7)) << 4)) = make_float4(v[0], v[1], v[2], v[3]);
-        else if (row < p.M) store(z, row, col0 + c, v);
+      // Where sums go: the output, or (split tiles) this CTA's share in the stages that no copy or product uses any more;
+      // 16-byte pieces of a row trade places so that eight rows meet eight bank groups.
+      auto put = [&](int r, int c, const float (&v)[4]) {
+        if (p.splits > 1) *reinterpret_cast<float4*>(smem + r * (BN * 4) + (((c >> 2) ^ (r & 7)) << 4)) = make_float4(v[0], v[1], v[2], v[3]);
+        else if (m0 + r < p.M) store(z, m0 + r, n0 + c, v);
       };
       if (again) {
-        const int k_end = min(p.K, (kb0 + num_kb) * FS_BK);
+        // Plain fused multiply-adds for the warp's 32 rows, 8 rows x 4 columns a lane, straight from global memory: the lines of
+        // the tile's operands, 24 KB, stay in the L1 cache while their 32 k are used.  Rows past an operand repeat its last one.
+        // A load takes the cache a cycle per line and eight lanes: eight neighbours share two rows of A and four of B.
+        int l = lane;
+        asm volatile("" : "+r"(l));      // (what follows from l is not to be kept in registers through the main loop)
+        const int r0 = q * 32 + ((l & 1) | (l >> 2 & 2)), c0 = half * COLS + ((l >> 1 & 3) | (l >> 2 & 4)) * 4, k_end = min(p.K, (kb0 + num_kb) * FS_BK);
+        const float* A = p.A + batch(z, p.a_b0, p.a_b1) + (int64_t)m0 * p.lda;
+        const float* B = p.B + batch(z, p.b_b0, p.b_b1) + (int64_t)n0 * p.ldb;
 #pragma unroll 1
-        for (int c = 0; c < COLS; c += 4) {
-          float v[4] = {0.f, 0.f, 0.f, 0.f};
-          if (row < p.M) {
-            const float* a = p.A + batch(z, p.a_b0, p.a_b1) + (int64_t)row * p.lda;
-            const float* b = p.B + batch(z, p.b_b0, p.b_b1) + (int64_t)(col0 + c) * p.ldb;
-#pragma unroll 1
-            for (int k = kb0 * FS_BK; k < k_end; ++k) {
+        for (int c = c0; c < half * COLS + COLS; c += 32) {
+          float v[8][4];
+          int oa[8], ob[4];
 #pragma unroll
-              for (int i = 0; i < 4; ++i)
-                if (col0 + c + i < p.N) v[i] = fmaf(a[k], b[(int64_t)i * p.ldb + k], v[i]);
+          for (int i = 0; i < 8; ++i) oa[i] = min(r0 + 4 * i, p.M - 1 - m0) * p.lda;
+#pragma unroll
+          for (int j = 0; j < 4; ++j) ob[j] = min(c + j, p.N - 1 - n0) * p.ldb;
+#pragma unroll
+          for (int i = 0; i < 8; ++i)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[i][j] = 0.f;
+#pragma unroll 1
+          for (int k = kb0 * FS_BK; k < k_end; k += 4) {
+            float4 b[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) b[j] = __ldg(reinterpret_cast<const float4*>(B + k + ob[j]));
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const float4 a = __ldg(reinterpret_cast<const float4*>(A + k + oa[i]));
+#pragma unroll
+              for (int j = 0; j < 4; ++j) v[i][j] = fmaf(a.w, b[j].w, fmaf(a.z, b[j].z, fmaf(a.y, b[j].y, fmaf(a.x, b[j].x, v[i][j]))));
             }
           }
-          put(c, v);
+#pragma unroll
+          for (int i = 0; i < 8; ++i) put(r0 + 4 * i, c, v[i]);
         }
       } else {
 #pragma unroll
         for (int c = 0; c < COLS; c += 4) {
           const float v[4] = {acc[c], acc[c + 1], acc[c + 2], acc[c + 3]};
-          put(c, v);
+          put(q * 32 + lane, half * COLS + c, v);
         }
       }
     }

@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from kandle_b200 import core
+from kandle_b200.backend import CudaEvent
 from kandle_b200.core import Tensor
 
 pytestmark = pytest.mark.gpu
@@ -66,3 +67,26 @@ def test_matmul_f32_tiny_operand(backend, scale):
     got = core.matmul(Tensor(a), Tensor(b), transposeB=True).dataAsync()
     exact = a.astype(np.float64) @ b.astype(np.float64).T
     assert (np.abs(got - exact) <= 16 * _bound(a, b)).all()
+
+
+@pytest.mark.parametrize("value", [1e-35, np.nan])
+def test_matmul_f32_numbers_without_a_split_are_no_cliff(backend, value):
+    """A number in every tile that sends it to plain multiply-adds: about 9 times the time of the split ones (that is the time
+    of matmul_f32_kernel); the bound leaves room for a busy machine, and a scalar loop took 240 times."""
+    a, b = _rand((512, 1024), 10), _rand((3072, 1024), 11)
+
+    def once(x):
+        ta, tb = Tensor(x), Tensor(b)
+        start, stop = CudaEvent(), CudaEvent()
+        best = np.inf
+        for _ in range(4):
+            start.record()
+            for _ in range(4):
+                core.matmul(ta, tb, transposeB=True).dispose()
+            stop.record()
+            best = min(best, start.elapsed_ms(stop))
+        return best
+
+    bad = a.copy()
+    bad[::16, 3] = value
+    assert once(bad) < 40 * once(a)
