@@ -15,6 +15,9 @@
 // NaN or number from 2^127 on end), are computed again by their accumulating warps with plain fused multiply-adds, in the
 // order of matmul_f32_kernel.  One such number costs its tiles, a denormal weight every row of tiles: 512 x 3072 x 1024 takes
 // 38 us, 356 with every tile computed again (matmul_f32_kernel 367); 2048 x 4096 x 4096 463 and 5512 us (7510).
+// Where an operand has numbers below 2^-50, the small terms of a product may be subnormal and lose bits to the tensor core;
+// that shows in sums below 2^-100 (8.9e-16, 7.9e-31), and 32 rows with such a sum are computed again likewise.  Operands of
+// 1e-20 at K = 1024: 4.0e-6 relative, 1.7e-5 by the split alone; of 1e-19 and 3e-20: 3.0e-7, 6.0e-7.
 //
 // Structure (one persistent CTA per SM, 640 threads):
 //   warps 0-7    global fp32 -> registers (next k-block in flight) -> three bf16 planes per operand in shared memory,
@@ -89,6 +92,9 @@ __device__ __forceinline__ uint32_t least(uint32_t now, float a, float b) {
   return min(now, min(2u * __float_as_uint(a) - 1u, 2u * __float_as_uint(b) - 1u));
 }
 constexpr uint32_t FS_LEAST = 2u * (27u << 23) - 1u;      // 2^-100
+// From 2^-50 on in both operands, the kept terms of a product that matter are normal numbers.
+constexpr uint32_t FS_LOW = 2u * (77u << 23) - 1u;        // 2^-50
+constexpr float FS_LOW_SUM = 0x1p-100f;
 
 template <int REGS>
 __device__ __forceinline__ void regs_dec() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS)); }
@@ -127,9 +133,10 @@ __global__ void __launch_bounds__(FS_THREADS, 1) gemm_f32_split_kernel(SplitPara
   uint64_t* rest_empty = rest_full + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(rest_empty + 2);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
-  // a tile outside the range of the split: its ordinal + 1.  The converting warps are at most four tiles ahead of the
-  // accumulating ones (two stages, two buffers of small terms).
+  // a tile with numbers below the range of the split, and one with numbers below FS_LOW: its ordinal + 1.  The converting
+  // warps are at most four tiles ahead of the accumulating ones (two stages, two buffers of small terms).
   volatile int* bad_tile = abort_flag + 1;
+  volatile int* low_tile = bad_tile + 8;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
@@ -139,7 +146,7 @@ __global__ void __launch_bounds__(FS_THREADS, 1) gemm_f32_split_kernel(SplitPara
       mbar_init(&rest_full[b], 1); mbar_init(&rest_empty[b], FS_ACC / 32);
     }
     *abort_flag = 0;
-    for (int i = 0; i < 8; ++i) bad_tile[i] = 0;
+    for (int i = 0; i < 16; ++i) bad_tile[i] = 0;
     fence_mbar_init();
   }
   if (warp == FS_WARP_MMA) {
@@ -284,7 +291,10 @@ __global__ void __launch_bounds__(FS_THREADS, 1) gemm_f32_split_kernel(SplitPara
           *reinterpret_cast<uint2*>(d + plane) = m;
           *reinterpret_cast<uint2*>(d + 2 * plane) = l;
         }
-        if (kb + 1 == num_kb && small < FS_LEAST) bad_tile[ordinal & 7] = ordinal + 1;
+        if (kb + 1 == num_kb && small < FS_LOW) {
+          low_tile[ordinal & 7] = ordinal + 1;
+          if (small < FS_LEAST) bad_tile[ordinal & 7] = ordinal + 1;
+        }
         fence_async_proxy();
         __syncwarp();
         if (lane == 0) mbar_arrive(&full[stage]);      // (an arrival of every thread takes longer than the products)
@@ -334,9 +344,10 @@ __global__ void __launch_bounds__(FS_THREADS, 1) gemm_f32_split_kernel(SplitPara
         for (int i = 0; i < 16; ++i) acc[c + i] += __uint_as_float(x[i]);
       }
       // infinity, NaN and numbers from 2^127 on leave no finite sum behind (their parts hold infinity less infinity)
+      const float least_sum = low_tile[ordinal & 7] == ordinal + 1 ? FS_LOW_SUM : 0.f;
       bool again = bad_tile[ordinal & 7] == ordinal + 1;
 #pragma unroll
-      for (int i = 0; i < COLS; ++i) again |= !(fabsf(acc[i]) < INFINITY);
+      for (int i = 0; i < COLS; ++i) again |= !(fabsf(acc[i]) < INFINITY) | (fabsf(acc[i]) < least_sum);
       again = __any_sync(0xffffffffu, again);
       tc_fence_before();
       __syncwarp();

@@ -90,3 +90,15 @@ def test_matmul_f32_numbers_without_a_split_are_no_cliff(backend, value):
     bad = a.copy()
     bad[::16, 3] = value
     assert once(bad) < 40 * once(a)
+
+
+@pytest.mark.parametrize("m,n,k", [(130, 130, 1024), (300, 1000, 512)])
+@pytest.mark.parametrize("sa,sb", [(1e-20, 1e-20), (3e-20, 1e-19), (1e-24, 1e-15)])
+def test_matmul_f32_products_near_the_least_number(backend, m, n, k, sa, sb):
+    """Operands inside the split's range whose products and sums are subnormal or nearly: K multiply-adds round by at most
+    half of the least number, or 2^-25 of the partial sum, each, independently of one another."""
+    a, b = _rand((m, k), 12) * np.float32(sa), _rand((n, k), 13) * np.float32(sb)
+    got = core.matmul(Tensor(a), Tensor(b), transposeB=True).dataAsync()
+    exact = a.astype(np.float64) @ b.astype(np.float64).T
+    step = 0.5 * np.sqrt(k) * (2.0 ** -149 + 2.0 ** -24 * np.sqrt((exact ** 2).mean()))
+    assert np.sqrt(((got - exact) ** 2).mean()) <= step
