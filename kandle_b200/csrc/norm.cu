@@ -147,9 +147,17 @@ __global__ void __launch_bounds__(THREADS) norm_kernel(const void* __restrict__ 
 }
 
 // bf16 rows of up to 2048 elements, dense: one warp per row, the row held in registers between the
-// statistics and the write (one read of x, 16-byte accesses), the next row fetched meanwhile.  Same arithmetic as norm_kernel.
-// HBM-bound; 96000 rows of 768: 64.3 us, 72.6 without the early fetch and with a fourth, empty vector a lane.
-template <int MODE, int NV>
+// statistics and the write (one read of x, 16-byte accesses).  Same arithmetic as norm_kernel.
+// HBM-bound.  How the loads are placed decides how many bytes a warp and an SM have on their way; times of the loads in turn:
+//   NORM_IN_TURN  each vector is loaded and summed: few registers, so many warps.  LayerNorm of 24000 rows of 1024: 22.6 us
+//                 (NORM_ROW 1.07, NORM_NEXT 1.30); of 256: NORM_NEXT 1.14.
+//   NORM_ROW      all vectors of the row before the first sum, for rows of many vectors: LayerNorm of 24000 rows of 2048
+//                 0.57, 6000 rows 0.83 (NORM_NEXT 1.22).
+//   NORM_NEXT     also the next row while this one is normalised: pays from the third row of a warp on, where the registers
+//                 allow it (RMSNorm needs fewer).  96000 rows of 768: 0.84 (NORM_ROW 0.98), 12000 rows 1.00 (0.96); RMSNorm
+//                 of 96000 rows of 1024: 0.92, of 1280: 0.47 (NORM_ROW 0.53).
+enum { NORM_IN_TURN = 0, NORM_ROW = 1, NORM_NEXT = 2 };
+template <int MODE, int NV, int LOADS>
 __global__ void __launch_bounds__(256) norm_rows_bf16_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                                                             const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y,
                                                             int64_t rows, int n, float eps) {
@@ -157,20 +165,22 @@ __global__ void __launch_bounds__(256) norm_rows_bf16_kernel(const __nv_bfloat16
   const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
   const int nvec = n >> 3;
-  uint4 raw[NV];      // the next row, on its way while this one is normalised
+  uint4 raw[NV];
   auto fetch = [&](int64_t row) {
 #pragma unroll
     for (int t = 0; t < NV; ++t)
       if (lane + t * 32 < nvec) raw[t] = reinterpret_cast<const uint4*>(x + row * n)[lane + t * 32];
   };
-  if (warp0 < rows) fetch(warp0);
+  if (LOADS == NORM_NEXT && warp0 < rows) fetch(warp0);
   for (int64_t row = warp0; row < rows; row += nwarps) {
+    if (LOADS == NORM_ROW) fetch(row);
     float v[NV][8];
     float s = 0.f;
 #pragma unroll
     for (int t = 0; t < NV; ++t) {
       const int vi = lane + t * 32;
       if (vi < nvec) {
+        if (LOADS == NORM_IN_TURN) raw[t] = reinterpret_cast<const uint4*>(x + row * n)[vi];
         const __nv_bfloat16* h = reinterpret_cast<const __nv_bfloat16*>(&raw[t]);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
@@ -179,7 +189,7 @@ __global__ void __launch_bounds__(256) norm_rows_bf16_kernel(const __nv_bfloat16
         }
       }
     }
-    if (row + nwarps < rows) fetch(row + nwarps);
+    if (LOADS == NORM_NEXT && row + nwarps < rows) fetch(row + nwarps);
     s = warp_sum(s);
     float mean = 0.f, sc;
     if (MODE == NORM_RMS) {
@@ -235,12 +245,12 @@ __global__ void __launch_bounds__(256) norm_rows_bf16_kernel(const __nv_bfloat16
   }
 }
 
-template <int MODE, int NV>
+template <int MODE, int NV, int LOADS>
 static void launch_norm_rows_bf16(const void* x, const void* w, const void* b, void* y, int64_t rows, int n, float eps) {
   int64_t blocks = (rows + 7) / 8;
   const int64_t cap = (int64_t)ctx().sm_count * 16;
   if (blocks > cap) blocks = cap;
-  norm_rows_bf16_kernel<MODE, NV><<<(int)blocks, 256, 0, ctx().stream>>>(
+  norm_rows_bf16_kernel<MODE, NV, LOADS><<<(int)blocks, 256, 0, ctx().stream>>>(
       static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w), static_cast<const __nv_bfloat16*>(b),
       static_cast<__nv_bfloat16*>(y), rows, n, eps);
 }
@@ -273,11 +283,16 @@ static int launch_norm(const kd_tensor* x, const kd_tensor* w, const kd_tensor* 
       ((reinterpret_cast<uintptr_t>(px) | reinterpret_cast<uintptr_t>(py) | reinterpret_cast<uintptr_t>(pw) |
         reinterpret_cast<uintptr_t>(pb)) & 15) == 0) {
     constexpr int M2 = MODE == NORM_SOFTMAX ? NORM_RMS : MODE;   // the softmax instantiation is never launched
-    if (n <= 256) launch_norm_rows_bf16<M2, 1>(px, pw, pb, py, rows, (int)n, eps);
-    else if (n <= 512) launch_norm_rows_bf16<M2, 2>(px, pw, pb, py, rows, (int)n, eps);
-    else if (n <= 768) launch_norm_rows_bf16<M2, 3>(px, pw, pb, py, rows, (int)n, eps);
-    else if (n <= 1024) launch_norm_rows_bf16<M2, 4>(px, pw, pb, py, rows, (int)n, eps);
-    else launch_norm_rows_bf16<M2, 8>(px, pw, pb, py, rows, (int)n, eps);
+    const bool many = rows > (int64_t)sms * 16 * 8 * 2;          // (the launch's warps take a third row)
+    constexpr int WIDE = MODE == NORM_RMS ? NORM_NEXT : NORM_ROW, WIDE4 = MODE == NORM_RMS ? NORM_NEXT : NORM_IN_TURN;
+    if (n <= 256) launch_norm_rows_bf16<M2, 1, NORM_IN_TURN>(px, pw, pb, py, rows, (int)n, eps);
+    else if (n <= 512) launch_norm_rows_bf16<M2, 2, NORM_IN_TURN>(px, pw, pb, py, rows, (int)n, eps);
+    else if (n <= 768) many ? launch_norm_rows_bf16<M2, 3, NORM_NEXT>(px, pw, pb, py, rows, (int)n, eps)
+                            : launch_norm_rows_bf16<M2, 3, NORM_ROW>(px, pw, pb, py, rows, (int)n, eps);
+    else if (n <= 1024) many ? launch_norm_rows_bf16<M2, 4, WIDE4>(px, pw, pb, py, rows, (int)n, eps)
+                             : launch_norm_rows_bf16<M2, 4, NORM_IN_TURN>(px, pw, pb, py, rows, (int)n, eps);
+    else many ? launch_norm_rows_bf16<M2, 8, WIDE>(px, pw, pb, py, rows, (int)n, eps)
+              : launch_norm_rows_bf16<M2, 8, NORM_ROW>(px, pw, pb, py, rows, (int)n, eps);
     return after_launch(name);
   }
   if (n <= 512) {

@@ -155,6 +155,15 @@ def test_norms_of_bf16_rows(backend, oracle, rows, n):
     close(core.rmsNorm(tx, (n,), tw, 1e-6).dataAsync(), oracle.rms_norm(x, w, 1e-6), 4e-3)
 
 
+@pytest.mark.parametrize("rows, n", [(37888, 520), (37889, 520), (37900, 1024), (37900, 1032)])
+def test_norms_of_very_many_bf16_rows(backend, oracle, rows, n):
+    """Both sides of the number of rows from which on a warp fetches its next row early."""
+    x, w, b = (lib.round_to_bf16(synth.normal(k, s)) for k, s in (("x", (rows, n)), ("w", (n,)), ("b", (n,))))
+    tx, tw, tb = (Tensor(v, dtype="bfloat16") for v in (x, w, b))
+    close(core.layerNorm(tx, (n,), tw, tb, 1e-5).dataAsync(), oracle.layer_norm(x, w, b, 1e-5), 4e-3)
+    close(core.rmsNorm(tx, (n,), tw, 1e-6).dataAsync(), oracle.rms_norm(x, w, 1e-6), 4e-3)
+
+
 @pytest.mark.parametrize("rows,n", [(9, 333), (2, 151936), (64, 77)])
 def test_softmax(backend, oracle, rows, n):
     x = synth.normal("x", (rows, n), 4.0)
