@@ -271,9 +271,10 @@ static bool attention_tile_fits(const void* pq, const void* pk, const void* pv, 
 
 template <int D>
 static int launch_attention_tile_rows(const void* pq, const void* pk, const void* pv, void* po, const AttnParams& p) {
-  // Rows a CTA: 32 (half the key reads a row) where that leaves a CTA for every SM, 16 otherwise.  Causal, heads of 128:
-  // 16 heads of 128 queries 14.5 us with 16 rows, 16.5 with 32; 64 heads of 512 queries 215 and 148 us (64 rows: 178).
-  if ((int64_t)p.Hq * p.B * ((p.Sq + 31) / 32) >= ctx().sm_count) return launch_attention_tile<D, 4>(pq, pk, pv, po, p);
+  // Rows a CTA: 32 (half the key reads a row) where there are more than 16 and that leaves a CTA for every SM, 16 otherwise.
+  // Causal, heads of 128: 16 heads of 128 queries 14.5 us with 16 rows, 16.5 with 32; 64 heads of 512 queries 215 and 148 us
+  // (64 rows: 178).  256 heads of 64, one query, one key: 4.9 us with 16 rows, 6.1 with 32 (attention_f32_kernel 5.0).
+  if (p.Sq > 16 && (int64_t)p.Hq * p.B * ((p.Sq + 31) / 32) >= ctx().sm_count) return launch_attention_tile<D, 4>(pq, pk, pv, po, p);
   return launch_attention_tile<D, 2>(pq, pk, pv, po, p);
 }
 
@@ -328,7 +329,10 @@ int attention_f32_dispatch(const kd_tensor* q, const kd_tensor* k, const kd_tens
   KD_REQUIRE(p.Skv > 0, "flash_attention: empty key/value sequence");
   KD_REQUIRE(p.Hq <= 65535 && p.B <= 65535, "flash_attention: too many heads or batches for one launch");
   KD_REQUIRE(p.D >= 1, "flash_attention: empty head dimension");
-  if (attention_tile_fits(pq, pk, pv, po, p))
+  // A few rows of heads of 128 against a few keys: the general kernel is through sooner (16 heads, one query: 1 key 5.4 us,
+  // 5.9 in tiles; 4 keys 5.5, 5.9; 8 keys 5.9, 5.9; 256 heads, 1 key: 10.0, 6.6)
+  const bool few = p.D == 128 && p.Skv <= 6 && p.Sq <= ATT_WARPS && (int64_t)p.Hq * p.B <= ctx().sm_count;
+  if (!few && attention_tile_fits(pq, pk, pv, po, p))
     return p.D == 64 ? launch_attention_tile_rows<64>(pq, pk, pv, po, p) : launch_attention_tile_rows<128>(pq, pk, pv, po, p);
   if (p.D <= 32) return launch_attention_f32<1>(pq, pk, pv, po, p);
   if (p.D <= 64) return launch_attention_f32<2>(pq, pk, pv, po, p);

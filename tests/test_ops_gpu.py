@@ -56,6 +56,15 @@ def test_sdpa_register_tiles(backend, oracle, heads, sq, skv, d):
         assert not np.isfinite(got[:, :, 32:]).any()
 
 
+@pytest.mark.parametrize("heads", [4, 148, 150])
+@pytest.mark.parametrize("sq, skv", [(1, 6), (1, 7), (16, 6), (17, 6), (6, 6)])
+def test_sdpa_a_few_rows_and_keys(backend, oracle, heads, sq, skv):
+    """Both sides of the rules for short calls: keys, rows and heads."""
+    q, k, v = synth.normal("q", (1, heads, sq, 128)), synth.normal("k", (1, heads // 2, skv, 128)), synth.normal("v", (1, heads // 2, skv, 128))
+    for causal in (False, True):
+        close(core.scaledDotProductAttention(Tensor(q), Tensor(k), Tensor(v), None, 0.0, causal).dataAsync(), oracle.sdpa(q, k, v, is_causal=causal))
+
+
 def test_sdpa_3d_and_strided_inputs(backend, oracle):
     q, k, v = synth.normal("q", (6, 20, 64)), synth.normal("k", (6, 20, 64)), synth.normal("v", (6, 20, 64))
     out = core.scaledDotProductAttention(Tensor(q), Tensor(k), Tensor(v))
