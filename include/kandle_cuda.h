@@ -117,6 +117,11 @@ int kd_workspace_bytes(uint64_t* bytes_out);
  * buffer of kd_attention_decode_noalloc with `byte_value` (stream-ordered), so that a test can tell
  * a kernel that read a slot it never wrote (0xFF gives NaN patterns) from one that did not. */
 int kd_debug_fill_scratch(int byte_value);
+/* Test support, no counterpart in the reference: which form the library would give a call on a GPU of `sms`
+ * multiprocessors.  Touch no device.
+ *   recurrence   whether kd_delta_rule (delta = 1) or kd_wkv takes a call of `tokens` tokens and `heads` heads (of all
+ *                sequences) through records, and the CTAs of that form's second kernel */
+int kd_debug_recurrence_plan(int delta, int bf16, int dim, int vdim, int heads, int tokens, int sms, int* records, int* ctas);
 int kd_empty_cache(void);
 
 /* ---------------------------------------------------------------------------------------------

@@ -891,7 +891,7 @@ static int launch_delta_few(const void* proj, const void* hist, int64_t hist_b, 
   RecStream r{};
   r.units = p.B * p.H; r.H = p.H; r.S = p.S; r.vdim = p.vdim; r.dk_pad = p.dk_pad; r.dv_pad = p.dv_pad;
   r.state = p.state; r.o = p.o;
-  return launch_recurrence<16 * LPC, true>(r, handled, [&](const RecStream& part) {
+  return launch_recurrence<16 * LPC, true, sizeof(T) == 2>(r, handled, [&](const RecStream& part) {
     const int64_t items = (int64_t)part.units * part.groups;
     KD_CUDA_CHECK(launch_ex(delta_prepare_kernel<T, LPC>, dim3((unsigned)((items + 3) / 4)), dim3(128), 0, (const T*)proj, (const T*)hist, hist_b, hist_ld, p, part));
     return after_launch("delta_prepare_kernel");
@@ -949,6 +949,16 @@ KD_API int kd_delta_state_shape(int dim, int vdim, int* rows_out, int* cols_out)
   while (r < dim) r *= 2;
   *rows_out = r;
   *cols_out = (vdim + 7) / 8 * 8;
+  return KD_OK;
+}
+
+KD_API int kd_debug_recurrence_plan(int delta, int bf16, int dim, int vdim, int heads, int tokens, int sms, int* records, int* ctas) {
+  KD_REQUIRE(records && ctas && heads >= 1 && tokens >= 1 && sms >= 1, "bad argument");
+  int rows, cols, warps, tiles;
+  KD_TRY(kd_delta_state_shape(dim, vdim, &rows, &cols));
+  recurrence_shape(rows, cols, &warps, &tiles);
+  *ctas = heads * tiles;
+  *records = recurrence_takes_records(delta != 0, bf16 != 0, rows, *ctas, tokens, sms);
   return KD_OK;
 }
 

@@ -467,6 +467,33 @@ constexpr int64_t REC_SCRATCH = 64 << 20;
 // ... but at least this many groups a portion, or loading and storing the states would count.
 constexpr int REC_LEAST_GROUPS = 32;
 
+// Least tokens of a call that take records, by [delta rule][16-bit inputs][key channels 32, 64, 128, 256][CTAs of the walk
+// in units of SMs, rounded up, 1 .. 4]; 0: none do.  Both forms measured for 10 to 592 CTAs and 32 to 1000 tokens; a number
+// stands where the records were the shorter from there on (time of the records over the one-kernel form's):
+//   delta, bf16  64 channels, 4: 0.92 to 1.07, no gain.  128, 3: 1.05 at 32 tokens, 0.97 at 40; 4: 1.14 at 32, 0.95 at 64
+//   delta, fp32  64, 4: 1.10 at 32, 0.96 at 40
+//   WKV, bf16    64, 4: 1.07 at 32, 0.97 at 48.  128, 3: 1.10 at 32, 0.98 at 48; 4: 1.38 at 32, 0.97 at 256.
+//                256, 2: 1.23 at 32, 0.95 at 64; 3: 1.58 at 32, 1.06 at 600; 4: 1.79 and 1.31
+//   WKV, fp32    128, 4: 1.28 at 32, 0.97 at 96.  256, 3: 1.11 at 32, 0.97 at 40; 4: 1.27 at 32, 0.89 at 96
+//   elsewhere    0.12 to 0.95; 16 tokens: 30 us against 28 (delta rule, 16 heads of 128)
+constexpr int REC_LEAST_TOKENS[2][2][4][4] = {
+    {{{32, 32, 32, 32}, {32, 32, 32, 32}, {32, 32, 32, 96}, {32, 32, 40, 96}},
+     {{32, 32, 32, 32}, {32, 32, 32, 48}, {32, 32, 48, 256}, {32, 64, 0, 0}}},
+    {{{32, 32, 32, 32}, {32, 32, 32, 40}, {32, 32, 32, 32}, {32, 32, 32, 32}},
+     {{32, 32, 32, 32}, {32, 32, 32, 0}, {32, 32, 40, 64}, {32, 32, 32, 32}}}};
+// Warps of a CTA and CTAs of a head whose state has dk rows and dv_pad columns.
+inline void recurrence_shape(int dk, int dv_pad, int* warps, int* tiles) {
+  const int cpw = REC_COLS * 32 * rec_rows(dk) / dk, all = (dv_pad + cpw - 1) / cpw;
+  *warps = all > REC_WARPS ? REC_WARPS : all;
+  *tiles = (dv_pad + *warps * cpw - 1) / (*warps * cpw);
+}
+inline bool recurrence_takes_records(bool delta, bool half, int dk, int64_t ctas, int S, int sms) {
+  const int64_t waves = (ctas + sms - 1) / sms;
+  if (waves < 1 || waves > 4) return false;
+  const int least = REC_LEAST_TOKENS[delta][half][dk <= 32 ? 0 : dk <= 64 ? 1 : dk <= 128 ? 2 : 3][waves - 1];
+  return least > 0 && S >= least;
+}
+
 template <int DK, bool DELTA>
 static int launch_recurrence_kernel(const RecStream& p, int warps) {
   const int smem = p.stages * REC_STAGE_GROUPS * (rec_floats(DELTA, DK) + p.dvc * 4) * 4;
@@ -481,21 +508,15 @@ static int launch_recurrence_kernel(const RecStream& p, int warps) {
 
 // Walks through a prompt in portions; prepare(portion) launches the layer's prepare kernel for one.  *handled = 0: the
 // heads fill the chip by themselves, or there is no room for records, and the caller's one-kernel form is to run.
-template <int DK, bool DELTA, typename Prepare>
+template <int DK, bool DELTA, bool HALF, typename Prepare>
 static int launch_recurrence(RecStream p, int* handled, Prepare&& prepare) {
   *handled = 0;
-  constexpr int CPW = REC_COLS * 32 * rec_rows(DK) / DK;
   const int sms = ctx().sm_count;
-  int warps = (p.dv_pad + CPW - 1) / CPW;
-  if (warps > REC_WARPS) warps = REC_WARPS;
-  p.dvc = warps * CPW;
-  p.tiles = (p.dv_pad + p.dvc - 1) / p.dvc;
+  int warps;
+  recurrence_shape(DK, p.dv_pad, &warps, &p.tiles);
+  p.dvc = warps * (REC_COLS * 32 * rec_rows(DK) / DK);
   const int64_t ctas = (int64_t)p.units * p.tiles;
-  // Where the line lies (microseconds of a call, this form against the one-kernel form; heads of 128 x 128 and 64 x 64):
-  //   delta, 1000 tokens  64 heads (512 CTAs) 553, 711; 80 heads (640) 743, 726; 128 heads 1063, 730
-  //   WKV, 1000 tokens    128 heads (256 CTAs) 232, 436; 192 heads (384) 297, 437; 256 heads (512) 433, 438
-  //   delta, 16 heads     16 tokens 30, 28; 64 tokens 33, 61; 8192 tokens 1553, 5666
-  if (ctas > 4 * sms || p.S < 32) return KD_OK;
+  if (!recurrence_takes_records(DELTA, HALF, DK, ctas, p.S, sms)) return KD_OK;
   const int stage_bytes = REC_STAGE_GROUPS * (rec_floats(DELTA, DK) + p.dvc * 4) * 4;
   const int room = (ctas <= sms ? 200 : ctas <= 2 * sms ? 100 : 50) * 1024 / stage_bytes;
   p.stages = room < 2 ? 2 : room > REC_MAX_STAGES ? REC_MAX_STAGES : room;

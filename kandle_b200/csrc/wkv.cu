@@ -648,7 +648,7 @@ static int launch_wkv_few(const void* r, const void* k, const void* v, const Wkv
   RecStream rs{};
   rs.units = p.B * p.H; rs.H = p.H; rs.S = p.S; rs.vdim = p.dim; rs.dk_pad = p.dk_pad; rs.dv_pad = p.dv_pad;
   rs.state = p.state; rs.o = p.o;
-  return launch_recurrence<16 * LPC, false>(rs, handled, [&](const RecStream& part) {
+  return launch_recurrence<16 * LPC, false, sizeof(T) == 2>(rs, handled, [&](const RecStream& part) {
     constexpr int PER = 4 * (LPC < 8 ? 8 / LPC : 1);
     const int64_t items = (int64_t)part.units * part.groups;
     KD_CUDA_CHECK(launch_ex(wkv_prepare_kernel<T, LPC>, dim3((unsigned)((items + PER - 1) / PER)), dim3(128), 0, (const T*)r, (const T*)k, (const T*)v, p, part));
