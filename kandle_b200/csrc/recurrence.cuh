@@ -373,6 +373,13 @@ recurrence_kernel(RecStream p) {
           u[2][c] = beta.z * ((v.z - u[2][c]) - fmaf(m1.z, u[1][c], m0.z * u[0][c]));
           u[3][c] = beta.w * ((v.w - u[3][c]) - fmaf(m2.w, u[2][c], fmaf(m1.w, u[1][c], m0.w * u[0][c])));
         }
+        // (a group's tokens past the end of the prompt write nothing, not even zero times an infinity)
+        if (t0 + 4 > p.S) {
+#pragma unroll
+          for (int t = 1; t < 4; ++t)
+#pragma unroll
+            for (int c = 0; c < C; ++c) u[t][c] = t0 + t < p.S ? u[t][c] : 0.f;
+        }
       } else {
 #pragma unroll
         for (int c = 0; c < C; ++c) {
@@ -405,7 +412,7 @@ recurrence_kernel(RecStream p) {
     } else {
       const float* direct = p.direct + ((int64_t)unit * p.groups + g) * 4 * DK;
 #pragma unroll 1
-      for (int t = 0; t < 4; ++t) {
+      for (int t = 0; t < 4 && t0 + t < p.S; ++t) {
         float x[C], u[C];
         auto sum = [&] {
 #pragma unroll
@@ -435,7 +442,7 @@ recurrence_kernel(RecStream p) {
         }
 #pragma unroll
         for (int c = 0; c < C; ++c)
-          if (j == 0 && t0 + t < p.S && col + c < p.vdim) out[(t0 + t) * o_ld + c] = x[c];
+          if (j == 0 && col + c < p.vdim) out[(t0 + t) * o_ld + c] = x[c];
       }
       fetch_next();
     }

@@ -318,3 +318,31 @@ def test_delta_rule_many_heads_share_a_block(backend):
     """Enough heads for several per block, in a batch: bf16 and fp32 agree with the plain form for every one."""
     _delta_case(20, 19, 16, 8, 64, 64, 4, "bfloat16", [18, 1])
     _delta_case(12, 19, 32, 16, 32, 32, 4, "float32", [2, 17])
+
+
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+@pytest.mark.parametrize("decay", [-3.0, 60.0])
+def test_delta_rule_infinities_at_the_end_of_a_prompt(backend, dtype, decay):
+    """The last token's value is infinite in some columns: the state behind a prompt of records (33 tokens, three of the last
+    record past the end) is finite, infinite and not a number where the one-kernel form leaves it so."""
+    S, H, dim = 33, 2, 64
+    rng = _rng(S, 5)
+    n, qk = 3 * H * dim + 8, H * dim
+    proj = _bf(rng.standard_normal((1, S, n)))
+    proj[0, -1, 2 * qk + 3:3 * qk:7] = np.inf
+    a, conv = np.zeros((S, H * dim), np.float32), [np.full((qk, 4), 0.5, np.float32)] * 3
+    states = []
+    for cuts in ([33], [31, 2]):
+        state, hist, at = core.zeros((1, H, 64, 64)), core.zeros((1, 3, 3 * qk), dtype), 0
+        for m in cuts:
+            pd, o, y = _put(proj[:, at:at + m], dtype), core.empty((m, qk)), core.empty((m, qk), dtype)
+            lib.call("kd_delta_rule", _r(pd), 0, qk, 2 * qk, 3 * qk, _r(_put(a[at:at + m])), H, H, dim, dim, *(_r(_put(x)) for x in conv), _r(_put(-np.ones(H, np.float32))),
+                     _r(_put(np.full(H * dim, decay, np.float32))), _r(hist), _r(state), _r(o))
+            lib.call("kd_delta_out", _r(o), _r(_put(np.ones((m, qk), np.float32), dtype)), _r(_put(np.ones(dim, np.float32))), F(1e-5), 0, _r(pd), 0, 4, _r(hist), _r(y))
+            at += m
+        states.append(_get(state)[0])
+    got, want = states
+    assert np.isinf(want).any() and np.isfinite(want).any()
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(got[np.isinf(want)], want[np.isinf(want)])
+    kept = np.isfinite(want)
+    assert np.abs(got[kept] - want[kept]).max() <= 1e-5 * np.abs(want[kept]).max()
