@@ -346,3 +346,29 @@ def test_delta_rule_infinities_at_the_end_of_a_prompt(backend, dtype, decay):
     assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(got[np.isinf(want)], want[np.isinf(want)])
     kept = np.isfinite(want)
     assert np.abs(got[kept] - want[kept]).max() <= 1e-5 * np.abs(want[kept]).max()
+
+
+@pytest.mark.parametrize("a_mean, a_sd, rate_sd", [(-2.0, 1.0, 1.0), (8.0, 12.0, 0.5)])
+def test_delta_rule_many_heads_over_long_prompts(backend, a_mean, a_sd, rate_sd):
+    """The one-kernel form where a batch takes it: more heads than records are worth, hundreds of tokens, decays from ordinary
+    ones to those that wipe the state.  (The 16-bit form's softplus, log(1 + exp x), is off by up to 2^-23 and a decay by its
+    rate times that: rates of exp(0.5 N), at most about 5 here, keep that at 6e-7 a token, well inside 3e-5; rates of
+    exp(2 N), up to 150 among 75 heads, do not.)"""
+    for case, dtype in (((5, 210, 15, 5, 128, 128), "bfloat16"), ((5, 201, 60, 30, 64, 64), "float32")):
+        assert not _takes_records(1, dtype, case[4], case[5], case[0] * case[2], case[1])
+        _delta_case(*case, 4, dtype, [case[1]], a_mean, a_sd, rate_sd)
+
+
+def _takes_records(delta, dtype, dim, vdim, heads, tokens):
+    records, ctas = ctypes.c_int(0), ctypes.c_int(0)
+    lib.call("kd_debug_recurrence_plan", delta, int(dtype == "bfloat16"), dim, vdim, heads, tokens, 148, ctypes.byref(records), ctypes.byref(ctas))
+    return bool(records.value)
+
+
+@pytest.mark.parametrize("size", SIZES, ids=str)
+@pytest.mark.parametrize("dtype", ["bfloat16", "float32"])
+def test_delta_rule_sizes_in_short_portions(backend, size, dtype):
+    """Every size in the one-kernel form too: portions below the records' least number of tokens, each longer than its blocks of 16."""
+    for cuts in ([31, 30], [17, 25, 19]):
+        assert not any(_takes_records(1, dtype, size[2], size[3], 2 * size[0], n) for n in cuts)
+        _delta_case(2, 61, *size, dtype, cuts)

@@ -454,3 +454,30 @@ def test_head_decay_delta_rule_long_and_wide(backend):
     _head_delta_case(1, 700, 2, 2, 64, 32, 4, "bfloat16", [400, 2, 298], a_mean=-5.0)
     _head_delta_case(20, 19, 16, 8, 64, 64, 4, "bfloat16", [18, 1])
     _head_delta_case(12, 19, 32, 16, 32, 32, 4, "float32", [2, 17])
+
+
+def _takes_records(delta, dtype, dim, heads, tokens):
+    records, ctas = ctypes.c_int(0), ctypes.c_int(0)
+    lib.call("kd_debug_recurrence_plan", delta, int(dtype == "bfloat16"), dim, dim, heads, tokens, 148, ctypes.byref(records), ctypes.byref(ctas))
+    return bool(records.value)
+
+
+@pytest.mark.parametrize("w_mean, w_sd", [(-1.0, 1.0), (3.0, 3.0)])
+def test_wkv_many_heads_over_long_prompts(backend, w_mean, w_sd):
+    """The one-kernel form where a batch takes it, decays that underflow among them."""
+    for (B, S, H, dim), dtype in (((5, 203, 15, 128), "bfloat16"), ((5, 201, 60, 64), "float32"), ((2, 130, 16, 192), "bfloat16")):
+        assert not _takes_records(0, dtype, dim, B * H, S)
+        _wkv_case(B, S, H, dim, dtype, [S], w_mean, w_sd)
+
+
+def test_head_decay_delta_rule_many_heads_over_long_prompts(backend):
+    for a_mean, a_sd in ((-2.0, 1.0), (8.0, 12.0)):
+        assert not _takes_records(1, "bfloat16", 128, 75, 210)
+        _head_delta_case(5, 210, 15, 5, 128, 128, 4, "bfloat16", [210], a_mean, a_sd)
+
+
+@pytest.mark.parametrize("H, dim", [(2, 16), (3, 64), (3, 20), (4, 128), (2, 130), (1, 256), (2, 33), (5, 48), (1, 7), (2, 96)])
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_wkv_sizes_in_short_portions(backend, H, dim, dtype):
+    """Every size in the one-kernel form too."""
+    _wkv_case(2, 61, H, dim, dtype, [31, 30])
