@@ -27,9 +27,8 @@ def oracle():
     return orc
 
 
-@pytest.fixture(autouse=True)
-def _garbage_first(request):
-    """Tests that account device memory start without garbage of earlier ones: an exception's traceback keeps its frames'
-    tensors until the cycle is collected, which may otherwise happen between two readings."""
-    if any(word in request.node.name for word in ("refcount", "alloc")):
-        gc.collect()
+@pytest.fixture
+def collected():
+    """For tests that account device memory: no garbage of earlier tests is left when they start.  An exception's traceback
+    keeps its frames' tensors until the cycle is collected, which may otherwise happen between two readings."""
+    gc.collect()

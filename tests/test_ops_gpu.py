@@ -304,6 +304,7 @@ def test_conv1d(backend, oracle):
         close(core.conv1d(Tensor(x), Tensor(w), Tensor(b), stride, 1).dataAsync(), oracle.conv1d(x, w, b, stride, 1))
 
 
+@pytest.mark.usefixtures("collected")
 def test_storage_refcount_and_allocator_reuse(backend):
     s0 = backend.memory_stats()
     t = core.zeros((1024, 1024))

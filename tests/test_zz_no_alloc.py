@@ -33,6 +33,7 @@ def _footprint(backend):
     return dict(backend.memory_stats(), workspace=ws.value)
 
 
+@pytest.mark.usefixtures("collected")
 def test_noalloc_decode_attention_matches_the_allocating_entry_point_twice(backend, oracle):
     """Two different problems back to back through the built-in buffer (the second has fewer splits
     and a shorter context, so partials of the first call lie right beside its own), then a call whose
