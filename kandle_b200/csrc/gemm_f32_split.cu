@@ -470,6 +470,23 @@ static int launch_split(SplitParams& p, int64_t batches) {
   return after_launch("gemm_f32_split_kernel");
 }
 
+// Tile width and split of K with the shortest estimate: rounds of CTAs over the SMs, each with its k-blocks and a fixed part.
+static int split_tile(int64_t batches, int64_t M, int64_t N, int64_t K, int64_t sms, int* splits) {
+  const int64_t m_tiles = (M + FS_BM - 1) / FS_BM, kbs = (K + FS_BK - 1) / FS_BK;
+  double best = 1e30;
+  int bn = 128;
+  *splits = 1;
+  for (int w = 64; w <= 128; w += 64) {
+    const int64_t tiles = batches * m_tiles * ((N + w - 1) / w);
+    for (int s = 1; s <= 4 && s <= kbs; s *= 2) {
+      if (s > 1 && tiles * s > sms) break;       // (a CTA of a split tile has one tile)
+      const double cost = (double)((tiles * s + sms - 1) / sms) * ((kbs + s - 1) / s) * (w == 64 ? FS_US_64 : FS_US_128) + (s > 1 ? FS_US_EXCHANGE : 0.0);
+      if (cost < best) { best = cost; bn = w; *splits = s; }
+    }
+  }
+  return bn;
+}
+
 int gemm_f32_split(const F32Gemm& g, int* handled) {
   *handled = 0;
   const uintptr_t base = reinterpret_cast<uintptr_t>(g.a) | reinterpret_cast<uintptr_t>(g.b);
@@ -494,21 +511,18 @@ int gemm_f32_split(const F32Gemm& g, int* handled) {
   // tiles that share the larger operand run side by side, so that it is read from HBM once
   p.m_inner = g.N >= g.M;
   p.err = ctx().error_flag;
-  // Tile width and split of K with the shortest estimate: rounds of CTAs over the SMs, each with its k-blocks and a fixed part.
-  const int64_t batches = g.b0 * g.b1, m_tiles = (g.M + FS_BM - 1) / FS_BM, sms = ctx().sm_count, kbs = (g.K + FS_BK - 1) / FS_BK;
-  double best = 1e30;
-  int bn = 128;
-  p.splits = 1;
-  for (int w = 64; w <= 128; w += 64) {
-    const int64_t tiles = batches * m_tiles * ((g.N + w - 1) / w);
-    for (int s = 1; s <= 4 && s <= kbs; s *= 2) {
-      if (s > 1 && tiles * s > sms) break;       // (a CTA of a split tile has one tile)
-      const double cost = (double)((tiles * s + sms - 1) / sms) * ((kbs + s - 1) / s) * (w == 64 ? FS_US_64 : FS_US_128) + (s > 1 ? FS_US_EXCHANGE : 0.0);
-      if (cost < best) { best = cost; bn = w; p.splits = s; }
-    }
-  }
+  const int64_t batches = g.b0 * g.b1;
+  const int bn = split_tile(batches, g.M, g.N, g.K, ctx().sm_count, &p.splits);
   *handled = 1;
   return bn == 64 ? launch_split<64>(p, batches) : launch_split<128>(p, batches);
 }
 
 }  // namespace kd
+
+using namespace kd;
+
+KD_API int kd_debug_matmul_f32_plan(int64_t batches, int64_t M, int64_t N, int64_t K, int sms, int* width, int* splits) {
+  KD_REQUIRE(width && splits && batches > 0 && M > 0 && N > 0 && K >= FS_BK && sms > 0, "bad argument");
+  *width = split_tile(batches, M, N, K, sms, splits);
+  return KD_OK;
+}

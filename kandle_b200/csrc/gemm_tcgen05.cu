@@ -11,7 +11,7 @@
 //   warp 1      one elected thread issues tcgen05.mma (M=128, N=BLOCK_N, K=16 x4 per stage) into a
 //               TMEM accumulator; tcgen05.commit releases the smem stage / publishes the tile.
 //   Few rows: a cluster of 2 or 4 CTAs shares a tile, each a range of k-blocks; the first adds the others' sums to its own
-//   and has the epilogue (choose_tile).
+//   and has the epilogue (linear_tile).
 //   warps 2-5   epilogue: tcgen05.ld the 128xBLOCK_N fp32 tile (one row per thread), apply the
 //               fused epilogue, convert and store.  Two TMEM accumulators let the epilogue of tile
 //               i overlap the mainloop of tile i+1.
@@ -684,7 +684,7 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams&
   p.num_m_tiles = (p.M + GEMM_BM - 1) / GEMM_BM + (p.groups ? (p.groups < p.M ? p.groups : p.M) : 0);
   p.num_n_tiles = (p.N + BLOCK_N - 1) / BLOCK_N;
   const int64_t total = (int64_t)p.num_m_tiles * p.num_n_tiles;
-  // (choose_tile shares no 256-wide tile; the epilogue over heads is in this instantiation, or the plain one would grow)
+  // (linear_tile shares no 256-wide tile; the epilogue over heads is in this instantiation, or the plain one would grow)
   if (BLOCK_N < 256 && (p.splits > 1 || p.epi == 3)) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)(total * p.splits));
@@ -708,24 +708,27 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams&
   return after_launch("gemm_bf16_tcgen05_kernel");
 }
 
-// Tile width and number of CTAs that share a tile (p.splits) where 256-wide tiles would leave more than half of the GPU idle;
-// widths from `narrowest` on.  An SM takes a k-block in the time of its copies from L2 (about 83 GB/s: 0.28, 0.38, 0.57 us
-// for 64-, 128- and 256-wide tiles); a shared tile costs two barriers of the cluster and the others' sums.  Measured, one CTA
-// and the chosen number a tile, 97 rows: N = 1024, K = 2048 16.3, 12.4 us; N = 1024, K = 3072 20.6, 14.5; N = 768, K = 3072
-// 18.6, 12.5; N = K = 768 8.4, 10.4 (not shared).  Above two rows of tiles it gave little or nothing (700 rows: 16.5, 18.5).
-static int choose_tile(GemmParams& p, int narrowest) {
-  const int64_t m_tiles = (p.M + GEMM_BM - 1) / GEMM_BM, kbs = (p.K + GEMM_BK - 1) / GEMM_BK, sms = ctx().sm_count;
+// Tile width and number of CTAs that share a tile; widths from `narrowest` on.  256 columns where such tiles occupy more than
+// half of the SMs; else the shortest estimate.  An SM takes a k-block in the time of its copies from L2 (about 83 GB/s: 0.28,
+// 0.38, 0.57 us for 64-, 128- and 256-wide tiles); a shared tile costs two barriers of the cluster and the others' sums.
+// One CTA and the chosen number a tile, 97 rows: N = 1024, K = 2048 12.4, 9.5 us; N = 1024, K = 3072 16.9, 10.6; N = 2560,
+// K = 9728 46.2, 22.7; N = K = 768 8.4, 10.4 (not shared).  Measured for 1 to 2103 rows and 15 shapes of weights, none above
+// the time of one CTA a tile by more than its runs differ.  Above two rows of tiles it gave little or nothing (700 rows,
+// N = 1024, K = 2048: 16.5, 18.5).
+static int linear_tile(int64_t M, int64_t N, int64_t K, int narrowest, int64_t sms, int* splits) {
+  const int64_t m_tiles = (M + GEMM_BM - 1) / GEMM_BM, kbs = (K + GEMM_BK - 1) / GEMM_BK;
+  *splits = 1;
+  if (N >= 256 && m_tiles * ((N + 255) / 256) * 2 > sms) return 256;
   double best = 1e30;
   int bn = 256;
-  p.splits = 1;
   for (int w = narrowest; w <= 256; w *= 2) {
-    const int64_t tiles = m_tiles * ((p.N + w - 1) / w);
+    const int64_t tiles = m_tiles * ((N + w - 1) / w);
     const double block = w == 64 ? 0.28 : w == 128 ? 0.38 : 0.57, wide = w == 64 ? 0.0 : 0.8;
     for (int s = 1; s <= (w == 256 || m_tiles > 2 ? 1 : 4); s *= 2) {
       // (a CTA of a shared tile has one tile; clusters of four do not fill every SM)
       if (s > 1 && (tiles * s > (s == 4 ? sms - sms / 8 : sms) || kbs < 2 * s)) break;
       const double cost = (double)((tiles * s + sms - 1) / sms) * ((kbs + s - 1) / s) * block + (s > 1 ? 1.5 + 0.75 * s + (s - 1) * wide : 0.0);
-      if (cost < best) { best = cost; bn = w; p.splits = s; }
+      if (cost < best) { best = cost; bn = w; *splits = s; }
     }
   }
   return bn;
@@ -769,8 +772,7 @@ int gemm_bf16_bias_act(const void* A, int64_t lda, const void* W, int64_t ldw, v
   p.err = ctx().error_flag;
   CUtensorMap ta, tb;
   KD_TRY(make_tmap_bf16_2d(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, GEMM_BM, GEMM_BK));
-  const int64_t wide = (int64_t)((M + GEMM_BM - 1) / GEMM_BM) * ((N + 255) / 256);
-  const int bn = N >= 256 && wide * 2 > ctx().sm_count ? 256 : choose_tile(p, 64);
+  const int bn = linear_tile(M, N, K, 64, ctx().sm_count, &p.splits);
   KD_TRY(make_tmap_bf16_2d(&tb, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, bn, GEMM_BK));
   if (bn == 256) return launch_gemm<256, 4>(ta, tb, p);
   if (bn == 128) return launch_gemm<128, 6>(ta, tb, p);
@@ -819,8 +821,7 @@ int gemm_bf16_qkv_rope(const void* A, int64_t lda, const void* W, int64_t ldw, i
   p.kc_b = kc_b; p.kc_h = kc_h; p.kc_s = kc_s;
   CUtensorMap ta, tb;
   KD_TRY(make_tmap_bf16_2d(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, GEMM_BM, GEMM_BK));
-  const int64_t wide = (int64_t)((M + GEMM_BM - 1) / GEMM_BM) * ((N + 255) / 256);
-  const int bn = wide * 2 > ctx().sm_count ? 256 : choose_tile(p, 128);      // (a head of 128 columns lies in one tile)
+  const int bn = linear_tile(M, N, K, 128, ctx().sm_count, &p.splits);      // (a head of 128 columns lies in one tile)
   KD_TRY(make_tmap_bf16_2d(&tb, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, bn, GEMM_BK));
   return bn == 256 ? launch_gemm<256, 4>(ta, tb, p) : launch_gemm<128, 6>(ta, tb, p);
 }
@@ -1095,3 +1096,11 @@ int matmul_tc_try(const kd_matmul_cfg* cfg, const kd_tensor* a, const kd_tensor*
 }
 
 }  // namespace kd
+
+using namespace kd;
+
+KD_API int kd_debug_linear_plan(int64_t M, int64_t N, int64_t K, int heads_of_128, int sms, int* width, int* sharing) {
+  KD_REQUIRE(width && sharing && M > 0 && N > 0 && K > 0 && sms > 0, "bad argument");
+  *width = linear_tile(M, N, K, heads_of_128 ? 128 : 64, sms, sharing);
+  return KD_OK;
+}

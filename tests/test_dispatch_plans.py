@@ -37,3 +37,31 @@ def test_recurrences_outside_the_measured_range_take_one_kernel():
         assert ctas >= heads
         assert not (records and (tokens < 32 or ctas > 4 * SMS))
 
+
+def test_linears_share_tiles_within_one_wave():
+    """A CTA of a shared tile has one tile and at least two k-blocks, 256-wide tiles and more than two rows of tiles are not
+    shared, and a head of 128 columns lies in one tile."""
+    rng = random.Random(2)
+    shared = set()
+    for _ in range(20000):
+        M, N, K, heads = rng.choice([1, 7, 97, 128, 129, 256, 257, 700]), 8 * rng.randint(1, 1300), 8 * rng.randint(1, 1300), rng.randint(0, 1)
+        N = max(384, N // 128 * 128) if heads else N
+        w, s = _two("kd_debug_linear_plan", M, N, K, heads, SMS)
+        rows, kbs = -(-M // 128), -(-K // 64)
+        assert w in ((128, 256) if heads else (64, 128, 256)) and s in (1, 2, 4)
+        if s > 1:
+            assert w < 256 and rows <= 2 and rows * -(-N // w) * s <= SMS and kbs >= 2 * s
+            shared.add((w, s))
+    assert shared == {(64, 2), (64, 4), (128, 2), (128, 4)}
+
+
+def test_fp32_matmuls_split_k_within_one_wave():
+    rng = random.Random(3)
+    seen = set()
+    for _ in range(20000):
+        batches, M, N, K = rng.choice([1, 1, 3, 16]), rng.randint(1, 1500), rng.randint(1, 4000), 4 * rng.randint(16, 1100)
+        w, s = _two("kd_debug_matmul_f32_plan", batches, M, N, K, SMS)
+        assert w in (64, 128) and s in (1, 2, 4) and s <= -(-K // 64) and (w // 4) % s == 0
+        assert s == 1 or batches * -(-M // 128) * -(-N // w) * s <= SMS
+        seen.add((w, s))
+    assert {(64, 4), (128, 1), (128, 2), (128, 4)} <= seen

@@ -45,7 +45,7 @@ def test_linear_bf16_matches_oracle(backend, oracle, m, n, k):
 @pytest.mark.parametrize("m", [2, 128, 129, 384])
 @pytest.mark.parametrize("n,k", [(64, 192), (200, 520), (1024, 3072), (4096, 1024), (768, 136)])
 def test_linear_bf16_few_rows_share_k(backend, oracle, m, n, k):
-    """One, two and four blocks to a tile, ranges of unequal length, remainders in every dimension."""
+    """Few rows: tiles of one block each and, for the deepest K, of four (test_shared_tiles_gpu.py has every shared form)."""
     x, w = lib.round_to_bf16(synth.normal("x", (m, k))), lib.round_to_bf16(synth.normal("w", (n, k), 0.05))
     ref = oracle.linear(x, w)
     got = _linear_bf16(x, w, out_dtype="float32")

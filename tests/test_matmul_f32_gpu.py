@@ -1,9 +1,11 @@
 """fp32 matmul on the tensor cores (gemm_f32_split.cu) against float64: edges of its 128 x 64/128 x 64 tiles, K split over
 a cluster, batches, alpha / beta / C, and numbers outside the range of the split."""
+import ctypes
+
 import numpy as np
 import pytest
 
-from kandle_b200 import core
+from kandle_b200 import core, lib
 from kandle_b200.backend import CudaEvent
 from kandle_b200.core import Tensor
 
@@ -102,3 +104,45 @@ def test_matmul_f32_products_near_the_least_number(backend, m, n, k, sa, sb):
     exact = a.astype(np.float64) @ b.astype(np.float64).T
     step = 0.5 * np.sqrt(k) * (2.0 ** -149 + 2.0 ** -24 * np.sqrt((exact ** 2).mean()))
     assert np.sqrt(((got - exact) ** 2).mean()) <= step
+
+
+def _plan(batches, m, n, k):
+    w, s = ctypes.c_int(0), ctypes.c_int(0)
+    lib.call("kd_debug_matmul_f32_plan", batches, m, n, k, 148, ctypes.byref(w), ctypes.byref(s))
+    return w.value, s.value
+
+
+# 19, 10, 34, 18 k-blocks: ranges of unequal length, zeros behind the last numbers of K in the last range
+@pytest.mark.parametrize("batches,m,n,k,plan", [(1, 130, 3000, 1160, (128, 2)), (3, 130, 1000, 584, (128, 2)), (1, 60, 100, 2116, (64, 4)), (1, 300, 1000, 1100, (128, 4))])
+def test_matmul_f32_split_over_a_cluster(backend, batches, m, n, k, plan):
+    assert _plan(batches, m, n, k) == plan
+    a, b, c = _rand((batches, m, k), 14), _rand((batches, n, k), 15), _rand((n,), 16)
+    exact = a.astype(np.float64) @ b.astype(np.float64).transpose(0, 2, 1)
+    bound = np.stack([_bound(x, y) for x, y in zip(a, b)])
+    assert (np.abs(core.matmul(Tensor(a), Tensor(b), transposeB=True, alpha=0.5).dataAsync() - 0.5 * exact) <= bound).all()
+    assert (np.abs(core.linear(Tensor(a[0]), Tensor(b[0]), Tensor(c)).dataAsync() - exact[0] - c) <= 2 * bound[0]).all()
+    a[0, 7, 3], a[0, m - 1, k - 1] = 1e-36, np.inf      # a range below the split's numbers, and one row that is not finite
+    got = core.matmul(Tensor(a), Tensor(b), transposeB=True).dataAsync()
+    with np.errstate(all="ignore"):
+        exact = a.astype(np.float64) @ b.astype(np.float64).transpose(0, 2, 1)
+    assert not np.isfinite(got[0, m - 1]).any() and np.array_equal(got[0, m - 1] > 0, exact[0, m - 1] > 0)
+    exact[0, m - 1] = got[0, m - 1] = 0
+    assert (np.abs(got - exact) <= 16 * bound).all()
+
+
+def test_matmul_f32_out_of_range_in_late_tiles(backend):
+    """More tiles than multiprocessors: a CTA's second and third tile, and none of the others."""
+    m, n, k = 2500, 2400, 128
+    assert _plan(1, m, n, k)[1] == 1 and -(-m // 128) * -(-n // 128) > 2 * 148
+    a, b = _rand((m, k), 17), _rand((n, k), 18)
+    clean = core.matmul(Tensor(a), Tensor(b), transposeB=True).dataAsync()
+    bad = a.copy()
+    bad[1900, 5], bad[2400, 60] = 1e-38, np.inf
+    got = core.matmul(Tensor(bad), Tensor(b), transposeB=True).dataAsync()
+    exact = a.astype(np.float64) @ b.astype(np.float64).T
+    exact[1900] -= a[1900, 5].astype(np.float64) * b[:, 5]
+    assert not np.isfinite(got[2400]).any()
+    exact[2400] = got[2400] = 0
+    assert (np.abs(got - exact) <= 16 * _bound(a, b)).all()
+    rows = [i for i in range(m) if i // 128 not in (1900 // 128, 2400 // 128)]
+    assert np.array_equal(got[rows], clean[rows])
