@@ -144,7 +144,9 @@ int kd_flash_attention(const kd_tensor* q, const kd_tensor* k, const kd_tensor* 
 /* Key `matmul` (cfg, a, b): MatmulDispatchResult,
  * packages/core/src/dispatch/matmulOps.ts:32-125; executor
  * packages/backend-webgpu/src/kernels/matrix/executor.ts:47-76,438-598.
- * out = beta*c + alpha*op(a)*op(b); batch dims broadcast; full strides honoured. */
+ * out = beta*c + alpha*op(a)*op(b); batch dims broadcast; full strides honoured.  fp32 operands whose K is contiguous are
+ * multiplied on the tensor cores in three bf16 parts each, with less error than a chain of fp32 multiply-adds; K is summed
+ * in ranges where the tiles are few, in a fixed order. */
 typedef struct kd_matmul_cfg {
   int64_t M, N, K;
   int32_t transpose_a, transpose_b; /* stored last two dims are [K,M] / [N,K] when set */
@@ -277,7 +279,11 @@ typedef enum kd_epilogue {
                           weight rows interleave 16 gate rows / 16 up rows per 32-row block      */
 } kd_epilogue;
 /* `linear` on the tensor cores (tcgen05): x [tokens,K] bf16, weight [N,K] bf16 (K-major, as
- * composite.ts:62-70 passes it), out [tokens,N] (or [tokens,N/2] for SWIGLU) bf16 or fp32. */
+ * composite.ts:62-70 passes it), out [tokens,N] (or [tokens,N/2] for SWIGLU) bf16 or fp32.
+ * The same call gives the same bits every time.  The order of a row's fp32 sums follows from the sizes: here and in
+ * the linears below (kd_linear_bf16_bias, kd_qkv_linear_norm_rope_cachewrite, kd_linear_ex, kd_linear_tanh,
+ * kd_linear_glu) calls of up to 256 tokens may sum K in two or four ranges, so a row can differ by fp32 roundings
+ * (after the rounding of the output: by one of its steps) from the same row among more tokens. */
 int kd_linear_bf16(const kd_tensor* x, const kd_tensor* weight, const kd_tensor* residual, int epilogue,
                    const kd_tensor* out);
 typedef enum kd_activation { KD_ACT_NONE = 0, KD_ACT_GELU = 1 } kd_activation;
@@ -612,7 +618,10 @@ int kd_latent_prefill(const kd_tensor* proj, int q_col, int heads, int dim, int 
  * with dt_bias [heads]; neg_rate = -exp(A_log) [heads], history [B,taps-1,channels] (q, k, v channels
  * side by side, the inputs before this call), state fp32 [B,heads,rows,cols] as kd_delta_state_shape says, updated in
  * place; out fp32 [T, heads*vdim].  The history is moved on by kd_delta_out, which divides every head's output by its root
- * mean square, multiplies by norm_weight [vdim] and the activated gate (kd_gate), and writes proj's type. */
+ * mean square, multiplies by norm_weight [vdim] and the activated gate (kd_gate), and writes proj's type.
+ * Calls of 32 tokens and more with few heads (kd_debug_recurrence_plan) keep up to 64 MB of intermediate values in the
+ * library's scratch buffer (kd_workspace_bytes), more with hundreds of heads of few value channels; where it cannot be had,
+ * they take the form without.  The two forms and other cuts of a prompt differ by fp32 roundings.  kd_wkv likewise. */
 typedef enum kd_gate { KD_GATE_SIGMOID = 0, KD_GATE_SILU = 1 } kd_gate;
 int kd_delta_rule(const kd_tensor* proj, int q_col, int k_col, int v_col, int b_col, const kd_tensor* decay, int heads, int kv_heads,
                   int dim, int vdim, const kd_tensor* conv_q, const kd_tensor* conv_k, const kd_tensor* conv_v,

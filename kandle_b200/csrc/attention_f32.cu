@@ -1,4 +1,4 @@
-// Key `flash_attention`, exact-fp32 path on the CUDA cores (any storage dtype, fp32 math).
+// Key `flash_attention`, fp32 path on the CUDA cores (any storage dtype, fp32 math).
 //
 // Two kernels: attention_f32_tile_kernel for fp32 operands with heads of 64 or 128 channels in rows of 16-byte pieces,
 // attention_f32_kernel for everything else.
@@ -108,7 +108,8 @@ __global__ void __launch_bounds__(ATT_WARPS * 32) attention_f32_kernel(const voi
 // attention_f32_kernel passes over (all masked, or past the end) are passed over here too: infinities among masked values
 // stay out of the sums.
 // Bound: shared-memory reads, (R + 4) 16-byte reads for 16 R multiply-adds; attention_f32_kernel, one row a warp, reads two
-// numbers a multiply-add.  16 heads of 128 channels, causal: 128 queries 14.5 us (30.8 before), 512 queries 61.6 us (254).
+// numbers a multiply-add.  16 heads of 128 channels, causal, replayed from a graph: 128 queries 12.3 us (28.5 before), 300 33.9
+// (108), 1000 136 (803); launched one by one 128 queries take 14.5.
 template <int D, int R>
 __global__ void __launch_bounds__(128) attention_f32_tile_kernel(const float* __restrict__ Q, const float* __restrict__ K, const float* __restrict__ V,
                                                                  float* __restrict__ O, AttnParams p) {
@@ -272,8 +273,8 @@ static bool attention_tile_fits(const void* pq, const void* pk, const void* pv, 
 template <int D>
 static int launch_attention_tile_rows(const void* pq, const void* pk, const void* pv, void* po, const AttnParams& p) {
   // Rows a CTA: 32 (half the key reads a row) where there are more than 16 and that leaves a CTA for every SM, 16 otherwise.
-  // Causal, heads of 128: 16 heads of 128 queries 14.5 us with 16 rows, 16.5 with 32; 64 heads of 512 queries 215 and 148 us
-  // (64 rows: 178).  256 heads of 64, one query, one key: 4.9 us with 16 rows, 6.1 with 32 (attention_f32_kernel 5.0).
+  // Causal, heads of 128, launched one by one: 16 heads of 128 queries 14.5 us with 16 rows, 16.5 with 32; 64 heads of 512
+  // queries 215 and 148 us (64 rows: 178).  256 heads of 64, one query, one key: 4.9 us with 16 rows, 6.1 with 32 (attention_f32_kernel 5.0).
   if (p.Sq > 16 && (int64_t)p.Hq * p.B * ((p.Sq + 31) / 32) >= ctx().sm_count) return launch_attention_tile<D, 4>(pq, pk, pv, po, p);
   return launch_attention_tile<D, 2>(pq, pk, pv, po, p);
 }
@@ -330,7 +331,7 @@ int attention_f32_dispatch(const kd_tensor* q, const kd_tensor* k, const kd_tens
   KD_REQUIRE(p.Hq <= 65535 && p.B <= 65535, "flash_attention: too many heads or batches for one launch");
   KD_REQUIRE(p.D >= 1, "flash_attention: empty head dimension");
   // A few rows of heads of 128 against a few keys: the general kernel is through sooner (16 heads, one query: 1 key 5.4 us,
-  // 5.9 in tiles; 4 keys 5.5, 5.9; 8 keys 5.9, 5.9; 256 heads, 1 key: 10.0, 6.6)
+  // 5.9 in tiles; 4 keys 5.5, 5.9; 8 keys 5.8, 5.9; 256 heads, 1 key: 10.0, 7.9)
   const bool few = p.D == 128 && p.Skv <= 6 && p.Sq <= ATT_WARPS && (int64_t)p.Hq * p.B <= ctx().sm_count;
   if (!few && attention_tile_fits(pq, pk, pv, po, p))
     return p.D == 64 ? launch_attention_tile_rows<64>(pq, pk, pv, po, p) : launch_attention_tile_rows<128>(pq, pk, pv, po, p);

@@ -9,8 +9,9 @@
 // fp32, so a chunked form on the tensor cores needs split operands (three products for one), a
 // triangular solve per chunk and per-channel decays inside every product.  Counted in instructions
 // that is no cheaper than the recurrence itself when the state lives in registers and the arithmetic
-// is packed (fma.rn.f32x2: two per lane and instruction).  And the result does not depend on where a
-// prompt is cut beyond the rounding of the decay products.
+// is packed (fma.rn.f32x2: two per lane and instruction).  A prompt's result depends on where it is cut, and on the
+// number of heads beside it, by fp32 roundings alone: of the decay products, and of sums that the form for few heads
+// associates in another order (three parts in 10^7 of an output at 300 tokens).
 //
 // Mapping.  A state column (one value channel) never meets another one, so a warp owns 32 / LPC
 // groups of 8 columns, and the LPC lanes of a group share its dim rows (16 rows a lane, in quads
@@ -25,7 +26,7 @@
 // next block of tokens (convolution, silu, unit norms, decays, step sizes) in shared memory while the
 // consumers walk through the current one.
 // That form needs a head for every SM: one sequence of 8192 tokens and 16 heads took 5.67 ms, 64 CTAs walking 1300 cycles
-// a token.  Calls with few heads take delta_prepare_kernel and recurrence_kernel instead (recurrence.cuh): 1.55 ms.
+// a token.  Calls with few heads take delta_prepare_kernel and recurrence_kernel instead (recurrence.cuh, which has the rule): 1.55 ms.
 // Bound: fp32 pipe in prefill (3.25 dim vdim multiply-adds per head and token), HBM in decode
 // (the state is read and written once per token: 8 dim vdim bytes per head and sequence).
 #include "common.cuh"

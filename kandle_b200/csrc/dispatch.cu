@@ -1,5 +1,5 @@
-// Entry points that choose between the exact-fp32 CUDA-core kernels and the bf16 tensor-core
-// kernels: `matmul`, `flash_attention`, `conv1d`.
+// Entry points that choose between the fp32 kernels (K-major matmuls in three bf16 parts on the tensor cores, the rest on
+// the CUDA cores) and the bf16 tensor-core kernels: `matmul`, `flash_attention`, `conv1d`, linears.
 #include "common.cuh"
 #include "kernels.cuh"
 
@@ -257,7 +257,7 @@ KD_API int kd_linear_ex(const kd_tensor* x, const kd_tensor* weight, const kd_te
       return gemm_bf16_bias_act(px, ldx, pw, K, po, ldo, f32, pr, N, (int)M, (int)N, (int)K, residual ? KD_EPI_RESIDUAL : KD_EPI_NONE, nullptr, 0,
                                 (float*)pt, tail ? (int)n_out : 0, tail ? tail->shape[1] : 0);
   }
-  // exact fp32, and sizes the tensor-core kernels do not take
+  // fp32, and sizes the bf16 kernels do not take
   for (int part = 0; part < (tail ? 2 : 1); ++part) {
     kd_tensor w = *weight;
     w.shape[0] = part ? N - n_out : n_out;

@@ -27,7 +27,8 @@
 //                (warps 17-19 idle: registers move between groups of four warps)
 // Bound: the split, about 35 instructions per 4 numbers of either operand and 1.8 us per 128 x 128 x 64 block, against
 // 0.8 us of MMA.  2048 x 4096 x 4096 takes 463 us = 148 TFLOP/s; matmul_f32_kernel reaches about 9.  Where the tiles
-// are too few for the SMs, K is shared: a cluster of 2 or 4 CTAs, each a range of k-blocks, adds its sums up through shared memory in a fixed order.
+// are too few for the SMs, K is shared: a cluster of 2 or 4 CTAs, each a range of k-blocks, adds its sums up through shared
+// memory in a fixed order.
 #include "common.cuh"
 #include "kernels.cuh"
 #include "sm100.cuh"

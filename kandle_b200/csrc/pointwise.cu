@@ -124,7 +124,9 @@ __global__ void pointwise_contig_kernel(const T* __restrict__ a, const T* __rest
 // dimensions merged where all operands allow it.  HBM-bound; pointwise_strided_kernel, one element a thread and a 64-bit
 // division per dimension, took 325 us to widen 65536 x 1024 bf16 numbers (403 MB), and 10.5 us for the 2 MB slices, head
 // permutations and broadcast products of rotary embeddings.
-struct FastDiv {      // n / d for n < 2^31 by a multiplication
+// n / d for n < 2^31 by a multiplication: division by an invariant integer after Granlund and Montgomery (1994), the
+// multiplier rounded up.
+struct FastDiv {
   uint32_t d, mul, shift;
   __device__ __forceinline__ uint32_t operator()(uint32_t n) const { return (__umulhi(n, mul) + n) >> shift; }
 };
