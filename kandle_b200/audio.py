@@ -6,7 +6,6 @@ kernel, the 400-point DFT as an fp32 GEMM with a precomputed basis, power, mel p
 log10 / clamp / scale step the reference runs in a host loop."""
 from __future__ import annotations
 
-import ctypes
 import math
 
 import numpy as np
@@ -18,7 +17,7 @@ WHISPER_AUDIO_CONFIG = {"SAMPLE_RATE": 16000, "N_FFT": 400, "HOP_LENGTH": 160, "
 
 
 def _r(t):
-    return ctypes.byref(t._handle.c()) if t is not None else None
+    return t._handle.ref() if t is not None else None
 
 
 def hann_window_host(window_length: int, periodic: bool | None = None) -> np.ndarray:

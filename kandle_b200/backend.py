@@ -101,7 +101,7 @@ class CudaTensorHandle:
         self.memoryFormat = memoryFormat
         self.id = next(_ids)
         self._disposed = False
-        self._packed_for = self._packed = None
+        self._described = None
 
     # --- metadata
     @property
@@ -138,16 +138,23 @@ class CudaTensorHandle:
         self.storage.incRef()
         return CudaTensorHandle(self.storage, shape, self.dtype, strides, offset)
 
-    def c(self) -> kd_tensor:
+    def ref(self):
+        """The descriptor by reference, for calls that only read it: they share one, made again when the metadata changed."""
         if self._disposed or self.storage.isDisposed:
             raise RuntimeError("tensor handle used after dispose()")
         now = (self.storage.handle, self.offset, self.dtype, self.shape, self.strides)
-        if now != self._packed_for:      # the bytes are kept with what they were packed from
+        if now != self._described:
             shape, strides = self.shape, self.strides
-            self._packed = _TENSOR.pack(self.storage.handle, self.offset, DTYPES[self.dtype][0], len(shape),
-                                        *shape, *_PAD[len(shape)], *strides, *_PAD[len(strides)])
-            self._packed_for = now
-        return kd_tensor.from_buffer_copy(self._packed)      # the caller's own
+            self._shared = kd_tensor.from_buffer_copy(_TENSOR.pack(self.storage.handle, self.offset, DTYPES[self.dtype][0], len(shape),
+                                                                   *shape, *_PAD[len(shape)], *strides, *_PAD[len(strides)]))
+            self._by_ref = ctypes.byref(self._shared)
+            self._described = now
+        return self._by_ref
+
+    def c(self) -> kd_tensor:
+        """A descriptor of the caller's own."""
+        self.ref()
+        return kd_tensor.from_buffer_copy(self._shared)
 
     # --- readback
     def dataAsync(self) -> np.ndarray:
@@ -158,7 +165,7 @@ class CudaTensorHandle:
         tmp = None
         if not (self.isContiguous()):
             tmp = CudaBackend.instance().createTensorHandle(self.shape, self.dtype, clear=False)
-            lib.call("kd_copy", ctypes.byref(tmp.c()), ctypes.byref(self.c()))
+            lib.call("kd_copy", tmp.ref(), self.ref())
             h = tmp
         code, esz, npdt = DTYPES[self.dtype]
         out = np.empty(self.shape, dtype=npdt)

@@ -36,7 +36,7 @@ from .model_utils.qwen3 import Qwen3Config
 
 
 def _r(t):
-    return ctypes.byref(t._handle.c()) if t is not None else None
+    return t._handle.ref() if t is not None else None
 
 
 def interleave_gate_up(gate: np.ndarray, up: np.ndarray) -> np.ndarray:

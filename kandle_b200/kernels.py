@@ -21,7 +21,7 @@ from .lib import POINTWISE_OPS, kd_matmul_cfg
 
 
 def _ref(h):
-    return ctypes.byref(h.c()) if h is not None else None
+    return h.ref() if h is not None else None
 
 
 @dataclass

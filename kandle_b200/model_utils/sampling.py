@@ -29,7 +29,7 @@ class SampleResult:                       # index.ts:60-72
 
 
 def _r(t):
-    return ctypes.byref(t._handle.c()) if t is not None else None
+    return t._handle.ref() if t is not None else None
 
 
 def sample(logits: Tensor, config: SamplerConfig | None = None, displayTopK: int = 0, uniform: float | None = None,

@@ -35,7 +35,7 @@ KD_ACT_NONE, KD_ACT_GELU = 0, 1
 
 
 def _r(t):
-    return ctypes.byref(t._handle.c()) if t is not None else None
+    return t._handle.ref() if t is not None else None
 
 
 class WhisperEncoderEngine:

@@ -124,5 +124,7 @@ def test_descriptors_belong_to_their_caller():
     t.shape[0], t.offset = 99, 5
     again = h.c()
     assert (again.storage, again.offset, again.ndim, list(again.shape[:3]), list(again.strides[:2])) == (7, 0, 2, [2, 3, 0], [3, 1])
+    shared = h.ref()
+    assert h.ref() is shared and shared._obj.shape[0] == 2
     h.offset, h.shape = 4, (1, 3)
-    assert (h.c().offset, h.c().shape[0], again.offset) == (4, 1, 0)
+    assert (h.c().offset, h.c().shape[0], h.ref()._obj.offset, again.offset) == (4, 1, 4, 0)
