@@ -7,6 +7,8 @@
 // holds rows (i LPC + j) 4 + e (i < 4, e < 4), as s[column][row pair].  State in memory is
 // [B, heads, rows, columns] with rows = 16 LPC and columns padded to a multiple of 8.
 #pragma once
+#include <type_traits>
+
 #include "common.cuh"
 #include "sm100.cuh"
 
@@ -151,9 +153,10 @@ __device__ __forceinline__ void group_sums(int j, float (&x)[8], float (&y)[8]) 
 }
 
 // ----------------------------------------------------------------------------- few heads
-// Where the heads of a call leave most of the chip idle, a prompt takes two kernels.  The layer's own prepare kernel turns every four tokens of a head into one record of what the
-// walk needs (the vectors with the decays in them, and the 4 x 4 products between the tokens), all tokens side by side; then
-// recurrence_kernel walks through the records with the state in registers:
+// Where the heads of a call leave most of the chip idle (REC_LEAST_TOKENS has the rule), a prompt takes two kernels.  The
+// layer's own prepare kernel turns every four tokens of a head into one record of what the walk needs (the vectors with the
+// decays in them, and the 4 x 4 products between the tokens), all tokens side by side; then recurrence_kernel walks through
+// the records with the state in registers:
 //   read     D = S^T k_t, O = S^T q_t for all four tokens at once, against the state before them
 //   solve    u_t = beta_t (v_t - D_t - sum_{s<t} (k_t . k_s) u_s)   (WKV: u_t = v_t)
 //   output   o_t = O_t + sum_{s<=t} (q_t . k_s) u_s
@@ -329,7 +332,11 @@ recurrence_kernel(RecStream p) {
   };
   bool ok = __all_sync(0xffffffffu, sm100::mbar_wait(&full[0], 0, abort_flag, p.err, 232));
   if (ok) fetch(sm);
-  for (int g = 0, at = 0; ok && g < p.groups; ++g) {
+  int at = 0;
+  // One record.  RAGGED: the last of a prompt, with tokens past the end.  A copy of the code: the masks cost every record 3 %
+  // (8192 tokens, 16 heads of 128: 1538 us, 1589 with masks), the copy a call that needs it 1.3 us.
+  auto walk = [&](int g, auto ragged) {
+    constexpr bool RAGGED = decltype(ragged)::value;
     const float* base = sm + stage * stage_floats;
     const float* rec = base + at * REC;
     const float* kw = rec + QV + 4 * DK;
@@ -373,8 +380,8 @@ recurrence_kernel(RecStream p) {
           u[2][c] = beta.z * ((v.z - u[2][c]) - fmaf(m1.z, u[1][c], m0.z * u[0][c]));
           u[3][c] = beta.w * ((v.w - u[3][c]) - fmaf(m2.w, u[2][c], fmaf(m1.w, u[1][c], m0.w * u[0][c])));
         }
-        // (a group's tokens past the end of the prompt write nothing, not even zero times an infinity)
-        if (t0 + 4 > p.S) {
+        // (tokens past the end write nothing, not even zero times an infinity)
+        if constexpr (RAGGED) {
 #pragma unroll
           for (int t = 1; t < 4; ++t)
 #pragma unroll
@@ -455,7 +462,11 @@ recurrence_kernel(RecStream p) {
     }
     stage = next_stage;
     phase = next_phase;
-  }
+  };
+  const int whole = DELTA && p.t0 + p.groups * 4 > p.S ? p.groups - 1 : p.groups;      // (WKV: zero values, no masks)
+  for (int g = 0; ok && g < whole; ++g) walk(g, std::false_type());
+  if constexpr (DELTA)
+    if (ok && whole < p.groups) walk(whole, std::true_type());
 #pragma unroll
   for (int c = 0; c < C; ++c)
 #pragma unroll
@@ -469,9 +480,11 @@ recurrence_kernel(RecStream p) {
         }
 }
 
-// Bytes of records that a portion of a prompt may take: they are written and read back inside the L2 cache.
+// Bytes of records that a portion of a prompt may take: they are written and read back inside the L2 cache.  They lie in the
+// library's workspace, which the first such call grows to 96 MB (1.5 times) for good.
 constexpr int64_t REC_SCRATCH = 64 << 20;
-// ... but at least this many groups a portion, or loading and storing the states would count.
+// ... but at least this many groups a portion, or loading and storing the states would count (that is below
+// REC_SCRATCH but for many heads of few value channels: 321 MB for 592 heads of 256 key and 16 value channels).
 constexpr int REC_LEAST_GROUPS = 32;
 
 // Least tokens of a call that take records, by [delta rule][16-bit inputs][key channels 32, 64, 128, 256][CTAs of the walk
