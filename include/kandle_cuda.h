@@ -478,6 +478,25 @@ int kd_decode_layer_fused(const kd_tensor* attn, const kd_tensor* w_o, const kd_
                           const kd_tensor* sin, const kd_tensor* pos, const kd_tensor* k_cache_next,
                           const kd_tensor* v_cache_next, const kd_tensor* block_table, const kd_tensor* q_out,
                           const kd_tensor* resid_out, const kd_tensor* x_final);
+/* A whole decode step of a few sequences as one persistent kernel: embedding rows of `ids`, every layer (QKV, q/k-norm, rotary
+ * embedding, cache write, attention over the cache, o_proj, SwiGLU MLP), the final norm and the lm_head over the embedding
+ * table (packages/model-utils/src/qwen3/for_causal_lm.ts:170-194,475-508).  Advances *pos and *ctx_len by one when it is done.
+ *   layer_tensors   per layer: input norm [H], W_qkv [(Hq+2Hkv)128,H], q norm [128], k norm [128], W_o [H,Hq*128], post norm [H],
+ *                   W_gate_up [2I,H] (16 gate rows, 16 up rows in turn), W_down [H,I], K cache, V cache; bf16, contiguous
+ *                   (caches: [B>=M,Hkv,maxS,128], or pools [pages,Hkv,128,128] with block_table int32 [B>=M,max_pages])
+ *   ids int64 [M], inv_freq fp32 [64], pos and ctx_len int32 scalars on the device, logits fp32 [M,V]
+ *   state           this caller's own hand-over words: kd_decode_step_state_bytes bytes, zero before the first step and then
+ *                   left alone; steps that may run at the same time need a state each
+ * kd_decode_step_state_bytes gives 0 for shapes that this form does not take: it takes 1 to 6 sequences whose activations
+ * fit shared memory beside the weights on their way, head_dim 128, 1, 2 or 4 query heads to a KV head, up to 64 layers, and
+ * widths that are multiples of 512 with at least one row per CTA (`grid` CTAs; 0: this device's).  A token outside the table is taken as zeros (code 101), a
+ * cache row outside [0, maxS) is not written (code 102), a wait that runs out reports 541-545.  Results are bit-identical from
+ * launch to launch; the order of the sums over keys follows the number of sequences and the position. */
+int kd_decode_step_state_bytes(int sequences, int hidden, int inter, int q_heads, int kv_heads, int head_dim, int vocab, int layers,
+                               int grid, uint64_t* bytes_out);
+int kd_decode_step(const kd_tensor* const* layer_tensors, int n_layers, const kd_tensor* embed, const kd_tensor* final_norm,
+                   const kd_tensor* ids, const kd_tensor* inv_freq, const kd_tensor* pos, const kd_tensor* ctx_len, float eps,
+                   float scale, const kd_tensor* block_table, const kd_tensor* state, const kd_tensor* logits);
 /* The tensor-parallel form (no counterpart in the reference): every rank passes ITS slices (W_o and
  * W_down: input columns; W_gate_up and W_qkv_next: rows; attn, caches and q_out: its heads) and the
  * same residual; the partial sums of o_proj and down_proj are exchanged INSIDE the kernel, unit by

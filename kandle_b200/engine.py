@@ -243,6 +243,8 @@ class Qwen3Engine(DecoderEngine):
         # (tensor parallel: the form of that kernel that exchanges the partial sums of o_proj and down_proj
         # with its peers inside the kernel, when the peer buffers are connected)
         self.use_fused_layer = self.D == 128 and self.H <= 8192
+        # ... and for a few sequences the whole step, lm_head included, as one kernel (kd_decode_step)
+        self.use_step_kernel = True
         # tensor parallel decode: sum the partial outputs over ranks through mapped peer memory when
         # the host program has connected the peer buffers (parallel.init_peer_buffers), else NCCL
         self.use_p2p = True
@@ -456,10 +458,24 @@ class Qwen3Engine(DecoderEngine):
         if self.use_chain and not self.use_fused_layer:
             d["qkv_p"].dispose()
             d["qkv_p"] = f(chain_splits(self.nqkv, self.H), B, self.nqkv)
+        d["step"] = self._step_kernel_state(B)
         d["pos"] = d["scalars"].slice([slice(0, 1)])
         d["ctx"] = d["scalars"].slice([slice(1, 2)])
         self._decode = d
         return d
+
+    def _step_kernel_state(self, B: int):
+        """What kd_decode_step needs beside a step's buffers (hand-over words, the layers' descriptors), or None where it
+        does not take the shape."""
+        c, n = self.cfg, ctypes.c_uint64(0)
+        if self.tp == 1 and self.use_fused_layer and self.use_step_kernel:
+            lib.call("kd_decode_step_state_bytes", B, self.H, self.I, self.Hq, self.Hkv, self.D, self.V, self.L, 0, ctypes.byref(n))
+        if not n.value:
+            return None
+        names = ("in_norm", "wqkv", "q_norm", "k_norm", "wo", "post_norm", "wgu", "wdown")
+        parts = [t for i, lw in enumerate(self.layers) for t in [lw[k] for k in names] + [self.k_cache[i], self.v_cache[i]]]
+        kept = [t._handle.c() for t in parts]
+        return {"words": core.zeros((n.value // 4,), "int32"), "kept": kept, "layers": (ctypes.POINTER(lib.kd_tensor) * len(kept))(*map(ctypes.pointer, kept))}
 
     def _enqueue_decode_step(self, d: dict) -> None:
         """One decode step for d['ids'] at device position d['pos']; leaves the next ids in d['ids']."""
@@ -475,6 +491,13 @@ class Qwen3Engine(DecoderEngine):
     def _decode_step_kernels(self, d: dict) -> None:
         c, B = self.cfg, d["B"]
         eps = ctypes.c_float(c.rmsNormEps)
+        if d["step"] is not None:
+            lib.call("kd_decode_step", d["step"]["layers"], self.L, _r(self.embed), _r(self.final_norm), _r(d["ids"]), _r(self.inv_freq), _r(d["pos"]),
+                     _r(d["ctx"]), eps, ctypes.c_float(self.scale), _r(self.block_table), _r(d["step"]["words"]), _r(d["logits"]))
+            lg = d["logits"].view(B, self.V)
+            self._next_tokens(lg, d["uniforms"], d["ids"])
+            lg.dispose()
+            return
         core._kernel("index_select")(self.embed._handle, d["ids"]._handle, {"dim": 0}, d["emb"]._handle)
         core.copy_(d["h"], d["emb"])
         lib.call("kd_rope_table", _r(self.inv_freq), _r(d["pos"]), 0, 1, _r(d["cos"]), _r(d["sin"]))
