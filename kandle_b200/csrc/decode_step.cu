@@ -24,9 +24,10 @@
 // rows of one operand in shared memory and a trip through tensor memory, which here only adds latency: an SM multiplies
 // 830 such tiles a layer, under 2 % of its time.
 //
-// Measured on B200, Qwen3-0.6B without the lm_head, us a step at a context of 300 (kernels per layer in brackets): 1 sequence 443
-// (1042), 2 478 (1061), 4 584 (1069), 6 752 (1102); 4B widths, 9 layers: 1 473 (687), 2 554 (685).  7 and 8 sequences, where
+// Measured on B200, Qwen3-0.6B without the lm_head, us a step at a context of 300 (kernels per layer in brackets): 1 sequence 446
+// (1042), 2 478 (1061), 4 584 (1069), 6 757 (1102); 4B widths, 9 layers: 1 472 (687), 2 554 (685).  7 and 8 sequences, where
 // registers run out, were 943 and 985 (1091, 1102) there and slower than the kernels per layer at 1200 keys: not taken.
+// Contexts that one CTA takes whole and keys of a split: 96 and 32 (446 us at 300 keys; 96 and 96: 464, 192 and 96: 464).
 //
 // All CTAs wait for one another, so the launch is cooperative, and every wait is bounded (codes 541-545): a CTA that
 // gives up goes on to the end without waiting, so that the step's ticket and tag stay in order.
@@ -278,11 +279,17 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
         if (!attends) continue;
         for (int key = keys.k0; ok && key < keys.k1; key += DS_KEYS) {
           const int n = min(DS_KEYS, keys.k1 - key), begin = claim(2, (uint32_t)n * 512u);
-          if (begin >= 0 && lane < n && lane % DS_COPY_WARPS == copier) {
+          if (begin < 0) break;
+          // one copy of keys and one of values where the rows lie side by side (8000 keys, 6 sequences: a copy per row kept the
+          // step at 3.2 ms)
+          const bool whole = p.kc_s == 128 && (!p.table || key % 128 + n <= 128);
+          if (whole ? lane == 0 && copier < 2 : lane < n && lane % DS_COPY_WARPS == copier) {
             const int64_t row = ds_cache_row(p, att_b, att_g, key + lane);
             uint64_t* bar = &full[(stage - 1) % DS_BARS];
-            bulk_load(smem + begin * DS_UNIT + lane * 256, w.kc + row, 256, bar);
-            bulk_load(smem + (begin + 1) * DS_UNIT + lane * 256, w.vc + row, 256, bar);
+            uint8_t* to = smem + begin * DS_UNIT + lane * 256;
+            const uint32_t bytes = whole ? n * 256u : 256u;
+            if (!whole || copier == 0) bulk_load(to, w.kc + row, bytes, bar);
+            if (!whole || copier == 1) bulk_load(to + DS_UNIT, w.vc + row, bytes, bar);
           }
         }
         continue;

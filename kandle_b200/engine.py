@@ -466,9 +466,11 @@ class Qwen3Engine(DecoderEngine):
 
     def _step_kernel_state(self, B: int):
         """What kd_decode_step needs beside a step's buffers (hand-over words, the layers' descriptors), or None where it
-        does not take the shape."""
-        c, n = self.cfg, ctypes.c_uint64(0)
-        if self.tp == 1 and self.use_fused_layer and self.use_step_kernel:
+        does not take the shape.  Its attention reads the cache at two thirds of the rate of kd_attention_decode: with six
+        sequences it is ahead up to 5000 keys (step of the 0.6B model: 0.76 ms against 1.10 at 300 keys, 1.1 against 1.3 at
+        2200, 2.2 against 2.0 at 8000), with one at any length (0.71 against 1.53 at 8000)."""
+        n = ctypes.c_uint64(0)
+        if self.tp == 1 and self.use_fused_layer and self.use_step_kernel and B * self.max_seq_len <= 32768:
             lib.call("kd_decode_step_state_bytes", B, self.H, self.I, self.Hq, self.Hkv, self.D, self.V, self.L, 0, ctypes.byref(n))
         if not n.value:
             return None
