@@ -361,7 +361,7 @@ int kd_increment_i32(const kd_tensor* scalar, int delta);
 
 /* CUDA-graph capture of everything enqueued between begin and end (no counterpart in the
  * reference, whose per-op host overhead is what this removes). */
-/* Enables programmatic dependent launch for the kernels of the decode step (they all begin with a
+/* Enables programmatic dependent launch for the kernels of the engines (they all begin with a
  * grid-dependency wait), so that each kernel's launch latency overlaps its predecessor.
  * enabled = 2 additionally lets kd_attention_decode[_paged/_noalloc] read the context length and
  * fetch the K/V tiles that do not hold the LAST position (context length - 1) BEFORE its
@@ -371,7 +371,9 @@ int kd_increment_i32(const kd_tensor* scalar, int delta);
  * earlier cache rows must date from launches that are separated from the call by at least one
  * kernel of this library other than the fused layer kernel and the decode attention itself
  * (every other kernel passes its grid-dependency wait before it lets its successor start).  A decode step that writes one new
- * row per layer, as Qwen3Engine's does, satisfies this. */
+ * row per layer, as Qwen3Engine's does, satisfies this.
+ * enabled = 3 (prompts): as 1, and the linears fetch their first matrix tiles before the wait.  The caller then promises that no
+ * matrix operand of a linear was written by the launch directly before it. */
 int kd_set_pdl(int enabled);
 int kd_graph_begin(void);
 int kd_graph_end(uint64_t* graph_out);
@@ -478,6 +480,19 @@ int kd_decode_layer_fused(const kd_tensor* attn, const kd_tensor* w_o, const kd_
                           const kd_tensor* sin, const kd_tensor* pos, const kd_tensor* k_cache_next,
                           const kd_tensor* v_cache_next, const kd_tensor* block_table, const kd_tensor* q_out,
                           const kd_tensor* resid_out, const kd_tensor* x_final);
+/* All layers of a prompt (packages/model-utils/src/qwen3/decoder_layer.ts:191-241), enqueued by one call: per layer kd_add_rmsnorm,
+ * kd_qkv_linear_norm_rope_cachewrite, kd_flash_attention, kd_linear_bf16 (+ residual), kd_add_rmsnorm, kd_linear_bf16 (SwiGLU) and
+ * kd_linear_bf16 (+ residual).  layer_tensors as in kd_decode_step (contiguous caches [>=B,Hkv,>=S,128]); x [B*S,H] bf16, h (the
+ * residual stream, in and out) and h1 [B*S,H] fp32, q and attn [B,S,Hq,128], act [B*S,I], cos and sin [S,64]. */
+int kd_qwen3_prompt_layers(const kd_tensor* const* layer_tensors, int n_layers, const kd_tensor* x, const kd_tensor* h, const kd_tensor* h1,
+                           const kd_tensor* q, const kd_tensor* attn, const kd_tensor* act, const kd_tensor* cos, const kd_tensor* sin,
+                           float eps, float scale);
+/* All blocks of Whisper's encoder (packages/model-utils/src/whisper/block.ts:150-200), enqueued by one call: per block
+ * kd_layer_norm, kd_linear_bf16_bias, kd_flash_attention over `heads` heads, kd_linear_bf16_bias (+ residual), kd_layer_norm, and
+ * the two linears of the MLP.  layer_tensors: per block attention norm weight, bias; in_proj [3E,E], bias; out_proj, bias; MLP norm
+ * weight, bias; fc1 [F,E], bias; fc2 [E,F], bias (biases may be NULL); eps: two per block; x and out contiguous bf16 [B,T,E]. */
+int kd_whisper_encoder_layers(const kd_tensor* const* layer_tensors, int n_layers, int heads, const float* eps, float scale, const kd_tensor* x,
+                              const kd_tensor* out);
 /* A whole decode step of a few sequences as one persistent kernel: embedding rows of `ids`, every layer (QKV, q/k-norm, rotary
  * embedding, cache write, attention over the cache, o_proj, SwiGLU MLP), the final norm and the lm_head over the embedding
  * table (packages/model-utils/src/qwen3/for_causal_lm.ts:170-194,475-508).  Advances *pos and *ctx_len by one when it is done.

@@ -151,6 +151,11 @@ class CudaTensorHandle:
             self._described = now
         return self._by_ref
 
+    def address(self) -> int:
+        """Of the descriptor that ref() shares."""
+        self.ref()
+        return ctypes.addressof(self._shared)
+
     def c(self) -> kd_tensor:
         """A descriptor of the caller's own."""
         self.ref()

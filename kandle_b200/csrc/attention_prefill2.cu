@@ -169,6 +169,8 @@ flash_attention_prefill2_kernel(const __grid_constant__ CUtensorMap tmap_q, cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  pdl_wait();      // nothing above touches global memory
+  pdl_trigger();   // after the TMEM allocation (see common.cuh)
   if (warp >= 8) {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
   if (warp == 8) {
@@ -401,7 +403,7 @@ static int launch_fa2(const CUtensorMap& tq, const CUtensorMap& tk, const CUtens
     KD_CUDA_CHECK(cudaFuncSetAttribute(flash_attention_prefill2_kernel<D, DR, WIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
     configured[ctx().device & 63] = true;
   }
-  flash_attention_prefill2_kernel<D, DR, WIN><<<grid, FA2_THREADS, SMEM, ctx().stream>>>(tq, tk, tv, tkr, p);
+  KD_CUDA_CHECK(launch_ex(flash_attention_prefill2_kernel<D, DR, WIN>, grid, dim3(FA2_THREADS), (size_t)SMEM, tq, tk, tv, tkr, p));
   return after_launch("flash_attention_prefill2_kernel");
 }
 

@@ -454,5 +454,6 @@ KD_API int kd_set_pdl(int enabled) {
   KD_TRY(require_init());
   ctx().pdl = enabled != 0;
   ctx().pdl_early_kv = enabled == 2;
+  ctx().pdl_weights = enabled == 3;
   return KD_OK;
 }

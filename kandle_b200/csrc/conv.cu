@@ -49,6 +49,8 @@ __global__ void bias_transpose_kernel(const void* __restrict__ tmp, int dt_t, co
 // coalesced on both sides.
 __global__ void im2col_tokens_bf16_kernel(const uint4* __restrict__ x, uint4* __restrict__ col, int B, int L, int cvec, int Wout,
                                           int ksz, int stride, int pad) {
+  pdl_wait();
+  pdl_trigger();
   const int64_t rowvec = (int64_t)ksz * cvec;
   const int64_t total = (int64_t)B * Wout * rowvec;
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
@@ -109,8 +111,8 @@ KD_API int kd_conv1d_tokens_bf16(const kd_tensor* input, const kd_tensor* weight
     int64_t blocks = (total + 255) / 256;
     const int64_t cap = (int64_t)ctx().sm_count * 32;
     if (blocks > cap) blocks = cap;
-    im2col_tokens_bf16_kernel<<<(int)blocks, 256, 0, ctx().stream>>>(static_cast<const uint4*>(px), static_cast<uint4*>(pcol), B, L, C / 8,
-                                                                    Wout, ksz, stride, padding);
+    launch_ex(im2col_tokens_bf16_kernel, dim3((unsigned)blocks), dim3(256), 0, (const uint4*)px, (uint4*)pcol, B, L, (int)(C / 8), (int)Wout, ksz, stride,
+              padding);
     st = after_launch("im2col_tokens_bf16_kernel");
   }
   if (st == KD_OK)

@@ -300,6 +300,8 @@ __global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const void* __restric
                                                             const void* __restrict__ w, int dt_w, float eps,
                                                             void* __restrict__ sum_out, int sum_f32, int round_sum,
                                                             __nv_bfloat16* __restrict__ norm_out, int64_t rows, int n) {
+  pdl_wait();
+  pdl_trigger();
   const int lane = threadIdx.x & 31;
   const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (row >= rows) return;
@@ -383,6 +385,8 @@ __global__ void __launch_bounds__(256) rmsnorm_rows_kernel(const void* __restric
 template <int NV>
 __global__ void __launch_bounds__(256) rmsnorm_plain_rows_kernel(const float* __restrict__ src, const __nv_bfloat16* __restrict__ w, float eps,
                                                                  __nv_bfloat16* __restrict__ norm_out, int64_t rows, int n) {
+  pdl_wait();
+  pdl_trigger();
   const int lane = threadIdx.x & 31;
   const int64_t row = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (row >= rows) return;
@@ -696,17 +700,13 @@ KD_API int kd_add_rmsnorm(const kd_tensor* x, const kd_tensor* residual, const k
     KD_REQUIRE((reinterpret_cast<uintptr_t>(pw) & 15) == 0, "weight must be 16-byte aligned");
     if (splits == 1 && !residual && !sum_out && weight->dtype == KD_BF16 && (reinterpret_cast<uintptr_t>(px) & 31) == 0) {
       auto k = n <= 8 * 32 * 4 ? rmsnorm_plain_rows_kernel<4> : n <= 8 * 32 * 10 ? rmsnorm_plain_rows_kernel<10> : rmsnorm_plain_rows_kernel<RWN_MAXV>;
-      k<<<(unsigned)((rows + 7) / 8), 256, 0, ctx().stream>>>((const float*)px, (const __nv_bfloat16*)pw, eps, (__nv_bfloat16*)pn, rows, (int)n);
+      KD_CUDA_CHECK(launch_ex(k, dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, (const float*)px, (const __nv_bfloat16*)pw, eps, (__nv_bfloat16*)pn, rows, (int)n));
       return after_launch("rmsnorm_plain_rows_kernel");
     }
-    if (n <= 8 * 32 * 4)
-      rmsnorm_rows_kernel<4><<<(unsigned)((rows + 7) / 8), 256, 0, ctx().stream>>>(
-          px, splits == 1, pr, residual ? residual->dtype == KD_F32 : 0, pw, weight->dtype, eps, ps, sum_f32, round_sum,
-          (__nv_bfloat16*)pn, rows, (int)n);
-    else
-      rmsnorm_rows_kernel<RWN_MAXV><<<(unsigned)((rows + 7) / 8), 256, 0, ctx().stream>>>(
-          px, splits == 1, pr, residual ? residual->dtype == KD_F32 : 0, pw, weight->dtype, eps, ps, sum_f32, round_sum,
-          (__nv_bfloat16*)pn, rows, (int)n);
+    auto k = n <= 8 * 32 * 4 ? rmsnorm_rows_kernel<4> : rmsnorm_rows_kernel<RWN_MAXV>;
+    KD_CUDA_CHECK(launch_ex(k, dim3((unsigned)((rows + 7) / 8)), dim3(256), 0, (const void*)px, (int)(splits == 1), (const void*)pr,
+                            (int)(residual ? residual->dtype == KD_F32 : 0), (const void*)pw, (int)weight->dtype, eps, ps, sum_f32, round_sum,
+                            (__nv_bfloat16*)pn, rows, (int)n));
     return after_launch("rmsnorm_rows_kernel");
   }
   KD_CUDA_CHECK(launch_ex(add_rmsnorm_kernel, dim3((unsigned)rows), dim3(ARN_THREADS), 0, (const void*)px, splits, (const void*)pr,

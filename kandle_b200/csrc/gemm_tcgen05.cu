@@ -117,6 +117,7 @@ struct GemmParams {
   // (group_off null) group_rows rows each
   const int* group_off;
   int groups, group_rows;
+  int early_w;            // the first W tiles may be fetched before the grid-dependency wait (kd_set_pdl(3))
   int splits;             // CTAs of a cluster that share a tile, each with a range of k-blocks (then a CTA has one tile)
   float glu_limit;        // epi == 4: clamped GLU, see clamped_glu_f; epi == 5: GELU(gate) * up
 };
@@ -220,7 +221,19 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  pdl_wait();      // nothing above touches global memory
+  // The first W tiles of this CTA, as many as the ring holds: they do not depend on the kernels before.  97 rows of the 0.6B
+  // widths: see the launches of a prompt in Qwen3Engine.prefill.
+  int early = 0;
+  if (p.early_w && warp == 0 && lane == 0) {
+    const int nkb = (p.K + GEMM_BK - 1) / GEMM_BK, rk = SHARED ? (int)(blockIdx.x % p.splits) : 0, tile = SHARED ? (int)(blockIdx.x / p.splits) : (int)blockIdx.x;
+    const int kb0 = SHARED ? nkb * rk / p.splits : 0, kb1 = SHARED ? nkb * (rk + 1) / p.splits : nkb;
+    if (tile < p.num_m_tiles * p.num_n_tiles)
+      for (; early < STAGES && kb0 + early < kb1; ++early) {
+        mbar_arrive_expect_tx(&full[early], STAGE_BYTES);
+        tma_load_2d(smem + early * STAGE_BYTES + A_BYTES, &tmap_b, &full[early], (kb0 + early) * GEMM_BK, tile % p.num_n_tiles * BLOCK_N);
+      }
+  }
+  pdl_wait();      // nothing above touches what the kernels before have written
   pdl_trigger();   // after the TMEM allocation (see common.cuh)
 
   const int num_k_blocks = (p.K + GEMM_BK - 1) / GEMM_BK;
@@ -274,11 +287,16 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
         int row0, row_end, w_row;
         locate(m_tile, row0, row_end, w_row);
         for (int kb = kb_begin; kb < kb_end; ++kb) {
-          if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.err, 201)) { ok = false; break; }
           uint8_t* sa = smem + stage * STAGE_BYTES;
-          mbar_arrive_expect_tx(&full[stage], STAGE_BYTES);
-          tma_load_2d(sa, &tmap_a, &full[stage], kb * GEMM_BK, row0);
-          tma_load_2d(sa + A_BYTES, &tmap_b, &full[stage], kb * GEMM_BK, w_row + n_tile * BLOCK_N);
+          if (early > 0) {                               // (the first stages: W is on its way)
+            --early;
+            tma_load_2d(sa, &tmap_a, &full[stage], kb * GEMM_BK, row0);
+          } else {
+            if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.err, 201)) { ok = false; break; }
+            mbar_arrive_expect_tx(&full[stage], STAGE_BYTES);
+            tma_load_2d(sa, &tmap_a, &full[stage], kb * GEMM_BK, row0);
+            tma_load_2d(sa + A_BYTES, &tmap_b, &full[stage], kb * GEMM_BK, w_row + n_tile * BLOCK_N);
+          }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
@@ -683,6 +701,7 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams&
   // (grouped: every group may end in a partial tile, and groups without rows have none)
   p.num_m_tiles = (p.M + GEMM_BM - 1) / GEMM_BM + (p.groups ? (p.groups < p.M ? p.groups : p.M) : 0);
   p.num_n_tiles = (p.N + BLOCK_N - 1) / BLOCK_N;
+  p.early_w = ctx().pdl_weights && p.groups == 0;
   const int64_t total = (int64_t)p.num_m_tiles * p.num_n_tiles;
   // (linear_tile shares no 256-wide tile; the epilogue over heads is in this instantiation, or the plain one would grow)
   if (BLOCK_N < 256 && (p.splits > 1 || p.epi == 3)) {

@@ -161,6 +161,8 @@ template <int MODE, int NV, int LOADS>
 __global__ void __launch_bounds__(256) norm_rows_bf16_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
                                                             const __nv_bfloat16* __restrict__ b, __nv_bfloat16* __restrict__ y,
                                                             int64_t rows, int n, float eps) {
+  pdl_wait();
+  pdl_trigger();
   const int lane = threadIdx.x & 31;
   const int64_t warp0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int64_t nwarps = ((int64_t)gridDim.x * blockDim.x) >> 5;
@@ -246,13 +248,13 @@ __global__ void __launch_bounds__(256) norm_rows_bf16_kernel(const __nv_bfloat16
 }
 
 template <int MODE, int NV, int LOADS>
-static void launch_norm_rows_bf16(const void* x, const void* w, const void* b, void* y, int64_t rows, int n, float eps) {
+static int launch_norm_rows_bf16(const void* x, const void* w, const void* b, void* y, int64_t rows, int n, float eps) {
   int64_t blocks = (rows + 7) / 8;
   const int64_t cap = (int64_t)ctx().sm_count * 16;
   if (blocks > cap) blocks = cap;
-  norm_rows_bf16_kernel<MODE, NV, LOADS><<<(int)blocks, 256, 0, ctx().stream>>>(
-      static_cast<const __nv_bfloat16*>(x), static_cast<const __nv_bfloat16*>(w), static_cast<const __nv_bfloat16*>(b),
-      static_cast<__nv_bfloat16*>(y), rows, n, eps);
+  KD_CUDA_CHECK(launch_ex(norm_rows_bf16_kernel<MODE, NV, LOADS>, dim3((unsigned)blocks), dim3(256), 0, static_cast<const __nv_bfloat16*>(x),
+                          static_cast<const __nv_bfloat16*>(w), static_cast<const __nv_bfloat16*>(b), static_cast<__nv_bfloat16*>(y), rows, n, eps));
+  return KD_OK;
 }
 
 template <int MODE>
@@ -285,14 +287,12 @@ static int launch_norm(const kd_tensor* x, const kd_tensor* w, const kd_tensor* 
     constexpr int M2 = MODE == NORM_SOFTMAX ? NORM_RMS : MODE;   // the softmax instantiation is never launched
     const bool many = rows > (int64_t)sms * 16 * 8 * 2;          // (the launch's warps take a third row)
     constexpr int WIDE = MODE == NORM_RMS ? NORM_NEXT : NORM_ROW, WIDE4 = MODE == NORM_RMS ? NORM_NEXT : NORM_IN_TURN;
-    if (n <= 256) launch_norm_rows_bf16<M2, 1, NORM_IN_TURN>(px, pw, pb, py, rows, (int)n, eps);
-    else if (n <= 512) launch_norm_rows_bf16<M2, 2, NORM_IN_TURN>(px, pw, pb, py, rows, (int)n, eps);
-    else if (n <= 768) many ? launch_norm_rows_bf16<M2, 3, NORM_NEXT>(px, pw, pb, py, rows, (int)n, eps)
-                            : launch_norm_rows_bf16<M2, 3, NORM_ROW>(px, pw, pb, py, rows, (int)n, eps);
-    else if (n <= 1024) many ? launch_norm_rows_bf16<M2, 4, WIDE4>(px, pw, pb, py, rows, (int)n, eps)
-                             : launch_norm_rows_bf16<M2, 4, NORM_IN_TURN>(px, pw, pb, py, rows, (int)n, eps);
-    else many ? launch_norm_rows_bf16<M2, 8, WIDE>(px, pw, pb, py, rows, (int)n, eps)
-              : launch_norm_rows_bf16<M2, 8, NORM_ROW>(px, pw, pb, py, rows, (int)n, eps);
+    const auto launch = n <= 256 ? launch_norm_rows_bf16<M2, 1, NORM_IN_TURN>
+                        : n <= 512 ? launch_norm_rows_bf16<M2, 2, NORM_IN_TURN>
+                        : n <= 768 ? (many ? launch_norm_rows_bf16<M2, 3, NORM_NEXT> : launch_norm_rows_bf16<M2, 3, NORM_ROW>)
+                        : n <= 1024 ? (many ? launch_norm_rows_bf16<M2, 4, WIDE4> : launch_norm_rows_bf16<M2, 4, NORM_IN_TURN>)
+                                    : (many ? launch_norm_rows_bf16<M2, 8, WIDE> : launch_norm_rows_bf16<M2, 8, NORM_ROW>);
+    KD_TRY(launch(px, pw, pb, py, rows, (int)n, eps));
     return after_launch(name);
   }
   if (n <= 512) {

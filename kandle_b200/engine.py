@@ -234,6 +234,7 @@ class Qwen3Engine(DecoderEngine):
             self.v_cache = [core.zeros((self.B, self.Hkv, max_seq_len, self.D), "bfloat16") for _ in range(self.L)]
         self.scale = 1.0 / math.sqrt(self.D)
         self._prefill_bufs = {}
+        self._refs = None
         self.use_early_kv = os.environ.get("KD_EARLY_KV", "1") != "0"
         # decode: run o_proj .. next layer's QKV as one persistent kernel per layer (kd_decode_layer_chain);
         # tensor parallelism needs an all-reduce after o_proj and down_proj, so it keeps separate kernels
@@ -349,6 +350,18 @@ class Qwen3Engine(DecoderEngine):
         if ids_t is None:
             core._backend().upload(w["ids"]._handle, ids.reshape(-1))
             ids_t = w["ids"]
+        # every kernel starts while the one before it drains, and the linears fetch their first weights meanwhile
+        # (0.6B: 97 tokens 2.07 -> 1.79 ms, 2103 3.87 -> 3.38, 8192 11.4 -> 10.9, 16384 and 32768 the same, 65536 81.0 -> 83.1)
+        lib.call("kd_set_pdl", 3 if self.use_pdl and self.tp == 1 and B * S <= 16384 else 0)
+        try:
+            full = self._prefill_kernels(w, ids_t, B, S, all_logits)
+        finally:
+            lib.call("kd_set_pdl", 0)
+        self.pos = S
+        self.cur_B = B
+        return (w["tok"], full) if all_logits else w["tok"]
+
+    def _prefill_kernels(self, w: dict, ids_t: Tensor, B: int, S: int, all_logits: bool):
         c = self.cfg
         T = B * S
         core._kernel("index_select")(self.embed._handle, ids_t._handle, {"dim": 0}, w["emb"]._handle)
@@ -359,7 +372,11 @@ class Qwen3Engine(DecoderEngine):
         attn2d = w["attn"].view(T, self.Hq * self.D)
         h, h1 = w["h"], w["h1"]
         table = self.block_table.slice([slice(0, B), slice(None)]) if self.paged else None
-        for li, lw in enumerate(self.layers):
+        native = self.tp == 1 and self.D == 128 and not self.paged
+        if native:
+            lib.call("kd_qwen3_prompt_layers", self._layer_refs(), self.L, _r(w["x"]), _r(h), _r(h1), _r(w["q"]), _r(w["attn"]), _r(w["act"]),
+                     _r(w["cos"]), _r(w["sin"]), ctypes.c_float(c.rmsNormEps), ctypes.c_float(self.scale))
+        for li, lw in enumerate(self.layers if not native else ()):
             if self.paged:
                 # the prompt's K/V go to a contiguous buffer that the attention reads, then into the pages
                 kc, vc = w["kt"].slice(":, :, :, :"), w["vt"].slice(":, :, :, :")
@@ -420,9 +437,7 @@ class Qwen3Engine(DecoderEngine):
             t.dispose()
         if table is not None:
             table.dispose()
-        self.pos = S
-        self.cur_B = B
-        return (w["tok"], full) if all_logits else w["tok"]
+        return full
 
     # ------------------------------------------------------------------ decode
     def _decode_state(self, B: int) -> dict:
@@ -464,9 +479,17 @@ class Qwen3Engine(DecoderEngine):
         self._decode = d
         return d
 
+    def _layer_refs(self):
+        """The layers' tensors as kd_decode_step and kd_qwen3_prompt_layers take them.  Laid out once: it takes 75 us, and the GPU
+        waits for it at the start of a prompt.  (The library looks the storages up at each call.)"""
+        if self._refs is None:
+            names = ("in_norm", "wqkv", "q_norm", "k_norm", "wo", "post_norm", "wgu", "wdown")
+            kept = [t._handle.c() for i, lw in enumerate(self.layers) for t in [lw[k] for k in names] + [self.k_cache[i], self.v_cache[i]]]
+            self._refs = (ctypes.c_void_p * len(kept))(*map(ctypes.addressof, kept)), kept
+        return self._refs[0]
+
     def _step_kernel_state(self, B: int):
-        """What kd_decode_step needs beside a step's buffers (hand-over words, the layers' descriptors), or None where it
-        does not take the shape.  Its attention reads the cache at two thirds of the rate of kd_attention_decode: with six
+        """The hand-over words that kd_decode_step needs beside a step's buffers, or None where it does not take the shape.  Its attention reads the cache at two thirds of the rate of kd_attention_decode: with six
         sequences it is ahead up to 5000 keys (step of the 0.6B model: 0.76 ms against 1.10 at 300 keys, 1.1 against 1.3 at
         2200, 2.2 against 2.0 at 8000), with one at any length (0.71 against 1.53 at 8000)."""
         n = ctypes.c_uint64(0)
@@ -474,10 +497,7 @@ class Qwen3Engine(DecoderEngine):
             lib.call("kd_decode_step_state_bytes", B, self.H, self.I, self.Hq, self.Hkv, self.D, self.V, self.L, 0, ctypes.byref(n))
         if not n.value:
             return None
-        names = ("in_norm", "wqkv", "q_norm", "k_norm", "wo", "post_norm", "wgu", "wdown")
-        parts = [t for i, lw in enumerate(self.layers) for t in [lw[k] for k in names] + [self.k_cache[i], self.v_cache[i]]]
-        kept = [t._handle.c() for t in parts]
-        return {"words": core.zeros((n.value // 4,), "int32"), "kept": kept, "layers": (ctypes.POINTER(lib.kd_tensor) * len(kept))(*map(ctypes.pointer, kept))}
+        return core.zeros((n.value // 4,), "int32")
 
     def _enqueue_decode_step(self, d: dict) -> None:
         """One decode step for d['ids'] at device position d['pos']; leaves the next ids in d['ids']."""
@@ -494,8 +514,8 @@ class Qwen3Engine(DecoderEngine):
         c, B = self.cfg, d["B"]
         eps = ctypes.c_float(c.rmsNormEps)
         if d["step"] is not None:
-            lib.call("kd_decode_step", d["step"]["layers"], self.L, _r(self.embed), _r(self.final_norm), _r(d["ids"]), _r(self.inv_freq), _r(d["pos"]),
-                     _r(d["ctx"]), eps, ctypes.c_float(self.scale), _r(self.block_table), _r(d["step"]["words"]), _r(d["logits"]))
+            lib.call("kd_decode_step", self._layer_refs(), self.L, _r(self.embed), _r(self.final_norm), _r(d["ids"]), _r(self.inv_freq), _r(d["pos"]),
+                     _r(d["ctx"]), eps, ctypes.c_float(self.scale), _r(self.block_table), _r(d["step"]), _r(d["logits"]))
             lg = d["logits"].view(B, self.V)
             self._next_tokens(lg, d["uniforms"], d["ids"])
             lg.dispose()

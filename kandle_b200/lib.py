@@ -91,6 +91,7 @@ if not os.path.exists(LIB_PATH):
 _lib = ctypes.CDLL(LIB_PATH)
 
 _T = ctypes.POINTER(kd_tensor)
+_REFS = ctypes.c_void_p       # array of descriptors' addresses (refs)
 _u64 = ctypes.c_uint64
 _SIGNATURES = {
     "kd_init": [ctypes.c_int, ctypes.c_uint],
@@ -156,7 +157,9 @@ _SIGNATURES = {
     "kd_decode_layer_chain": [_T, _T, _T, _T, _T, _T, _T, ctypes.c_float, _T, _T, _T, _T, _T, _T],
     "kd_decode_layer_fused": [_T, _T, _T, _T, _T, _T, _T, ctypes.c_float, _T, _T, _T, _T, _T, _T, _T, _T, _T, _T, _T, _T],
     "kd_decode_layer_fused_tp": [_T, _T, _T, _T, _T, _T, _T, ctypes.c_float, _T, _T, _T, _T, _T, _T, _T, _T, _T, _T, _T, _T],
-    "kd_decode_step": [ctypes.POINTER(_T), ctypes.c_int] + [_T] * 6 + [ctypes.c_float] * 2 + [_T] * 3,
+    "kd_decode_step": [_REFS, ctypes.c_int] + [_T] * 6 + [ctypes.c_float] * 2 + [_T] * 3,
+    "kd_qwen3_prompt_layers": [_REFS, ctypes.c_int] + [_T] * 8 + [ctypes.c_float] * 2,
+    "kd_whisper_encoder_layers": [_REFS, ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_float), ctypes.c_float, _T, _T],
     "kd_decode_step_state_bytes": [ctypes.c_int] * 9 + [ctypes.POINTER(_u64)],
     "kd_debug_decode_layer_plan": [ctypes.c_int] * 9 + [ctypes.POINTER(ctypes.c_int), ctypes.c_int],
     "kd_debug_decode_layer_trace": [ctypes.POINTER(ctypes.c_uint64), ctypes.c_int],
@@ -235,6 +238,11 @@ def call(name: str, *args) -> None:
     st = getattr(_lib, name)(*args)
     if st != 0:
         raise KandleCudaError(st, f"{name}: {last_error()}")
+
+
+def refs(tensors):
+    """Descriptors of tensors (None allowed) as the library takes them in an array; the tensors have to stay while it is used."""
+    return (ctypes.c_void_p * len(tensors))(*[None if t is None else t._handle.address() for t in tensors])
 
 
 def raw():
