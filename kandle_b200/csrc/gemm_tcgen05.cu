@@ -184,15 +184,19 @@ __device__ __forceinline__ float4 ld_peer_f4(uint32_t addr, uint32_t rank) {
   return v;
 }
 
-// SHARED: the CTAs of a cluster share a tile (an instantiation of its own: the plain one took 0.6 us longer with it inside)
-template <int BLOCK_N, int STAGES, bool SHARED>
+// SHARED: the CTAs of a cluster share a tile (an instantiation of its own: the plain one took 0.6 us longer with it inside).
+// PAIR: a cluster of two CTAs works on tiles of 256 rows with MMAs across both SMs (cta_group::2).  Each brings in its 128 rows of
+// A and half of the W tile, so a k-block costs an SM 32 KB of copies and of operand reads instead of 48, and six stages
+// fit instead of four.
+template <int BLOCK_N, int STAGES, bool SHARED, bool PAIR = false>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, GemmParams p) {
   constexpr int A_BYTES = GEMM_BM * GEMM_BK * 2;
-  constexpr int B_BYTES = BLOCK_N * GEMM_BK * 2;
+  constexpr int B_BYTES = (PAIR ? BLOCK_N / 2 : BLOCK_N) * GEMM_BK * 2;
   constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
+  constexpr int TILE_M = PAIR ? 2 * GEMM_BM : GEMM_BM;
   constexpr uint32_t TMEM_COLS = 2 * BLOCK_N < 32 ? 32 : 2 * BLOCK_N;
-  constexpr uint32_t IDESC = make_idesc_bf16(GEMM_BM, BLOCK_N, 0, 0);
+  constexpr uint32_t IDESC = make_idesc_bf16(TILE_M, BLOCK_N, 0, 0);
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -207,30 +211,46 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-    for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], 4); }
+    for (int b = 0; b < 2; ++b) { mbar_init(&tmem_full[b], 1); mbar_init(&tmem_empty[b], PAIR ? 8 : 4); }
     *abort_flag = 0;
     fence_mbar_init();
     prefetch_tmap(&tmap_a);
     prefetch_tmap(&tmap_b);
   }
   if (warp == 1) {
-    tmem_alloc(tmem_slot, TMEM_COLS);
-    tmem_relinquish();
+    if constexpr (PAIR) {
+      tmem_alloc_pair(tmem_slot, TMEM_COLS);
+      tmem_relinquish_pair();
+    } else {
+      tmem_alloc(tmem_slot, TMEM_COLS);
+      tmem_relinquish();
+    }
   }
   tc_fence_before();
   __syncthreads();
+  if (PAIR) cluster_sync();       // both CTAs' barriers exist and both have their tensor memory
   tc_fence_after();
+  const uint32_t pair_rank = PAIR ? cluster_rank() : 0u;
+  // a full stage is announced to the CTA that issues the MMAs
+  auto full_bar = [&](int stage) { return PAIR ? peer_smem(&full[stage], 0u) : smem_u32(&full[stage]); };
+  auto load = [&](void* dst, const CUtensorMap* m, int stage, int x, int y) {
+    if constexpr (PAIR) tma_load_2d_pair(dst, m, full_bar(stage), x, y);
+    else tma_load_2d(dst, m, &full[stage], x, y);
+  };
+  auto expect = [&](int stage) {
+    if (!PAIR || pair_rank == 0) mbar_arrive_expect_tx(&full[stage], PAIR ? 2 * STAGE_BYTES : STAGE_BYTES);
+  };
   const uint32_t tmem_base = *tmem_slot;
   // The first W tiles of this CTA, as many as the ring holds: they do not depend on the kernels before.  97 rows of the 0.6B
   // widths: see the launches of a prompt in Qwen3Engine.prefill.
   int early = 0;
   if (p.early_w && warp == 0 && lane == 0) {
-    const int nkb = (p.K + GEMM_BK - 1) / GEMM_BK, rk = SHARED ? (int)(blockIdx.x % p.splits) : 0, tile = SHARED ? (int)(blockIdx.x / p.splits) : (int)blockIdx.x;
+    const int nkb = (p.K + GEMM_BK - 1) / GEMM_BK, rk = SHARED ? (int)(blockIdx.x % p.splits) : 0, tile = SHARED ? (int)(blockIdx.x / p.splits) : PAIR ? (int)(blockIdx.x / 2) : (int)blockIdx.x;
     const int kb0 = SHARED ? nkb * rk / p.splits : 0, kb1 = SHARED ? nkb * (rk + 1) / p.splits : nkb;
     if (tile < p.num_m_tiles * p.num_n_tiles)
       for (; early < STAGES && kb0 + early < kb1; ++early) {
-        mbar_arrive_expect_tx(&full[early], STAGE_BYTES);
-        tma_load_2d(smem + early * STAGE_BYTES + A_BYTES, &tmap_b, &full[early], (kb0 + early) * GEMM_BK, tile % p.num_n_tiles * BLOCK_N);
+        expect(early);
+        load(smem + early * STAGE_BYTES + A_BYTES, &tmap_b, early, (kb0 + early) * GEMM_BK, tile % p.num_n_tiles * BLOCK_N + (int)pair_rank * (BLOCK_N / 2));
       }
   }
   pdl_wait();      // nothing above touches what the kernels before have written
@@ -261,12 +281,12 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     num_m_tiles = group_tile[p.groups];
   }
   const int total_tiles = num_m_tiles * p.num_n_tiles;
-  const int rank = SHARED ? (int)(blockIdx.x % p.splits) : 0, first = SHARED ? (int)(blockIdx.x / p.splits) : (int)blockIdx.x;
-  const int step = SHARED ? (int)(gridDim.x / p.splits) : (int)gridDim.x;
+  const int rank = SHARED ? (int)(blockIdx.x % p.splits) : 0, first = SHARED ? (int)(blockIdx.x / p.splits) : PAIR ? (int)(blockIdx.x / 2) : (int)blockIdx.x;
+  const int step = SHARED ? (int)(gridDim.x / p.splits) : PAIR ? (int)(gridDim.x / 2) : (int)gridDim.x;
   const int kb_begin = SHARED ? num_k_blocks * rank / p.splits : 0, kb_end = SHARED ? num_k_blocks * (rank + 1) / p.splits : num_k_blocks;
   // first A row, end of the valid rows and first W row of tile row m_tile
   auto locate = [&](int m_tile, int& row0, int& row_end, int& w_row) {
-    if (p.groups == 0) { row0 = m_tile * GEMM_BM; row_end = p.M; w_row = 0; return; }
+    if (PAIR || p.groups == 0) { row0 = m_tile * TILE_M + (int)pair_rank * GEMM_BM; row_end = p.M; w_row = 0; return; }
     int lo = 0, hi = p.groups - 1;                     // last group whose first tile is <= m_tile
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
@@ -290,19 +310,19 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
           uint8_t* sa = smem + stage * STAGE_BYTES;
           if (early > 0) {                               // (the first stages: W is on its way)
             --early;
-            tma_load_2d(sa, &tmap_a, &full[stage], kb * GEMM_BK, row0);
+            load(sa, &tmap_a, stage, kb * GEMM_BK, row0);
           } else {
             if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.err, 201)) { ok = false; break; }
-            mbar_arrive_expect_tx(&full[stage], STAGE_BYTES);
-            tma_load_2d(sa, &tmap_a, &full[stage], kb * GEMM_BK, row0);
-            tma_load_2d(sa + A_BYTES, &tmap_b, &full[stage], kb * GEMM_BK, w_row + n_tile * BLOCK_N);
+            expect(stage);
+            load(sa, &tmap_a, stage, kb * GEMM_BK, row0);
+            load(sa + A_BYTES, &tmap_b, stage, kb * GEMM_BK, w_row + n_tile * BLOCK_N + (int)pair_rank * (BLOCK_N / 2));
           }
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (lane == 0 && pair_rank == 0) {
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
@@ -321,19 +341,26 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
           for (int k = 0; k < GEMM_BK / 16; ++k) {
             const uint64_t adesc = make_smem_desc_sw128(a_addr + k * 32, 16, 1024);
             const uint64_t bdesc = make_smem_desc_sw128(b_addr + k * 32, 16, 1024);
-            umma_ss(d_tmem, adesc, bdesc, IDESC, ((kb - kb_begin) | k) != 0 ? 1u : 0u);
+            if constexpr (PAIR) umma_ss_pair(d_tmem, adesc, bdesc, IDESC, ((kb - kb_begin) | k) != 0 ? 1u : 0u);
+            else umma_ss(d_tmem, adesc, bdesc, IDESC, ((kb - kb_begin) | k) != 0 ? 1u : 0u);
           }
-          umma_commit(&empty[stage]);
+          if constexpr (PAIR) umma_commit_pair(&empty[stage]);
+          else umma_commit(&empty[stage]);
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        umma_commit(&tmem_full[acc]);
+        if constexpr (PAIR) umma_commit_pair(&tmem_full[acc]);
+        else umma_commit(&tmem_full[acc]);
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1;
       }
     }
   } else {
     const int q = warp & 3;  // TMEM lane quarter this warp may access
+    auto give_back = [&](int a) {            // the accumulator, to whoever issues the MMAs
+      if (PAIR && pair_rank != 0) mbar_arrive_peer(peer_smem(&tmem_empty[a], 0u));
+      else mbar_arrive(&tmem_empty[a]);
+    };
     int acc = 0;
     uint32_t acc_phase = 0;
     for (int tile = first; tile < total_tiles; tile += step) {
@@ -507,7 +534,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
           } else {
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&tmem_empty[acc]);
+            if (lane == 0) give_back(acc);
             released = true;
           }
           process(rb, c0 + 32);
@@ -656,7 +683,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
           } else {
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive(&tmem_empty[acc]);
+            if (lane == 0) give_back(acc);
             released = true;
           }
           process(rb, c0 + 32);
@@ -665,7 +692,7 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
       if (!released) {
         tc_fence_before();
         __syncwarp();
-        if (lane == 0) mbar_arrive(&tmem_empty[acc]);
+        if (lane == 0) give_back(acc);
       }
       acc ^= 1;
       if (acc == 0) acc_phase ^= 1;
@@ -680,11 +707,48 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
   // teardown: every role falls through to here, also after an aborted wait
   tc_fence_before();
   __syncthreads();
+  if (PAIR) {
+    __syncwarp();
+    cluster_sync();       // neither leaves while the other may arrive on its barriers or issue MMAs for it
+  }
   if (warp == 1) {
     __syncwarp();
     tc_fence_after();
-    tmem_dealloc(tmem_base, TMEM_COLS);
+    if constexpr (PAIR) tmem_dealloc_pair(tmem_base, TMEM_COLS);
+    else tmem_dealloc(tmem_base, TMEM_COLS);
   }
+}
+
+// Tiles of 256 x 256 by pairs of CTAs.
+static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams& p) {
+  constexpr int BLOCK_N = 256, STAGES = 6, SMEM = STAGES * (GEMM_BM + BLOCK_N / 2) * GEMM_BK * 2 + 1024 + 256;
+  const auto kernel = gemm_bf16_tcgen05_kernel<BLOCK_N, STAGES, false, true>;
+  static bool configured[64] = {false};
+  if (!configured[ctx().device & 63]) {
+    KD_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+    configured[ctx().device & 63] = true;
+  }
+  p.num_m_tiles = (p.M + 2 * GEMM_BM - 1) / (2 * GEMM_BM);
+  p.num_n_tiles = (p.N + BLOCK_N - 1) / BLOCK_N;
+  p.early_w = ctx().pdl_weights;
+  p.splits = 1;
+  const int64_t tiles = (int64_t)p.num_m_tiles * p.num_n_tiles;
+  const int pairs = (int)std::min<int64_t>(tiles, ctx().sm_count / 2);
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(2 * pairs));
+  cfg.blockDim = dim3(GEMM_THREADS);
+  cfg.dynamicSmemBytes = SMEM;
+  cfg.stream = ctx().stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = ctx().pdl ? 2 : 1;
+  KD_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, ta, tb, p));
+  return after_launch("gemm_bf16_tcgen05_kernel<pair>");
 }
 
 template <int BLOCK_N, int STAGES>
@@ -753,6 +817,18 @@ static int linear_tile(int64_t M, int64_t N, int64_t K, int narrowest, int64_t s
   return bn;
 }
 
+// Whether 256-wide tiles are worked on by pairs of CTAs.  A launch of pairs costs 1 to 2 us more (two cluster barriers, tensor memory
+// for both); it gains where the SMs multiply long enough: by K (less copied and read per k-block: N = 2560, K = 9728, 2103 rows
+// 128 -> 111 us; N = 1024, K = 3072, 8192 rows 56 -> 49, 4096 rows 29 -> 31) and where the chip runs at its power limit (65536 rows:
+// N = 4096, K = 1024 475 -> 395 to 458 us, N = 6144 630 -> 572; 96000 rows, K = 768: N = 2304 319 -> 300, N = 3072 427 -> 382).
+// Between, at K = 1024, it is even (16384 rows: N = 4096 113 -> 111, N = 6144 153 -> 159); N = 768 loses up to 24576 rows (16384 rows,
+// K = 3072 67 -> 72).
+static bool linear_pair(int64_t M, int64_t N, int64_t K, int64_t sms) {
+  const int64_t n_tiles = (N + 255) / 256, kbs = (K + GEMM_BK - 1) / GEMM_BK;
+  const int64_t waves = ((M + 127) / 128 * n_tiles + sms - 1) / sms, pair_waves = ((M + 255) / 256 * n_tiles + sms / 2 - 1) / (sms / 2);
+  return pair_waves <= waves && (M >= 24576 || (N >= 1024 && waves * kbs >= (K >= 1024 ? 96 : 132)));
+}
+
 // out[M, N or N/2] = epilogue(A[M,K] * W[N,K]^T).  Pointers are device pointers; ld* in elements.
 int gemm_bf16(const void* A, int64_t lda, const void* W, int64_t ldw, void* out, int64_t ldo, int out_f32,
               const void* resid, int64_t ldr, int M, int N, int K, int epi) {
@@ -792,7 +868,9 @@ int gemm_bf16_bias_act(const void* A, int64_t lda, const void* W, int64_t ldw, v
   CUtensorMap ta, tb;
   KD_TRY(make_tmap_bf16_2d(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, GEMM_BM, GEMM_BK));
   const int bn = linear_tile(M, N, K, 64, ctx().sm_count, &p.splits);
-  KD_TRY(make_tmap_bf16_2d(&tb, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, bn, GEMM_BK));
+  const bool pair = bn == 256 && linear_pair(M, N, K, ctx().sm_count);
+  KD_TRY(make_tmap_bf16_2d(&tb, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, pair ? 128 : bn, GEMM_BK));
+  if (pair) return launch_gemm_pair(ta, tb, p);
   if (bn == 256) return launch_gemm<256, 4>(ta, tb, p);
   if (bn == 128) return launch_gemm<128, 6>(ta, tb, p);
   return launch_gemm<64, 8>(ta, tb, p);
@@ -841,7 +919,9 @@ int gemm_bf16_qkv_rope(const void* A, int64_t lda, const void* W, int64_t ldw, i
   CUtensorMap ta, tb;
   KD_TRY(make_tmap_bf16_2d(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, GEMM_BM, GEMM_BK));
   const int bn = linear_tile(M, N, K, 128, ctx().sm_count, &p.splits);      // (a head of 128 columns lies in one tile)
-  KD_TRY(make_tmap_bf16_2d(&tb, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, bn, GEMM_BK));
+  const bool pair = bn == 256 && linear_pair(M, N, K, ctx().sm_count);
+  KD_TRY(make_tmap_bf16_2d(&tb, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, pair ? 128 : bn, GEMM_BK));
+  if (pair) return launch_gemm_pair(ta, tb, p);
   return bn == 256 ? launch_gemm<256, 4>(ta, tb, p) : launch_gemm<128, 6>(ta, tb, p);
 }
 
@@ -1117,6 +1197,13 @@ int matmul_tc_try(const kd_matmul_cfg* cfg, const kd_tensor* a, const kd_tensor*
 }  // namespace kd
 
 using namespace kd;
+
+KD_API int kd_debug_linear_pair(int64_t M, int64_t N, int64_t K, int heads_of_128, int sms, int* pair) {
+  KD_REQUIRE(pair && M > 0 && N > 0 && K > 0 && sms > 0, "bad argument");
+  int sharing = 1;
+  *pair = linear_tile(M, N, K, heads_of_128 ? 128 : 64, sms, &sharing) == 256 && linear_pair(M, N, K, sms);
+  return KD_OK;
+}
 
 KD_API int kd_debug_linear_plan(int64_t M, int64_t N, int64_t K, int heads_of_128, int sms, int* width, int* sharing) {
   KD_REQUIRE(width && sharing && M > 0 && N > 0 && K > 0 && sms > 0, "bad argument");
