@@ -122,11 +122,13 @@ int kd_debug_fill_scratch(int byte_value);
  *   linear       width of the output tiles of kd_linear_bf16 and its relatives (heads_of_128: of
  *                kd_qkv_linear_norm_rope_cachewrite) and the CTAs that share a tile's K
  *   pair         whether pairs of CTAs work on its 256-wide tiles
+ *   linear_few   CTAs of a cluster and its weight rows where linears of up to 32 rows take the kernel for a few rows, else 0
  *   matmul_f32   as linear, for kd_matmul with K-major fp32 operands
  *   recurrence   whether kd_delta_rule (delta = 1) or kd_wkv takes a call of `tokens` tokens and `heads` heads (of all
  *                sequences) through records, and the CTAs of that form's second kernel */
 int kd_debug_linear_plan(int64_t M, int64_t N, int64_t K, int heads_of_128, int sms, int* width, int* sharing);
 int kd_debug_linear_pair(int64_t M, int64_t N, int64_t K, int heads_of_128, int sms, int* pair);
+int kd_debug_linear_few_plan(int64_t M, int64_t N, int64_t K, int sms, int* ctas, int* rows);
 int kd_debug_matmul_f32_plan(int64_t batches, int64_t M, int64_t N, int64_t K, int sms, int* width, int* splits);
 int kd_debug_recurrence_plan(int delta, int bf16, int dim, int vdim, int heads, int tokens, int sms, int* records, int* ctas);
 int kd_empty_cache(void);

@@ -57,6 +57,12 @@ int gemm_skinny_auto_splits(int N, int K);
 int gemm_bf16_skinny(const void* x, int64_t ldx, const void* W, int64_t ldw, int Mb, int N, int K, int splits,
                      float* out_f32, void* out_bf16, int glu, float alpha = 1.0f, float* tail = nullptr, int tail_row = 0,
                      int ld_tail = 0, int groups = 1);
+// x [M <= 32, K] * W[N, K]^T by all SMs at once (linear_few.cu), where linear_few_rows says so.  Pointers 16-byte aligned, W dense.  epi: KD_EPI_NONE,
+// KD_EPI_RESIDUAL (resid of the output's type, ldr), KD_EPI_SWIGLU, KD_EPI_GEGLU, or LINEAR_FEW_TANH; columns from tail_col on go to `tail` in fp32.
+constexpr int LINEAR_FEW_TANH = 6;
+bool linear_few_rows(int64_t M, int64_t N, int64_t K);
+int linear_few(const void* x, int64_t ldx, const void* w, void* out, int64_t ldo, int out_f32, const void* resid, int64_t ldr, int M, int N, int K, int epi,
+               float* tail = nullptr, int tail_col = 0, int64_t ld_tail = 0);
 size_t attention_decode_scratch_bytes(int B, int Hkv, int group, int splits, int D);
 int attention_decode(const kd_tensor* q, const kd_tensor* k, const kd_tensor* v, const kd_tensor* out, float scale,
                      const int* ctx_dev, int ctx_host, const int* block_table, int max_pages, int splits,

@@ -373,6 +373,7 @@ KD_API int kd_linear_glu(const kd_tensor* x, const kd_tensor* weight, int epilog
   KD_TRY(tensor_ptr(weight, &pw));
   KD_TRY(tensor_ptr(out, &po));
   if (x->dtype == KD_BF16 && K % 8 == 0 && ((reinterpret_cast<uintptr_t>(px) | reinterpret_cast<uintptr_t>(pw) | reinterpret_cast<uintptr_t>(po)) & 15) == 0) {
+    if (linear_few_rows(M, N, K)) return linear_few(px, K, pw, po, N / 2, 0, nullptr, 0, (int)M, (int)N, (int)K, epilogue);
     // a handful of rows: the kernel that streams the weights, where its 128-row tiles are enough to fill the GPU
     if (M <= 64 && N >= 128ll * (ctx().sm_count / 2))
       return gemm_bf16_skinny(px, K, pw, K, (int)M, (int)N, (int)K, 1, nullptr, po, epilogue == KD_EPI_GEGLU ? 2 : 1);

@@ -668,7 +668,7 @@ class HybridEngine(DecoderEngine):
         return d
 
     def _enqueue_decode_step(self, d: dict) -> None:
-        lib.call("kd_set_pdl", 1 if self.use_pdl else 0)
+        lib.call("kd_set_pdl", 3 if self.use_pdl else 0)      # linears fetch their first weights while the kernel before drains
         try:
             h = self._run(d["ws"], d["ids"], d["B"], 1, d["pos"], 0)
             self._logits(d["ws"], h, d["logits"])

@@ -118,6 +118,7 @@ _SIGNATURES = {
     "kd_workspace_bytes": [ctypes.POINTER(_u64)],
     "kd_debug_fill_scratch": [ctypes.c_int],
     "kd_debug_linear_pair": [ctypes.c_int64] * 3 + [ctypes.c_int] * 2 + [ctypes.POINTER(ctypes.c_int)],
+    "kd_debug_linear_few_plan": [ctypes.c_int64] * 3 + [ctypes.c_int] + [ctypes.POINTER(ctypes.c_int)] * 2,
     "kd_debug_linear_plan": [ctypes.c_int64] * 3 + [ctypes.c_int] * 2 + [ctypes.POINTER(ctypes.c_int)] * 2,
     "kd_debug_matmul_f32_plan": [ctypes.c_int64] * 4 + [ctypes.c_int] + [ctypes.POINTER(ctypes.c_int)] * 2,
     "kd_debug_recurrence_plan": [ctypes.c_int] * 7 + [ctypes.POINTER(ctypes.c_int)] * 2,
