@@ -503,7 +503,8 @@ int kd_whisper_encoder_layers(const kd_tensor* const* layer_tensors, int n_layer
  *   layer_tensors   per layer: input norm [H], W_qkv [(Hq+2Hkv)128,H], q norm [128], k norm [128], W_o [H,Hq*128], post norm [H],
  *                   W_gate_up [2I,H] (16 gate rows, 16 up rows in turn), W_down [H,I], K cache, V cache; bf16, contiguous
  *                   (caches: [B>=M,Hkv,maxS,128], or pools [pages,Hkv,128,128] with block_table int32 [B>=M,max_pages])
- *   ids int64 [M], inv_freq fp32 [64], pos and ctx_len int32 scalars on the device, logits fp32 [M,V]
+ *   ids int64 [M], inv_freq fp32 [64], pos and ctx_len int32 scalars on the device, logits fp32 [M,V]; next_ids int64 [M] or NULL:
+ *                   the greedy next tokens, as kd_argmax of the logits gives them (may be ids)
  *   state           this caller's own hand-over words: kd_decode_step_state_bytes bytes, zero before the first step and then
  *                   left alone; steps that may run at the same time need a state each
  * kd_decode_step_state_bytes gives 0 for shapes that this form does not take: it takes 1 to 6 sequences whose activations
@@ -515,7 +516,7 @@ int kd_decode_step_state_bytes(int sequences, int hidden, int inter, int q_heads
                                int grid, uint64_t* bytes_out);
 int kd_decode_step(const kd_tensor* const* layer_tensors, int n_layers, const kd_tensor* embed, const kd_tensor* final_norm,
                    const kd_tensor* ids, const kd_tensor* inv_freq, const kd_tensor* pos, const kd_tensor* ctx_len, float eps,
-                   float scale, const kd_tensor* block_table, const kd_tensor* state, const kd_tensor* logits);
+                   float scale, const kd_tensor* block_table, const kd_tensor* state, const kd_tensor* logits, const kd_tensor* next_ids);
 /* The tensor-parallel form (no counterpart in the reference): every rank passes ITS slices (W_o and
  * W_down: input columns; W_gate_up and W_qkv_next: rows; attn, caches and q_out: its heads) and the
  * same residual; the partial sums of o_proj and down_proj are exchanged INSIDE the kernel, unit by

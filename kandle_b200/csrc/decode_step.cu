@@ -75,6 +75,8 @@ struct DsParams {
   const int* table;           // paged cache (null: contiguous)
   int* err;
   unsigned* state;            // [0] steps done, [1] tickets of the step that runs
+  u64* best;                  // [M] largest logit so far of the step that runs (ds_key), zero between steps
+  int64_t* next;              // [M] greedy next tokens, or null
   u64 *qkv, *part, *attn, *h1, *act, *h2;     // tagged words
   int64_t kc_b, kc_h, kc_s;
   float eps, scale_log2;
@@ -136,6 +138,13 @@ __device__ __forceinline__ float ds_hi(uint32_t v) { return __uint_as_float(v & 
 __device__ __forceinline__ uint32_t ds_pack(float a, float b) {
   const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<const uint32_t*>(&h);
+}
+// A logit and its column as a number that is larger for the larger logit and, among equals, the lower column; 0 for what is no maximum
+// of anything (argmax_kernel's rule: compared with the lowest float by `greater than`).
+__device__ __forceinline__ u64 ds_key(float v, int column) {
+  if (!(v > -3.402823466e38f)) return 0;
+  const uint32_t b = __float_as_uint(v + 0.0f);          // (-0 is 0)
+  return (u64)(b & 0x80000000u ? ~b : b | 0x80000000u) << 32 | (0xffffffffu - (uint32_t)column);
 }
 template <int LANES>
 __device__ __forceinline__ float ds_sum(float v) {        // over groups of lanes
@@ -339,6 +348,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
     ds_bar();
 
     int flip = 0;                                            // which of the two reduction buffers
+    u64 top = 0;                                             // of the logits that this thread has stored, all of sequence t / 64
     const float inv_h = 1.0f / (float)p.H;
     const int nqkv = (p.Hq + 2 * p.Hkv) * 128;
     const bool x_mine = (lane >> 2) < M;
@@ -688,10 +698,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
               const float v = total(m, r);
               if (hidden) {
                 const float y = v * inv_rms(norm_flip, m);
-                if (out) {
-                  if (phase == DS_QKV) out_s[m * 64 + r] = __float_as_uint(y);
-                  else p.logits[(size_t)m * p.V + n0 + b + r] = y;
-                }
+                if (out) out_s[m * 64 + r] = __float_as_uint(y);
               } else if (out) {
                 float& h = hid[m * p.h_rows + b + r];                   // (always this thread's)
                 h += v;
@@ -700,28 +707,53 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
             }
           }
         }
-        if (phase != DS_HEAD) {
-          // together: stored by the warps that sum them, a step of one sequence took 550 us instead of 443
-          ds_bar();
-          const int m = t >> 6, r = t & 63, words = phase == DS_GU ? n / 2 : n;
-          if (m < M && r < words) {
+        // together: stored by the warps that sum them, a step of one sequence took 550 us instead of 443
+        ds_bar();
+        const int m = t >> 6, r = t & 63, words = phase == DS_GU ? n / 2 : n;
+        if (m < M && r < words) {
+          const uint32_t v = out_s[m * 64 + r];
+          if (phase == DS_HEAD) {
+            const u64 key = ds_key(__uint_as_float(v), n0 + b + r);
+            p.logits[(size_t)m * p.V + n0 + b + r] = __uint_as_float(v);
+            top = key > top ? key : top;
+          } else {
             u64* dst = phase == DS_QKV ? p.qkv + m * nqkv + n0 + b : phase == DS_GU ? p.act + m * (p.I / 2) + (n0 + b) / 2 : (phase == DS_O ? p.h1 : p.h2) + m * p.H + n0 + b;
-            ds_st(dst + r, out_s[m * 64 + r], tag);
+            ds_st(dst + r, v, tag);
           }
         }
         flip ^= 1;
       }
     }
+    if (p.next) {
+#pragma unroll
+      for (int x = 16; x > 0; x >>= 1) {
+        const u64 o = __shfl_xor_sync(0xffffffffu, top, x);
+        top = o > top ? o : top;
+      }
+      if (lane == 0 && (t >> 6) < M) atomicMax(p.best + (t >> 6), top);
+    }
   }
 
   __syncthreads();
-  if (t == 0) {
-    const unsigned n = atomicAdd(p.state + 1, 1u);
-    if (n == (unsigned)G - 1) {                    // every CTA has read the step's position and tag
-      p.state[1] = 0u;
-      p.state[0] += 1u;
-      *p.pos += 1;
-      *p.ctx += 1;
+  if (warp == 0) {
+    unsigned n = 0;
+    if (lane == 0) {
+      __threadfence();                             // (this CTA's shares of `best`, ordered before its ticket)
+      n = atomicAdd(p.state + 1, 1u);
+      __threadfence();
+    }
+    n = __shfl_sync(0xffffffffu, n, 0);
+    if (n == (unsigned)G - 1) {                    // every CTA has read the step's position, tokens and tag
+      if (p.next && lane < M) {
+        const u64 key = atomicExch(p.best + lane, 0ull);
+        p.next[lane] = key ? (int64_t)(0xffffffffu - (uint32_t)key) : 0;
+      }
+      if (lane == 0) {
+        p.state[1] = 0u;
+        p.state[0] += 1u;
+        *p.pos += 1;
+        *p.ctx += 1;
+      }
     }
   }
 }
@@ -799,7 +831,7 @@ KD_API int kd_decode_step_state_bytes(int sequences, int hidden, int inter, int 
 
 KD_API int kd_decode_step(const kd_tensor* const* layer_tensors, int n_layers, const kd_tensor* embed, const kd_tensor* final_norm,
                           const kd_tensor* ids, const kd_tensor* inv_freq, const kd_tensor* pos, const kd_tensor* ctx_len, float eps,
-                          float scale, const kd_tensor* block_table, const kd_tensor* state, const kd_tensor* logits) {
+                          float scale, const kd_tensor* block_table, const kd_tensor* state, const kd_tensor* logits, const kd_tensor* next_ids) {
   KD_TRY(require_init());
   KD_REQUIRE(layer_tensors && embed && final_norm && ids && inv_freq && pos && ctx_len && state && logits, "null tensor");
   KD_REQUIRE(n_layers >= 1 && n_layers <= DS_MAX_LAYERS, "decode step: %d layers; this path takes 1..%d", n_layers, DS_MAX_LAYERS);
@@ -826,6 +858,7 @@ KD_API int kd_decode_step(const kd_tensor* const* layer_tensors, int n_layers, c
   KD_REQUIRE(ds_dense(ids, KD_I64, s.M) && ds_dense(inv_freq, KD_F32, 64) && pos->dtype == KD_I32 && numel(pos) == 1 && ctx_len->dtype == KD_I32 && numel(ctx_len) == 1,
              "decode step: ids int64 [M], inv_freq fp32 [64], position and context length int32 scalars");
   KD_REQUIRE(ds_dense(logits, KD_F32, (int64_t)s.M * s.V), "decode step: logits must be contiguous fp32 [M,V]");
+  KD_REQUIRE(!next_ids || ds_dense(next_ids, KD_I64, s.M), "decode step: next_ids must be int64 [M]");
   KD_REQUIRE(is_contiguous(state) && (uint64_t)numel(state) * dtype_size(state->dtype) >= plan.state_bytes, "decode step: state must hold %llu bytes",
              (unsigned long long)plan.state_bytes);
   if (block_table)
@@ -856,7 +889,7 @@ KD_API int kd_decode_step(const kd_tensor* const* layer_tensors, int n_layers, c
     const auto w = [&](int i) { return static_cast<const __nv_bfloat16*>(q[i]); };
     p.layer[l] = DsLayer{w(0), w(1), w(2), w(3), w(4), w(5), w(6), w(7), static_cast<__nv_bfloat16*>(q[8]), static_cast<__nv_bfloat16*>(q[9])};
   }
-  void *pe, *pf, *pi, *pv, *pp, *pc, *ps, *pl, *pt = nullptr;
+  void *pe, *pf, *pi, *pv, *pp, *pc, *ps, *pl, *pt = nullptr, *pn = nullptr;
   KD_TRY(ds_ptr(embed, "the embedding", &pe));
   KD_TRY(ds_ptr(final_norm, "the final norm", &pf));
   KD_TRY(tensor_ptr(ids, &pi));
@@ -866,6 +899,7 @@ KD_API int kd_decode_step(const kd_tensor* const* layer_tensors, int n_layers, c
   KD_TRY(ds_ptr(state, "the state", &ps));
   KD_TRY(tensor_ptr(logits, &pl));
   if (block_table) KD_TRY(tensor_ptr(block_table, &pt));
+  if (next_ids) KD_TRY(tensor_ptr(next_ids, &pn));
   p.embed = p.head = static_cast<const __nv_bfloat16*>(pe);
   p.final_norm = static_cast<const __nv_bfloat16*>(pf);
   p.ids = static_cast<const int64_t*>(pi);
@@ -878,6 +912,8 @@ KD_API int kd_decode_step(const kd_tensor* const* layer_tensors, int n_layers, c
   p.max_s = block_table ? p.max_pages * 128 : (int)kc0->shape[2];
   p.err = c.error_flag;
   p.state = static_cast<unsigned*>(ps);
+  p.best = reinterpret_cast<u64*>(static_cast<char*>(ps) + 64);
+  p.next = static_cast<int64_t*>(pn);
   u64* words = reinterpret_cast<u64*>(static_cast<char*>(ps) + 256);
   u64** to[6] = {&p.qkv, &p.part, &p.attn, &p.h1, &p.act, &p.h2};
   for (int i = 0; i < 6; ++i) {

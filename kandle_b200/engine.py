@@ -515,10 +515,12 @@ class Qwen3Engine(DecoderEngine):
         eps = ctypes.c_float(c.rmsNormEps)
         if d["step"] is not None:
             lib.call("kd_decode_step", self._layer_refs(), self.L, _r(self.embed), _r(self.final_norm), _r(d["ids"]), _r(self.inv_freq), _r(d["pos"]),
-                     _r(d["ctx"]), eps, ctypes.c_float(self.scale), _r(self.block_table), _r(d["step"]), _r(d["logits"]))
-            lg = d["logits"].view(B, self.V)
-            self._next_tokens(lg, d["uniforms"], d["ids"])
-            lg.dispose()
+                     _r(d["ctx"]), eps, ctypes.c_float(self.scale), _r(self.block_table), _r(d["step"]), _r(d["logits"]),
+                     _r(d["ids"]) if self.sampler is None else None)
+            if self.sampler is not None:
+                lg = d["logits"].view(B, self.V)
+                self._next_tokens(lg, d["uniforms"], d["ids"])
+                lg.dispose()
             return
         core._kernel("index_select")(self.embed._handle, d["ids"]._handle, {"dim": 0}, d["emb"]._handle)
         core.copy_(d["h"], d["emb"])

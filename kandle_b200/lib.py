@@ -159,7 +159,7 @@ _SIGNATURES = {
     "kd_decode_layer_chain": [_T, _T, _T, _T, _T, _T, _T, ctypes.c_float, _T, _T, _T, _T, _T, _T],
     "kd_decode_layer_fused": [_T, _T, _T, _T, _T, _T, _T, ctypes.c_float, _T, _T, _T, _T, _T, _T, _T, _T, _T, _T, _T, _T],
     "kd_decode_layer_fused_tp": [_T, _T, _T, _T, _T, _T, _T, ctypes.c_float, _T, _T, _T, _T, _T, _T, _T, _T, _T, _T, _T, _T],
-    "kd_decode_step": [_REFS, ctypes.c_int] + [_T] * 6 + [ctypes.c_float] * 2 + [_T] * 3,
+    "kd_decode_step": [_REFS, ctypes.c_int] + [_T] * 6 + [ctypes.c_float] * 2 + [_T] * 4,
     "kd_qwen3_prompt_layers": [_REFS, ctypes.c_int] + [_T] * 8 + [ctypes.c_float] * 2,
     "kd_whisper_encoder_layers": [_REFS, ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_float), ctypes.c_float, _T, _T],
     "kd_decode_step_state_bytes": [ctypes.c_int] * 9 + [ctypes.POINTER(_u64)],

@@ -35,8 +35,9 @@ def _forced(eng, ids, prompt, use_graph):
     out = []
     for t in range(STEPS):
         eng.start_decode(Tensor(ids[:, prompt + t].astype(np.int64)), use_graph)
-        eng.decode_step()
+        tokens = eng.decode_step().dataAsync()
         out.append(eng._decode["logits"].dataAsync()[0])
+        assert np.array_equal(tokens, out[-1].argmax(-1))
     return np.stack(out, 1)
 
 
@@ -72,6 +73,19 @@ def test_step_kernel_on_a_paged_cache(backend):
     assert flat._decode["step"] is not None and paged._decode["step"] is not None and np.array_equal(a, b)
     flat.dispose()
     paged.dispose()
+
+
+def test_the_lowest_of_equal_logits_is_the_next_token(backend):
+    eng, w = _engine((2, 512, 512, 4, 2, 9))
+    rows = w["model.embed_tokens.weight"].copy()
+    rows[500:] = rows[:500]
+    eng.embed = Tensor(rows, dtype="bfloat16")
+    got = _forced(eng, synth.token_ids("step.ids", (2, 9 + STEPS), 1000), 9, True)
+    assert np.array_equal(got[..., :500], got[..., 500:])                  # (and _forced has compared the tokens)
+    eng.dispose()
+    eng.embed = Tensor(np.zeros_like(rows), dtype="bfloat16")
+    assert not _forced(eng, synth.token_ids("step.ids", (2, 9 + STEPS), 1000), 9, True).any()
+    eng.dispose()
 
 
 def test_step_kernel_reports_bad_tokens_and_positions(backend):
