@@ -225,7 +225,8 @@ flash_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  if (DECODE) pdl_trigger();   // after the TMEM allocation
+  if (!DECODE) pdl_wait();      // nothing above touches global memory
+  pdl_trigger();                // after the TMEM allocation
 
   if (warp == 0) {
     if (lane == 0) {
@@ -565,7 +566,7 @@ flash_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const
         l *= alpha;
       }
       // P = exp2(s - m_used) as packed bf16 into the first 64 columns of this S buffer
-      float sum0 = 0.f, sum1 = 0.f;
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
       for (int c = 0; c < CW / 64; ++c) {
         uint32_t pk[32];
@@ -574,14 +575,14 @@ flash_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const
           const int e = c * 64 + 2 * i;
           const float p0 = fast_exp2(fmaf(__uint_as_float(sr[e >> 5][e & 31]), p.scale_log2, -m_used));
           const float p1 = fast_exp2(fmaf(__uint_as_float(sr[(e + 1) >> 5][(e + 1) & 31]), p.scale_log2, -m_used));
-          sum0 += p0;
-          sum1 += p1;
+          sum[2 * (i & 1)] += p0;
+          sum[2 * (i & 1) + 1] += p1;
           __nv_bfloat162 v = __floats2bfloat162_rn(p0, p1);
           pk[i] = *reinterpret_cast<uint32_t*>(&v);
         }
         tmem_st_32x32(s_addr + wg * (CW / 2) + c * 32, pk);
       }
-      l += sum0 + sum1;
+      l += (sum[0] + sum[1]) + (sum[2] + sum[3]);
       tmem_wait_st();
       tc_fence_before();
       __syncwarp();
@@ -699,12 +700,22 @@ static int launch_fa(const CUtensorMap& tq, const CUtensorMap& tk, const CUtenso
     configured[ctx().device & 63] = true;
   }
   if (DECODE) KD_CUDA_CHECK(launch_ex(flash_attention_tcgen05_kernel<D, DECODE>, grid, dim3(FA_THREADS), (size_t)SMEM, tq, tk, tv, p));
-  else flash_attention_tcgen05_kernel<D, DECODE><<<grid, FA_THREADS_PREFILL, SMEM, ctx().stream>>>(tq, tk, tv, p);
+  else KD_CUDA_CHECK(launch_ex(flash_attention_tcgen05_kernel<D, DECODE>, grid, dim3(FA_THREADS_PREFILL), (size_t)SMEM, tq, tk, tv, p));
   return after_launch(DECODE ? "flash_attention_tcgen05_kernel<decode>" : "flash_attention_tcgen05_kernel");
 }
 
 // attention_prefill2.cu: two query sub-tiles per CTA share each K/V tile.
 int attention_prefill2(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnParams& a, void* out);
+
+// Whether the kernel that shares K/V tiles between two query sub-tiles of a CTA takes the call: it reads K and V half as often and
+// keeps the tensor pipe busy during a softmax, but leaves SMs idle where one tile a CTA is a single wave (us, two tiles and one: 16 heads of
+// 128, causal, 1 x 300 12.5, 10.5; 1 x 1024 24.1, 16.8; 2 x 700 18.7, 20.8; 3 x 701 20.7, 24.9; 12 heads of 64, 1 x 1500 28.5, 20.6;
+// 2 x 750 17.9, 14.5; 2 x 1500 28.9, 37.1).  Single query tiles gain nothing from the other kernel (1 x 20 8.5, 9.1; 8 x 97 9.2, 9.5).
+static bool attention_two_tiles(const AttnParams& a, int sms) {
+  const int64_t tiles = (a.Sq + FA_BQ - 1) / FA_BQ;
+  if ((a.Hq / a.Hkv) % 2 != 0 && tiles == 1) return false;      // one query tile per KV head
+  return tiles == 1 || tiles * a.Hq * a.B > sms;
+}
 
 int attention_tc_try(const kd_tensor* q, const kd_tensor* k, const kd_tensor* v, const kd_tensor* out,
                      const AttnParams& a, int* handled) {
@@ -732,10 +743,9 @@ int attention_tc_try(const kd_tensor* q, const kd_tensor* k, const kd_tensor* v,
   KD_TRY(make_tmap_bhsd(&tq, pq, eq, a.sq, FA_BQ));
   KD_TRY(make_tmap_bhsd(&tk, pk, ek, a.sk, FA_BKV));
   KD_TRY(make_tmap_bhsd(&tv, pv, ek, a.sv, FA_BKV));
-  // More than one query tile per KV head: the kernel that shares K/V tiles between two sub-tiles.
   // KD_ATTENTION_ONE_TILE=1 in the environment keeps the one-tile kernel (for comparisons).
   static const bool one_tile = [] { const char* e = getenv("KD_ATTENTION_ONE_TILE"); return e && e[0] == '1'; }();
-  if (!one_tile && ((a.Hq / a.Hkv) % 2 == 0 || a.Sq > FA_BQ)) {
+  if (!one_tile && attention_two_tiles(a, ctx().sm_count)) {
     KD_TRY(attention_prefill2(tq, tk, tv, a, po));
     *handled = 1;
     return KD_OK;
