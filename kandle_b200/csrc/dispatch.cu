@@ -71,6 +71,9 @@ KD_API int kd_linear_bf16(const kd_tensor* x, const kd_tensor* weight, const kd_
                "residual must be contiguous, of the output's shape and dtype");
     KD_TRY(tensor_ptr(residual, &pr));
   }
+  if (weight->strides[0] == K && (epilogue != KD_EPI_SWIGLU || (N % 32 == 0 && out->dtype == KD_BF16)) && linear_few_rows(M, N, K) &&
+      ((reinterpret_cast<uintptr_t>(px) | reinterpret_cast<uintptr_t>(pw) | reinterpret_cast<uintptr_t>(pr) | reinterpret_cast<uintptr_t>(po)) & 15) == 0)
+    return linear_few(px, K, pw, po, n_out, out->dtype == KD_F32, pr, N, (int)M, (int)N, (int)K, epilogue);
   return gemm_bf16(px, K, pw, weight->strides[0], po, n_out, out->dtype == KD_F32, pr, N, (int)M, (int)N, (int)K, epilogue);
 }
 

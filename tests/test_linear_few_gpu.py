@@ -88,6 +88,9 @@ def test_results(backend, M, N, K):
     out = core.full((M, N), float("nan"), "bfloat16")
     lib.call("kd_linear_ex", _r(tx), _r(tw), None, F(1.0), _r(out), None)
     _close(out.dataAsync(), y, 2.0 ** -8)
+    dense, r16 = _put(x), _bf((M, N), 4)                                     # (the linear that prompts use)
+    lib.call("kd_linear_bf16", _r(dense), _r(tw), _r(_put(r16)), 1, _r(out))
+    _close(out.dataAsync(), y + r16, 2.0 ** -8)
     lib.call("kd_linear_tanh", _r(tx), _r(tw), _r(out))
     _close(out.dataAsync(), np.tanh(y), 2.0 ** -8)
     n = N // 64 * 32
@@ -106,6 +109,10 @@ def test_gated_results(backend, M, ff, K, epilogue):
     x, g, u = _bf((M, K), 5), _bf((ff, K), 6, 2 * K ** -0.5), _bf((ff, K), 7, K ** -0.5)
     out = core.full((M, ff), float("nan"), "bfloat16")
     lib.call("kd_linear_glu", _r(_put(x)), _r(_put(interleave_gate_up(g, u))), epilogue, _r(out))
+    if epilogue == 2:
+        again = core.full((M, ff), float("nan"), "bfloat16")
+        lib.call("kd_linear_bf16", _r(_put(x)), _r(_put(interleave_gate_up(g, u))), None, 2, _r(again))
+        assert np.array_equal(again.dataAsync(), out.dataAsync())
     xd = x.astype(np.float64)
     want = (vogozen.silu if epilogue == 2 else vogozen.gelu_tanh)(xd @ g.T) * (xd @ u.T)
     assert (np.abs(out.dataAsync() - want) <= 2.0 ** -8 * np.abs(want) + 2e-5 * np.abs(want).max()).all()
