@@ -8,7 +8,7 @@
 // Structure (one persistent CTA per SM, 192 threads):
 //   warp 0      TMA producer: 128x64 A tile + BLOCK_Nx64 W tile per stage, 128-byte swizzle,
 //               mbarrier complete_tx; loads are plain tiled loads (no cluster multicast).
-//   warp 1      one elected thread issues tcgen05.mma (M=128, N=BLOCK_N, K=16 x4 per stage) into a
+//   warp 1      an elected lane issues tcgen05.mma (M=128, N=BLOCK_N, K=16 x4 per stage) into a
 //               TMEM accumulator; tcgen05.commit releases the smem stage / publishes the tile.
 //   Few rows: a cluster of 2 or 4 CTAs shares a tile, each a range of k-blocks; the first adds the others' sums to its own
 //   and has the epilogue (linear_tile).
@@ -78,6 +78,23 @@ int make_tmap_bf16_3d(CUtensorMap* out, const void* base, uint64_t d2, uint64_t 
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(KD_ERR_CUDA, "cuTensorMapEncodeTiled (3-D) failed with code %d", (int)r);
+  return KD_OK;
+}
+
+// The same matrix as [K / 64][rows][64] (K a multiple of 64): one copy brings in `depth` k-blocks, each as the MMA wants it.
+static int make_tmap_bf16_blocks(CUtensorMap* out, const void* base, uint64_t rows, uint64_t K, uint64_t row_stride, uint32_t box_rows, uint32_t depth) {
+  EncodeTiledFn fn = encode_fn();
+  if (!fn) return fail(KD_ERR_CUDA, "cuTensorMapEncodeTiled is not available from the driver");
+  KD_REQUIRE((reinterpret_cast<uintptr_t>(base) & 15) == 0, "TMA base address must be 16-byte aligned");
+  KD_REQUIRE((row_stride * 2) % 16 == 0 && K % 64 == 0, "TMA strides must be multiples of 16 bytes");
+  cuuint64_t gdim[3] = {64, rows, K / 64};
+  cuuint64_t gstr[2] = {row_stride * 2, 128};
+  cuuint32_t box[3] = {64, box_rows, depth};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUresult r = fn(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), gdim, gstr, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(KD_ERR_CUDA, "cuTensorMapEncodeTiled (k-blocks) failed with code %d", (int)r);
   return KD_OK;
 }
 
@@ -297,60 +314,69 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
     w_row = lo * p.N;
   };
 
+  // Warps 0 and 1 walk through the k-blocks as whole warps and an elected lane issues copies and MMAs, so that addresses and
+  // descriptors stay in uniform registers: with a loop inside `if (lane == 0)` a k-block took its warp 0.29 us whatever the
+  // width of the tile, now 0.22.  Prompts of 97 and 3 x 701 tokens: 1774 and 3384 us before, 1650 and 3232 now; 32 x 2048: 0.8 % less.
   if (warp == 0) {
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int tile = first; ok && tile < total_tiles; tile += step) {
-        const int m_tile = tile / p.num_n_tiles, n_tile = tile - m_tile * p.num_n_tiles;
-        int row0, row_end, w_row;
-        locate(m_tile, row0, row_end, w_row);
-        for (int kb = kb_begin; kb < kb_end; ++kb) {
-          uint8_t* sa = smem + stage * STAGE_BYTES;
-          if (early > 0) {                               // (the first stages: W is on its way)
-            --early;
-            load(sa, &tmap_a, stage, kb * GEMM_BK, row0);
-          } else {
-            if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.err, 201)) { ok = false; break; }
-            expect(stage);
-            load(sa, &tmap_a, stage, kb * GEMM_BK, row0);
-            load(sa + A_BYTES, &tmap_b, stage, kb * GEMM_BK, w_row + n_tile * BLOCK_N + (int)pair_rank * (BLOCK_N / 2));
-          }
-          if (++stage == STAGES) { stage = 0; phase ^= 1; }
+    early = __shfl_sync(0xffffffffu, early, 0);
+    int stage = 0;
+    uint32_t phase = 0;
+    bool ok = true;
+    for (int tile = first; ok && tile < total_tiles; tile += step) {
+      const int m_tile = tile / p.num_n_tiles, n_tile = tile - m_tile * p.num_n_tiles;
+      int row0, row_end, w_row;
+      locate(m_tile, row0, row_end, w_row);
+      for (int kb = kb_begin; kb < kb_end; ++kb) {
+        uint8_t* sa = smem + stage * STAGE_BYTES;
+        const bool w_here = early > 0;                   // (the first stages: W is on its way)
+        if (w_here) --early;
+        else ok = __all_sync(0xffffffffu, mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.err, 201));
+        if (!ok) break;
+        if (elect_one()) {
+          if (!w_here) expect(stage);
+          load(sa, &tmap_a, stage, kb * GEMM_BK, row0);
+          if (!w_here) load(sa + A_BYTES, &tmap_b, stage, kb * GEMM_BK, w_row + n_tile * BLOCK_N + (int)pair_rank * (BLOCK_N / 2));
         }
+        __syncwarp();
+        if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && pair_rank == 0) {
+    if (pair_rank == 0) {
+      const uint64_t adesc0 = make_smem_desc_sw128(smem_u32(smem), 16, 1024), bdesc0 = make_smem_desc_sw128(smem_u32(smem + A_BYTES), 16, 1024);
       int stage = 0;
       uint32_t phase = 0;
       int acc = 0;
       uint32_t acc_phase = 0;
       bool ok = true;
       for (int tile = first; ok && tile < total_tiles; tile += step) {
-        if (!mbar_wait(&tmem_empty[acc], acc_phase ^ 1, abort_flag, p.err, 202)) break;
+        ok = __all_sync(0xffffffffu, mbar_wait(&tmem_empty[acc], acc_phase ^ 1, abort_flag, p.err, 202));
+        if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BLOCK_N);
         for (int kb = kb_begin; kb < kb_end; ++kb) {
-          if (!mbar_wait(&full[stage], phase, abort_flag, p.err, 203)) { ok = false; break; }
+          ok = __all_sync(0xffffffffu, mbar_wait(&full[stage], phase, abort_flag, p.err, 203));
+          if (!ok) break;
           tc_fence_after();
-          const uint32_t a_addr = smem_u32(smem + stage * STAGE_BYTES);
-          const uint32_t b_addr = a_addr + A_BYTES;
+          if (elect_one()) {
+            const uint64_t adesc = adesc0 + (uint32_t)(stage * (STAGE_BYTES >> 4)), bdesc = bdesc0 + (uint32_t)(stage * (STAGE_BYTES >> 4));
 #pragma unroll
-          for (int k = 0; k < GEMM_BK / 16; ++k) {
-            const uint64_t adesc = make_smem_desc_sw128(a_addr + k * 32, 16, 1024);
-            const uint64_t bdesc = make_smem_desc_sw128(b_addr + k * 32, 16, 1024);
-            if constexpr (PAIR) umma_ss_pair(d_tmem, adesc, bdesc, IDESC, ((kb - kb_begin) | k) != 0 ? 1u : 0u);
-            else umma_ss(d_tmem, adesc, bdesc, IDESC, ((kb - kb_begin) | k) != 0 ? 1u : 0u);
+            for (int k = 0; k < GEMM_BK / 16; ++k) {
+              if constexpr (PAIR) umma_ss_pair(d_tmem, adesc + k * 2, bdesc + k * 2, IDESC, ((kb - kb_begin) | k) != 0 ? 1u : 0u);
+              else umma_ss(d_tmem, adesc + k * 2, bdesc + k * 2, IDESC, ((kb - kb_begin) | k) != 0 ? 1u : 0u);
+            }
+            if constexpr (PAIR) umma_commit_pair(&empty[stage]);
+            else umma_commit(&empty[stage]);
           }
-          if constexpr (PAIR) umma_commit_pair(&empty[stage]);
-          else umma_commit(&empty[stage]);
+          __syncwarp();
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        if constexpr (PAIR) umma_commit_pair(&tmem_full[acc]);
-        else umma_commit(&tmem_full[acc]);
+        if (elect_one()) {
+          if constexpr (PAIR) umma_commit_pair(&tmem_full[acc]);
+          else umma_commit(&tmem_full[acc]);
+        }
+        __syncwarp();
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1;
       }
@@ -933,9 +959,20 @@ int gemm_bf16_qkv_rope(const void* A, int64_t lda, const void* W, int64_t ldw, i
 // The problem is HBM-bound (every weight byte is used once per step), so the kernel is organised
 // around streaming W: the operands are swapped, W rows become the M dimension of the MMA (128 rows
 // per CTA, all of them useful) and the few activation rows become the N dimension (16..128).  Each
-// stage then carries 16 KB of weights and only a few KB of activations, and a deep TMA ring keeps
-// ~100+ KB of weight traffic in flight per SM.  When N/128 gives too few CTAs the K range is split
-// across CTAs; every split writes fp32 partial sums [split][m][n], which the consumer kernels
+// k-block then carries 16 KB of weights and only a few KB of activations, and a deep TMA ring keeps
+// ~100+ KB of weight traffic in flight per SM.
+//
+// What bounds a CTA is not its copies but how fast one warp gets through a step of the ring: about 0.15 us to wait, expect
+// and start two copies, as much to wait, start four MMAs and commit.  So a step is two k-blocks where the ring has room for
+// that (one copy of each operand, from the matrix as [K / 64][rows][64]), and the loops run as whole warps of which an
+// elected lane issues (uniform registers).  Where there are more tiles than SMs, two CTAs share one (a shallower ring).
+// Microseconds, one k-block a step and a loop of one lane before / now (weights from HBM, in a programmatic chain):
+// 4 x 6144 x 4096 (rows x N x K) 22.3, 14.6; 32 x 6144 x 4096 24.5, 16.8; 32 x 12288 x 2048 16.2, 13.8; 32 x 6144 x 1024 10.3, 8.4;
+// 32 x 32768 x 2048 32.8, 26.0; 4 x 32768 x 1024 18.4, 14.1; 32 x 19456 x 2560 36.1, 23.4 (21.9 with one k-block a step);
+// 128 x 12288 x 2048 24.6, 23.1 (one k-block a step); 32 x 151936 x 1024 62.9, 60.9.
+//
+// When N/128 gives too few CTAs the K range is split across CTAs; every split writes fp32 partial sums [split][m][n],
+// which the consumer kernels
 // (norm+RoPE, SwiGLU, residual+RMSNorm) add up while they do their own work.
 // Roofline: HBM, N*K*2 bytes of weights per call.
 struct SkinnyParams {
@@ -943,6 +980,7 @@ struct SkinnyParams {
   int mb_pad;             // MMA N extent: multiple of 16 covering Mb
   int x_box;              // rows of the activation TMA box (smem rows per stage)
   int splits, kblocks_per_split, stages;
+  int blocked;            // K is a multiple of 64: a stage is one copy of each operand
   uint32_t tmem_cols;
   float* out_f32;         // [splits][Mb][N]
   int64_t ldo;            // row stride of out_bf16
@@ -955,12 +993,12 @@ struct SkinnyParams {
   int* err;
 };
 
+template <int PER_STAGE>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_skinny_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                            SkinnyParams p) {
-  constexpr int W_BYTES = 128 * GEMM_BK * 2;
-  const int x_bytes = p.x_box * GEMM_BK * 2;
-  const int stage_bytes = W_BYTES + x_bytes;
+  const int w_bytes = PER_STAGE * 128 * GEMM_BK * 2, x_bytes = p.x_box * GEMM_BK * 2;
+  const int stage_bytes = w_bytes + PER_STAGE * x_bytes;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + p.stages * stage_bytes);
@@ -996,37 +1034,50 @@ gemm_skinny_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const __g
   pdl_trigger();   // after the TMEM allocation (see common.cuh)
 
   if (warp == 0) {
-    if (lane == 0) {
-      int stage = 0;
-      uint32_t phase = 0;
-      for (int i = 0; i < n_kb; ++i) {
-        if (!mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.err, 211)) break;
-        uint8_t* sw = smem + stage * stage_bytes;
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int i = 0; i < n_kb; i += PER_STAGE) {
+      const bool ok = mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.err, 211);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      if (elect_one()) {
+        uint8_t *sw = smem + stage * stage_bytes, *sx = sw + w_bytes;
+        const int kb = kb_begin + i, w_row = group * p.N + n_tile * 128, x_row = group * p.Mb;
         mbar_arrive_expect_tx(&full[stage], (uint32_t)stage_bytes);
-        tma_load_2d(sw, &tmap_w, &full[stage], (kb_begin + i) * GEMM_BK, group * p.N + n_tile * 128);
-        tma_load_2d(sw + W_BYTES, &tmap_x, &full[stage], (kb_begin + i) * GEMM_BK, group * p.Mb);
-        if (++stage == p.stages) { stage = 0; phase ^= 1; }
+        if (p.blocked) {
+          tma_load_3d(sw, &tmap_w, &full[stage], 0, w_row, kb);
+          tma_load_3d(sx, &tmap_x, &full[stage], 0, x_row, kb);
+        } else {
+          for (int b = 0; b < PER_STAGE; ++b) {
+            tma_load_2d(sw + b * (128 * GEMM_BK * 2), &tmap_w, &full[stage], (kb + b) * GEMM_BK, w_row);
+            tma_load_2d(sx + b * x_bytes, &tmap_x, &full[stage], (kb + b) * GEMM_BK, x_row);
+          }
+        }
       }
+      __syncwarp();
+      if (++stage == p.stages) { stage = 0; phase ^= 1; }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      const uint32_t idesc = make_idesc_bf16(128, p.mb_pad, 0, 0);
-      int stage = 0;
-      uint32_t phase = 0;
-      bool ok = true;
-      for (int i = 0; i < n_kb; ++i) {
-        if (!mbar_wait(&full[stage], phase, abort_flag, p.err, 212)) { ok = false; break; }
-        tc_fence_after();
-        const uint32_t w_addr = smem_u32(smem + stage * stage_bytes);
-        const uint32_t x_addr = w_addr + W_BYTES;
+    const uint32_t idesc = make_idesc_bf16(128, p.mb_pad, 0, 0);
+    const uint64_t wdesc = make_smem_desc_sw128(smem_u32(smem), 16, 1024), xdesc = make_smem_desc_sw128(smem_u32(smem + w_bytes), 16, 1024);
+    int stage = 0;
+    uint32_t phase = 0;
+    for (int i = 0; i < n_kb; i += PER_STAGE) {
+      const bool ok = mbar_wait(&full[stage], phase, abort_flag, p.err, 212);
+      if (!__all_sync(0xffffffffu, ok)) break;
+      tc_fence_after();
+      if (elect_one()) {
+        const int valid = min(PER_STAGE, n_kb - i);      // (the blocks behind belong to the next split)
+        uint64_t wd = wdesc + (uint32_t)(stage * (stage_bytes >> 4)), xd = xdesc + (uint32_t)(stage * (stage_bytes >> 4));
 #pragma unroll
-        for (int k = 0; k < GEMM_BK / 16; ++k)
-          umma_ss(tmem_base, make_smem_desc_sw128(w_addr + k * 32, 16, 1024), make_smem_desc_sw128(x_addr + k * 32, 16, 1024),
-                  idesc, (i | k) != 0 ? 1u : 0u);
+        for (int b = 0; b < PER_STAGE; ++b, wd += 128 * GEMM_BK * 2 >> 4, xd += x_bytes >> 4)
+          if (b < valid)
+#pragma unroll
+          for (int k = 0; k < GEMM_BK / 16; ++k) umma_ss(tmem_base, wd + k * 2, xd + k * 2, idesc, (i | b | k) != 0 ? 1u : 0u);
         umma_commit(&empty[stage]);
-        if (++stage == p.stages) { stage = 0; phase ^= 1; }
+        if (i + PER_STAGE >= n_kb) umma_commit(acc_full);
       }
-      if (ok) umma_commit(acc_full);
+      __syncwarp();
+      if (++stage == p.stages) { stage = 0; phase ^= 1; }
     }
   } else {
     const int q = warp & 3;
@@ -1108,18 +1159,20 @@ int gemm_bf16_skinny(const void* x, int64_t ldx, const void* W, int64_t ldw, int
   SkinnyParams p{};
   p.Mb = Mb; p.N = N; p.K = K;
   p.mb_pad = (Mb + 15) / 16 * 16;
-  p.x_box = p.mb_pad <= 32 ? 32 : (p.mb_pad <= 64 ? 64 : 128);
-  const int total_kb = (K + GEMM_BK - 1) / GEMM_BK;
+  p.x_box = p.mb_pad <= 16 ? 16 : p.mb_pad <= 32 ? 32 : (p.mb_pad <= 64 ? 64 : 128);
+  const int total_kb = (K + GEMM_BK - 1) / GEMM_BK, tiles = (N + 127) / 128;
   if (splits > total_kb) splits = total_kb;
   p.kblocks_per_split = (total_kb + splits - 1) / splits;
   p.splits = splits;
-  const int stage_bytes = 128 * GEMM_BK * 2 + p.x_box * GEMM_BK * 2;
+  int per_stage = p.x_box <= 64 && p.kblocks_per_split > 1 ? 2 : 1;
+  p.blocked = K % GEMM_BK == 0;
+  const int stage_bytes = per_stage * (128 + p.x_box) * GEMM_BK * 2;
+  const int steps = (p.kblocks_per_split + per_stage - 1) / per_stage;
   int stages = (200 * 1024) / stage_bytes;
   if (stages > 10) stages = 10;
-  if (stages > p.kblocks_per_split) stages = p.kblocks_per_split < 2 ? 2 : p.kblocks_per_split;
-  // many tiles (lm_head): a shallower ring lets two CTAs share an SM, so that one CTA's prologue and
-  // epilogue overlap the other's streaming
-  if ((int64_t)((N + 127) / 128) * splits * groups >= 2 * ctx().sm_count) {
+  if (stages > steps) stages = steps < 2 ? 2 : steps;
+  // more tiles than SMs: a shallower ring lets two CTAs share an SM
+  if ((int64_t)tiles * splits * groups > ctx().sm_count) {
     const int two_per_sm = (108 * 1024) / stage_bytes;
     if (stages > two_per_sm) stages = two_per_sm;
   }
@@ -1131,19 +1184,25 @@ int gemm_bf16_skinny(const void* x, int64_t ldx, const void* W, int64_t ldw, int
   p.alpha = alpha;
   p.tail = tail; p.tail_row = tail_row; p.ld_tail = ld_tail;
   p.ldo = tail ? tail_row : N;
-  p.group_tiles = (N + 127) / 128;
+  p.group_tiles = tiles;
   p.err = ctx().error_flag;
   CUtensorMap tw, tx;
-  KD_TRY(make_tmap_bf16_2d(&tw, W, (uint64_t)N * groups, (uint64_t)K, (uint64_t)ldw, 128, GEMM_BK));
-  KD_TRY(make_tmap_bf16_2d(&tx, x, (uint64_t)Mb * groups, (uint64_t)K, (uint64_t)ldx, (uint32_t)p.x_box, GEMM_BK));
+  if (p.blocked) {
+    KD_TRY(make_tmap_bf16_blocks(&tw, W, (uint64_t)N * groups, (uint64_t)K, (uint64_t)ldw, 128, (uint32_t)per_stage));
+    KD_TRY(make_tmap_bf16_blocks(&tx, x, (uint64_t)Mb * groups, (uint64_t)K, (uint64_t)ldx, (uint32_t)p.x_box, (uint32_t)per_stage));
+  } else {
+    KD_TRY(make_tmap_bf16_2d(&tw, W, (uint64_t)N * groups, (uint64_t)K, (uint64_t)ldw, 128, GEMM_BK));
+    KD_TRY(make_tmap_bf16_2d(&tx, x, (uint64_t)Mb * groups, (uint64_t)K, (uint64_t)ldx, (uint32_t)p.x_box, GEMM_BK));
+  }
   const int smem = stages * stage_bytes + 1024 + 256;
   static bool skinny_configured[64] = {false};   // per device
   if (!skinny_configured[ctx().device & 63]) {
-    KD_CUDA_CHECK(cudaFuncSetAttribute(gemm_skinny_tcgen05_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
+    KD_CUDA_CHECK(cudaFuncSetAttribute(gemm_skinny_tcgen05_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
+    KD_CUDA_CHECK(cudaFuncSetAttribute(gemm_skinny_tcgen05_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 210 * 1024));
     skinny_configured[ctx().device & 63] = true;
   }
   dim3 grid(p.group_tiles * groups, splits);
-  KD_CUDA_CHECK(launch_ex(gemm_skinny_tcgen05_kernel, grid, dim3(GEMM_THREADS), (size_t)smem, tw, tx, p));
+  KD_CUDA_CHECK(launch_ex(per_stage == 2 ? gemm_skinny_tcgen05_kernel<2> : gemm_skinny_tcgen05_kernel<1>, grid, dim3(GEMM_THREADS), (size_t)smem, tw, tx, p));
   return after_launch("gemm_skinny_tcgen05_kernel");
 }
 
