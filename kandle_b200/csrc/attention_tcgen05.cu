@@ -268,27 +268,31 @@ flash_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      bool ok = mbar_wait(q_full, 0, abort_flag, p.err, 303);
+    {
+      auto wait = [&](uint64_t* bar, uint32_t parity, int code) { return (bool)__all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, p.err, code)); };
+      bool ok = wait(q_full, 0, 303);
       const uint32_t q_addr = smem_u32(q_smem);
       // S(j) = Q K(j)^T into S buffer j % NSBUF   (j counts this CTA's key tiles from 0)
       auto issue_qk = [&](int j) -> bool {
         const int t = 2 * j, stage = t % NSLOT;
-        if (!mbar_wait(&t_full[stage], (uint32_t)((t / NSLOT) & 1), abort_flag, p.err, 304)) return false;
+        if (!wait(&t_full[stage], (uint32_t)((t / NSLOT) & 1), 304)) return false;
         tc_fence_after();
         const uint32_t k_addr = smem_u32(ring + stage * KV_BYTES);
         const uint32_t d_tmem = tmem_base + S_COL0 + (uint32_t)((j % NSBUF) * BKV);
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t qoff = (uint32_t)((k / 4) * Q_SLAB + (k % 4) * 32);
-          const uint32_t koff = (uint32_t)((k / 4) * SLAB_BYTES + (k % 4) * 32);
+        if (elect_one()) {
           // colsplit: a stride of 0 between the 8-row groups of the A tile makes every group read rows
           // 0-7 of the Q tile, i.e. query r appears in S rows r, 8 + r, ..., 120 + r
-          umma_ss(d_tmem, make_smem_desc_sw128(q_addr + qoff, 16, (DECODE && p.colsplit) ? 0u : 1024u),
-                  make_smem_desc_sw128(k_addr + koff, 16, 1024), IDESC_QK, k != 0 ? 1u : 0u);
+          const uint64_t qdesc = make_smem_desc_sw128(q_addr, 16, (DECODE && p.colsplit) ? 0u : 1024u), kdesc = make_smem_desc_sw128(k_addr, 16, 1024);
+#pragma unroll
+          for (int k = 0; k < D / 16; ++k) {
+            const uint32_t qoff = (uint32_t)((k / 4) * Q_SLAB + (k % 4) * 32) >> 4;
+            const uint32_t koff = (uint32_t)((k / 4) * SLAB_BYTES + (k % 4) * 32) >> 4;
+            umma_ss(d_tmem, qdesc + qoff, kdesc + koff, IDESC_QK, k != 0 ? 1u : 0u);
+          }
+          umma_commit(&t_empty[stage]);
+          umma_commit(&s_full[j % NSBUF]);
         }
-        umma_commit(&t_empty[stage]);
-        umma_commit(&s_full[j % NSBUF]);
+        __syncwarp();
         return true;
       };
       if (ok) ok = issue_qk(0);
@@ -298,21 +302,22 @@ flash_attention_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_q, const
           if (!issue_qk(j + 1)) break;
         }
         const int t = 2 * j + 1, stage = t % NSLOT;
-        if (!mbar_wait(&p_ready[j % NSBUF], (uint32_t)((j / NSBUF) & 1), abort_flag, p.err, 305)) break;
-        if (!mbar_wait(&t_full[stage], (uint32_t)((t / NSLOT) & 1), abort_flag, p.err, 306)) break;
+        if (!wait(&p_ready[j % NSBUF], (uint32_t)((j / NSBUF) & 1), 305)) break;
+        if (!wait(&t_full[stage], (uint32_t)((t / NSLOT) & 1), 306)) break;
         tc_fence_after();
         const uint32_t v_addr = smem_u32(ring + stage * KV_BYTES);
         const uint32_t p_tmem = tmem_base + S_COL0 + (uint32_t)((j % NSBUF) * BKV);
         const uint32_t o_tmem = tmem_base + O_COL0;
-#pragma unroll
-        for (int k = 0; k < BKV / 16; ++k) {
+        if (elect_one()) {
           // V tile is [kv rows][64-wide d slabs]: MN-major B; 16 kv rows = 2048 bytes per k step
-          const uint64_t vdesc = make_smem_desc_sw128(v_addr + (uint32_t)(k * 2048), SLAB_BYTES, 1024);
-          umma_ts(o_tmem, p_tmem + (uint32_t)(k * 8), vdesc, IDESC_PV, (j | k) != 0 ? 1u : 0u);
+          const uint64_t vdesc = make_smem_desc_sw128(v_addr, SLAB_BYTES, 1024);
+#pragma unroll
+          for (int k = 0; k < BKV / 16; ++k) umma_ts(o_tmem, p_tmem + (uint32_t)(k * 8), vdesc + (uint32_t)(k * 128), IDESC_PV, (j | k) != 0 ? 1u : 0u);
+          umma_commit(&t_empty[stage]);
+          umma_commit(o_done);
+          if (j + 1 == n_blocks) umma_commit(o_final);
         }
-        umma_commit(&t_empty[stage]);
-        umma_commit(o_done);
-        if (j + 1 == n_blocks) umma_commit(o_final);
+        __syncwarp();
         // one S buffer: the next QK^T overwrites P, so it is issued after PV (in-order pipe)
         if (NSBUF == 1 && j + 1 < n_blocks) {
           if (!issue_qk(j + 1)) break;

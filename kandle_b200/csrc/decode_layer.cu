@@ -431,11 +431,12 @@ decode_layer_kernel(const __grid_constant__ DlMaps maps, const __grid_constant__
     }
   } else if (warp == 1 || warp == 6) {
     // ------------------------------------------------------------------ MMA issuers
-    // One thread issues a tcgen05.mma of this size every ~55-95 cycles however narrow it is, while
-    // the tensor pipe takes one every ~40-50: two issuing warps share a unit's k-blocks (even ones to
+    // A thread inside `if (lane == 0)` issues a tcgen05.mma of this size every ~55-95 cycles however narrow it is, while the
+    // tensor pipe takes one every ~40-50; an elected lane of a warp that walks through the loop as a whole (descriptors in
+    // uniform registers) one every 13.  Two issuing warps share a unit's k-blocks (even ones to
     // warp 1, odd ones to warp 6), each accumulating into its own half of the buffer; the epilogue
     // adds the halves.
-    if (lane == 0) {
+    {
       const int me = warp == 1 ? 0 : 1;
       int stage = 0;
       uint32_t ring_phase = 0;
@@ -453,12 +454,12 @@ decode_layer_kernel(const __grid_constant__ DlMaps maps, const __grid_constant__
         const uint32_t idesc = make_idesc_bf16(128, g.n_unit, 0, 0);
         for (int u = wk.first; ok && u < g.units && wk.kb0 < wk.kb1; u += wk.step) {
           const int buf = acc_n & 1, use = acc_n >> 1;
-          if (!mbar_wait(&acc_empty[buf], (uint32_t)((use & 1) ^ 1), abort_flag, p.err, 524)) { ok = false; break; }
+          if (!__all_sync(0xffffffffu, mbar_wait(&acc_empty[buf], (uint32_t)((use & 1) ^ 1), abort_flag, p.err, 524))) { ok = false; break; }
           tc_fence_after();
           const uint32_t d_tmem = tmem_base + (uint32_t)buf * 256u + (uint32_t)me * 128u;
           uint32_t acc = 0u;
           for (int kb = wk.kb0; kb < wk.kb1; kb += g.kg) {
-            if (!mbar_wait(&full[stage], ring_phase, abort_flag, p.err, 525)) { ok = false; break; }
+            if (!__all_sync(0xffffffffu, mbar_wait(&full[stage], ring_phase, abort_flag, p.err, 525))) { ok = false; break; }
             tc_fence_after();
             // an activation tile holds x_box rows; the MMA's other rows are read from whatever follows
             // it in the slot (later tiles, the weight area) and give accumulator rows of no sequence
@@ -466,20 +467,24 @@ decode_layer_kernel(const __grid_constant__ DlMaps maps, const __grid_constant__
             const int j0 = (kb + me) & 1 ? 1 : 0;          // this issuer's first k-block of the group: global index parity == me
             uint32_t xl = smem_lo + (uint32_t)(stage * (DL_SLOT >> 4)) + (uint32_t)j0 * x_step;
             uint32_t wl = smem_lo + (uint32_t)(stage * (DL_SLOT >> 4)) + (uint32_t)(DL_X_AREA >> 4) + (uint32_t)j0 * w_step;
-            for (int j = j0; j < nk; j += 2) {
-              umma_ss_lohi(d_tmem, xl, wl, DESC_HI, idesc, acc);
-              umma_ss_lohi(d_tmem, xl + 2, wl + 2, DESC_HI, idesc, 1u);
-              umma_ss_lohi(d_tmem, xl + 4, wl + 4, DESC_HI, idesc, 1u);
-              umma_ss_lohi(d_tmem, xl + 6, wl + 6, DESC_HI, idesc, 1u);
-              acc = 1u;
-              xl += 2 * x_step;
-              wl += 2 * w_step;
+            if (elect_one()) {
+              for (int j = j0; j < nk; j += 2) {
+                umma_ss_lohi(d_tmem, xl, wl, DESC_HI, idesc, j != j0 ? 1u : acc);
+                umma_ss_lohi(d_tmem, xl + 2, wl + 2, DESC_HI, idesc, 1u);
+                umma_ss_lohi(d_tmem, xl + 4, wl + 4, DESC_HI, idesc, 1u);
+                umma_ss_lohi(d_tmem, xl + 6, wl + 6, DESC_HI, idesc, 1u);
+                xl += 2 * x_step;
+                wl += 2 * w_step;
+              }
+              umma_commit(&empty[stage]);
             }
-            umma_commit(&empty[stage]);
+            __syncwarp();
+            if (j0 < nk) acc = 1u;
             if (++stage == DL_STAGES) { stage = 0; ring_phase ^= 1; }
           }
           if (!ok) break;
-          umma_commit(&acc_full[buf]);
+          if (elect_one()) umma_commit(&acc_full[buf]);
+          __syncwarp();
           ++acc_n;
         }
       }
