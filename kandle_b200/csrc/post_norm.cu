@@ -84,7 +84,9 @@ __device__ __forceinline__ float block_total(float v, float* red) {
 // NV chunks of four columns a thread.  Bound: the latency of its loads, so all of them are on their way at once (the weights, and up
 // to AHEAD partial sums beside the first): a decode step of the hybrid in 6 layers, 12 such kernels: 32 sequences of 2048
 // columns 502 -> 491 us, 4 of 1024 243 -> 237, against one partial sum after the other and the weights behind the sum.
-template <int NV>
+// With one partial sum (prompts: many rows, bound by HBM) the registers for that would only cost warps: 8192 rows of 2048, a
+// prompt of the hybrid in 6 layers 10.1 ms without, 10.9 with them.
+template <int NV, bool SPLIT>
 __global__ void __launch_bounds__(256) residual_post_norm_kernel(PostNormParams p) {
   __shared__ float red[2][32];
   pdl_wait();
@@ -98,29 +100,30 @@ __global__ void __launch_bounds__(256) residual_post_norm_kernel(PostNormParams 
     if (col < p.width) {
       load4(p.y, p.dt_y, row * p.width + col, y[i]);
       load4(p.x, KD_F32, row * p.width + col, x[i]);
-      load4(p.w, KD_F32, col, w[i]);
+      if (SPLIT) load4(p.w, KD_F32, col, w[i]);
     } else {
 #pragma unroll
       for (int e = 0; e < 4; ++e) x[i][e] = y[i][e] = 0.f;
     }
   }
-  for (int s = 1; s < p.splits; s += AHEAD) {
-    float t[AHEAD][NV][4];
+  if (SPLIT)
+    for (int s = 1; s < p.splits; s += AHEAD) {
+      float t[AHEAD][NV][4];
 #pragma unroll
-    for (int u = 0; u < AHEAD; ++u)
+      for (int u = 0; u < AHEAD; ++u)
 #pragma unroll
-      for (int i = 0; i < NV; ++i) {
-        const int col = (i * blockDim.x + threadIdx.x) * 4;
-        if (s + u < p.splits && col < p.width) load4(p.y, p.dt_y, ((int64_t)(s + u) * p.rows + row) * p.width + col, t[u][i]);
-      }
+        for (int i = 0; i < NV; ++i) {
+          const int col = (i * blockDim.x + threadIdx.x) * 4;
+          if (s + u < p.splits && col < p.width) load4(p.y, p.dt_y, ((int64_t)(s + u) * p.rows + row) * p.width + col, t[u][i]);
+        }
 #pragma unroll
-    for (int u = 0; u < AHEAD; ++u)
+      for (int u = 0; u < AHEAD; ++u)
 #pragma unroll
-      for (int i = 0; i < NV; ++i)
-        if (s + u < p.splits && (i * (int)blockDim.x + (int)threadIdx.x) * 4 < p.width)
+        for (int i = 0; i < NV; ++i)
+          if (s + u < p.splits && (i * (int)blockDim.x + (int)threadIdx.x) * 4 < p.width)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) y[i][e] += t[u][i][e];
-  }
+            for (int e = 0; e < 4; ++e) y[i][e] += t[u][i][e];
+    }
 #pragma unroll
   for (int i = 0; i < NV; ++i)
 #pragma unroll
@@ -131,6 +134,7 @@ __global__ void __launch_bounds__(256) residual_post_norm_kernel(PostNormParams 
   for (int i = 0; i < NV; ++i) {
     const int col = (i * blockDim.x + threadIdx.x) * 4;
     if (col < p.width) {
+      if (!SPLIT) load4(p.w, KD_F32, col, w[i]);
 #pragma unroll
       for (int e = 0; e < 4; ++e) {
         x[i][e] = fmaf(y[i][e] * inv, w[i][e], x[i][e]);
@@ -244,7 +248,8 @@ KD_API int kd_residual_post_norm(const kd_tensor* x, const kd_tensor* y, const k
   if (W % 4 == 0 && (all & 15) == 0 && W <= 8192) {
     threads = W >= 1024 ? 256 : W >= 512 ? 128 : 64;
     const int64_t chunks = (W / 4 + threads - 1) / threads;
-    kernel = chunks <= 1 ? residual_post_norm_kernel<1> : chunks <= 2 ? residual_post_norm_kernel<2> : chunks <= 4 ? residual_post_norm_kernel<4> : residual_post_norm_kernel<8>;
+    if (p.splits > 1) kernel = chunks <= 1 ? residual_post_norm_kernel<1, true> : chunks <= 2 ? residual_post_norm_kernel<2, true> : chunks <= 4 ? residual_post_norm_kernel<4, true> : residual_post_norm_kernel<8, true>;
+    else kernel = chunks <= 1 ? residual_post_norm_kernel<1, false> : chunks <= 2 ? residual_post_norm_kernel<2, false> : chunks <= 4 ? residual_post_norm_kernel<4, false> : residual_post_norm_kernel<8, false>;
   }
   KD_CUDA_CHECK(launch_ex(kernel, dim3((unsigned)rows), dim3(threads), 0, p));
   return after_launch("residual_post_norm_kernel");
