@@ -240,7 +240,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
   if (t == 0) {
     *abort_flag = 0;
     for (int i = 0; i < DS_BARS; ++i) {
-      mbar_init(&full[i], 1);
+      mbar_init(&full[i], DS_COPY_WARPS);
       mbar_init(&empty[i], DS_WARPS);
     }
     fence_mbar_init();
@@ -258,41 +258,48 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
   if (warp >= DS_WARPS) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(DS_REGS_COPY));
     // ------------------------------------------------------------ the copying warps: they go through the same stages, and each
-    // copies every fourth row (key) of a unit
+    // copies every fourth row (key) of a unit.  Each announces its own bytes (there may be none) on every stage's `full`: a stage
+    // is not there before all four have come to it, so none falls behind by more than a ring of stages, and the parity of
+    // `empty` is enough for it (a warp that had no part in a stage could miss two phases of a barrier and wait for a third).
     const int copier = warp - DS_WARPS;
     stage_units += copier * DS_BARS;
     int stage = 0, tail = 0, free = p.units, unit = 0;       // stages begun, stages given back, units free, next unit
     bool ok = true;
-    auto claim = [&](int n, uint32_t bytes) {                // room for a stage, when its readers have left it
+    auto claim = [&](int n) {                                // room for a stage, when its readers have left it
       const int begin = ds_stage_at(unit, n, p.units), need = n + (begin < unit ? p.units - unit : 0);
-      while (ok && free < need) {
-        ok = mbar_wait(&empty[tail % DS_BARS], (uint32_t)(tail / DS_BARS) & 1u, abort_flag, p.err, 544);
+      while (free < need) {
+        // (readers that have given up release stages that are not there yet: such a release is none)
+        ok = mbar_wait(&empty[tail % DS_BARS], (uint32_t)(tail / DS_BARS) & 1u, abort_flag, p.err, 544) && !*abort_flag;
         ok = __all_sync(0xffffffffu, ok);
+        if (!ok) return -1;
         free += stage_units[tail % DS_BARS];
         ++tail;
       }
-      if (!ok) return -1;
-      if (lane == 0) {
-        stage_units[stage % DS_BARS] = (uint8_t)need;
-        if (copier == 0) mbar_arrive_expect_tx(&full[stage % DS_BARS], bytes);      // (before or after the others' copies land)
-      }
+      if (lane == 0) stage_units[stage % DS_BARS] = (uint8_t)need;
       __syncwarp();
       free -= need;
       unit = begin + n;
       ++stage;
       return begin;
     };
+    // this warp's part of the claimed stage: `bytes` in each of its lanes that copy
+    auto announce = [&](bool copies, uint32_t bytes) {
+      const uint32_t lanes = __popc(__ballot_sync(0xffffffffu, copies));
+      if (lane == 0) mbar_arrive_expect_tx(&full[(stage - 1) % DS_BARS], lanes * bytes);      // (before or after the copies land)
+    };
     for (int l = 0, phase = DS_QKV; ok && phase != DS_DONE; ds_next(l, phase, p.L)) {
       const DsLayer& w = tab.layer[l];
       if (phase == DS_ATT) {
         if (!attends) continue;
         for (int key = keys.k0; ok && key < keys.k1; key += DS_KEYS) {
-          const int n = min(DS_KEYS, keys.k1 - key), begin = claim(2, (uint32_t)n * 512u);
+          const int n = min(DS_KEYS, keys.k1 - key), begin = claim(2);
           if (begin < 0) break;
           // one copy of keys and one of values where the rows lie side by side (8000 keys, 6 sequences: a copy per row kept the
           // step at 3.2 ms)
           const bool whole = p.kc_s == 128 && (!p.table || key % 128 + n <= 128);
-          if (whole ? lane == 0 && copier < 2 : lane < n && lane % DS_COPY_WARPS == copier) {
+          const bool copies = whole ? lane == 0 && copier < 2 : lane < n && lane % DS_COPY_WARPS == copier;
+          announce(copies, whole ? n * 256u : 512u);
+          if (copies) {
             const int64_t row = ds_cache_row(p, att_b, att_g, key + lane);
             uint64_t* bar = &full[(stage - 1) % DS_BARS];
             uint8_t* to = smem + begin * DS_UNIT + lane * 256;
@@ -314,19 +321,35 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
           // a block: 8 rows, or four channels' gate rows and their up rows (16 gate rows, then their 16 up rows)
           const int i = r0 + rb * per + (phase == DS_GU ? rr & 3 : rr), c = n0 + i;
           const int row = phase == DS_GU ? c + (c & ~15) + ((rr & 4) << 2) : c;
-          const int rows = phase == DS_GU ? 2 * min(nn - r0, nrb * per) : min(nn - r0, nrb * per);
-          const int begin = claim(n, (uint32_t)(rows * (n / nrb)) * (DS_SEG * 2));
+          const int begin = claim(n);
           if (begin < 0) break;
+          announce(u < n && i < nn, DS_SEG * 2);
           if (u < n && i < nn)
             bulk_load(smem + (begin + u) * DS_UNIT + rr * DS_UNIT_ROW, W + (int64_t)row * K + (s0 + sg) * DS_SEG, DS_SEG * 2, &full[(stage - 1) % DS_BARS]);
         }
       }
     }
-    // no copy is on its way when the CTA ends, whoever has given up
-    for (int i = tail; i < stage; ++i) {
-      volatile int never = 0;
-      mbar_wait(&full[i % DS_BARS], (uint32_t)(i / DS_BARS) & 1u, &never, p.err, 544);
+    // No copy is on its way when the CTA ends, whoever has given up.  The copying warps agree on the last stage that one of them
+    // has begun, announce nothing for those that they have not come to, and wait for all that none has seen released (fewer
+    // than there are barriers), within one limit.
+    __syncwarp();
+    volatile int* mine = reinterpret_cast<volatile int*>(stage_units);       // (its entries are not needed any more)
+    if (lane == 0) {
+      mine[0] = stage;
+      mine[1] = tail;
     }
+    asm volatile("bar.sync 2, 128;" ::: "memory");
+    int last = stage, first = tail;
+    for (int i = 0; i < DS_COPY_WARPS; ++i) {
+      const volatile int* of = mine + (i - copier) * (DS_BARS / 4);
+      last = max(last, of[0]);
+      first = max(first, of[1]);
+    }
+    if (lane == 0)
+      for (int i = stage; i < last; ++i) mbar_arrive(&full[i % DS_BARS]);
+    volatile int never = 0;
+    for (int i = first; i < last; ++i)
+      if (!mbar_wait(&full[i % DS_BARS], (uint32_t)(i / DS_BARS) & 1u, &never, p.err, 544)) break;
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(DS_REGS_WORK));
     int stage = 0, unit = 0;

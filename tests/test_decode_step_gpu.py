@@ -14,17 +14,21 @@ pytestmark = pytest.mark.gpu
 
 # sequences, hidden, inter, heads, kv_heads, prompt: rows that leave one to six blocks of eight to a CTA, one and several
 # segments of columns, one to six sequences, 1, 2 and 4 query heads to a KV head, contexts of one key, at the last unsplit one
-# and beyond it, with unequal splits, and of more keys than the ring holds
+# and beyond it, with unequal splits, and (24 and 32 KV heads leave a CTA all keys of a head) of more keys than the ring holds and
+# of more stages than there are barriers; an lm_head of more rows than a CTA takes at once
 CASES = [(1, 512, 512, 4, 2, 1), (1, 1536, 1024, 4, 4, 64), (2, 512, 1536, 8, 2, 97), (3, 1024, 3072, 16, 8, 130), (4, 512, 1024, 4, 2, 96),
-         (1, 1024, 3072, 16, 8, 900), (2, 512, 4096, 8, 2, 33), (6, 1024, 3072, 16, 8, 300), (1, 2560, 9728, 32, 8, 200), (5, 2560, 1024, 32, 8, 70)]
+         (1, 1024, 3072, 16, 8, 900), (2, 512, 4096, 8, 2, 33), (6, 1024, 3072, 16, 8, 300), (1, 2560, 9728, 32, 8, 200), (5, 2560, 1024, 32, 8, 70),
+         (6, 512, 512, 24, 24, 1300), (4, 512, 1024, 64, 32, 1157)]
+VOCABS = {(2, 512, 512, 4, 2, 40): 20011}
 STEPS = 3
 
 
 def _engine(c, paged=False):
     B, hidden, inter, heads, kv, prompt = c
-    dims = dict(vocab=1000, hidden=hidden, inter=inter, layers=2, heads=heads, kv_heads=kv, head_dim=128)
+    vocab = VOCABS.get(c, 1000)
+    dims = dict(vocab=vocab, hidden=hidden, inter=inter, layers=2, heads=heads, kv_heads=kv, head_dim=128)
     w = {k: lib.round_to_bf16(v) for k, v in synth.qwen3_weights(std=0.03, norm_jitter=0.05, **dims).items()}
-    cfg = Qwen3Config(vocabSize=1000, hiddenSize=hidden, intermediateSize=inter, numHiddenLayers=2, numAttentionHeads=heads, numKeyValueHeads=kv,
+    cfg = Qwen3Config(vocabSize=vocab, hiddenSize=hidden, intermediateSize=inter, numHiddenLayers=2, numAttentionHeads=heads, numKeyValueHeads=kv,
                       headDim=128, dtype="bfloat16")
     return Qwen3Engine(cfg, w, B, -(-(prompt + STEPS) // 128) * 128, paged=paged), w
 
@@ -41,7 +45,7 @@ def _forced(eng, ids, prompt, use_graph):
     return np.stack(out, 1)
 
 
-@pytest.mark.parametrize("c", CASES)
+@pytest.mark.parametrize("c", CASES + list(VOCABS))
 def test_step_kernel_follows_the_oracle(backend, oracle, c):
     B, hidden, inter, heads, kv, prompt = c
     eng, w = _engine(c)
@@ -58,18 +62,20 @@ def test_step_kernel_follows_the_oracle(backend, oracle, c):
         b = t.dataAsync()[:, :, prompt:prompt + STEPS]
         assert np.linalg.norm(a - b) <= 1e-2 * np.linalg.norm(b)
     eng.dispose()
-    ocfg = oracle.Qwen3Config(vocab_size=1000, hidden_size=hidden, intermediate_size=inter, num_hidden_layers=2, num_attention_heads=heads,
+    ocfg = oracle.Qwen3Config(vocab_size=VOCABS.get(c, 1000), hidden_size=hidden, intermediate_size=inter, num_hidden_layers=2, num_attention_heads=heads,
                               num_key_value_heads=kv, head_dim=128)
     ref = oracle.Qwen3Oracle(ocfg, w).logits(ids)[:, prompt:]
     err, before = np.linalg.norm(got - ref), np.linalg.norm(other - ref)
     assert err <= 1e-2 * np.linalg.norm(ref) and err <= 1.2 * before       # bf16 activations: 2^-8 each
 
 
-def test_step_kernel_on_a_paged_cache(backend):
-    c = (3, 512, 512, 4, 2, 150)
-    ids = synth.token_ids("step.ids", (3, 150 + STEPS), 1000)
+# (splits that begin inside a page and cross its end, over two and over twelve pages; whole caches of eleven pages)
+@pytest.mark.parametrize("c", [(3, 512, 512, 4, 2, 150), (2, 512, 512, 8, 4, 1500), (6, 512, 512, 24, 24, 1300)])
+def test_step_kernel_on_a_paged_cache(backend, c):
+    B, prompt = c[0], c[-1]
+    ids = synth.token_ids("step.ids", (B, prompt + STEPS), 1000)
     flat, paged = _engine(c)[0], _engine(c, paged=True)[0]
-    a, b = _forced(flat, ids, 150, True), _forced(paged, ids, 150, True)
+    a, b = _forced(flat, ids, prompt, True), _forced(paged, ids, prompt, True)
     assert flat._decode["step"] is not None and paged._decode["step"] is not None and np.array_equal(a, b)
     flat.dispose()
     paged.dispose()
