@@ -514,6 +514,10 @@ int kd_whisper_encoder_layers(const kd_tensor* const* layer_tensors, int n_layer
  * launch to launch; the order of the sums over keys follows the number of sequences and the position. */
 int kd_decode_step_state_bytes(int sequences, int hidden, int inter, int q_heads, int kv_heads, int head_dim, int vocab, int layers,
                                int grid, uint64_t* bytes_out);
+/* The longest context (keys in the cache before a step) up to which kd_decode_step is faster than the kernels per layer for the
+ * same shapes: 0 where it never is or does not take them, INT_MAX where it always is. */
+int kd_decode_step_max_context(int sequences, int hidden, int inter, int q_heads, int kv_heads, int head_dim, int vocab, int layers,
+                               int grid, int* keys_out);
 int kd_decode_step(const kd_tensor* const* layer_tensors, int n_layers, const kd_tensor* embed, const kd_tensor* final_norm,
                    const kd_tensor* ids, const kd_tensor* inv_freq, const kd_tensor* pos, const kd_tensor* ctx_len, float eps,
                    float scale, const kd_tensor* block_table, const kd_tensor* state, const kd_tensor* logits, const kd_tensor* next_ids);

@@ -32,6 +32,7 @@
 // All CTAs wait for one another, so the launch is cooperative, and every wait is bounded (codes 541-545): a CTA that
 // gives up goes on to the end without waiting, so that the step's ticket and tag stay in order.
 #include <algorithm>
+#include <climits>
 #include <cstddef>
 #include <type_traits>
 
@@ -820,6 +821,28 @@ static bool ds_plan(const DsShape& s, int G, DsPlan* out) {
   return true;
 }
 
+// The longest context at which the step kernel is faster than the kernels per layer.  Those read the cache at HBM's rate; here a CTA
+// walks its share of a head's keys at 15, 17.6 and 33 to 59 ns a key for 1, 2 and 4 query heads (with 4, registers run out
+// beyond three sequences), which is slower wherever the heads do not fill the SMs.  Against that stands what a layer saves
+// in launches and hand-overs: 31 us for one sequence, less for more, and for three less by what they cost beside large weights
+// (the ring shrinks by their activations).  Measured, us a layer here / kernels per layer: 1024 wide, 16 query heads on 8: 1 sequence
+// at 40000 keys 56 / 78, 2 at 16000 49 / 65, 3 at 16000 67 / 72, 4 at 8000 57 / 61, 16000 92 / 81, 6 at 2000 42 / 49, 8000 79 / 70; 32
+// on 8: 1 at 16000 51 / 64, 40000 96 / 81, 2 at 4000 40 / 53, 16000 92 / 67, 5 at 300 43 / 45, 1000 55 / 47; 512 wide, 8 on 2: 4 at 8000 41 / 49, 16000 62 / 55; 2560 wide: 3 at 1000
+// 74 / 82, 4000 92 / 88; 4096 wide: 2 at 4000 104 / 117, 3 at 300 115 / 109.
+static int ds_max_context(const DsShape& s, int G) {
+  DsPlan plan;
+  if (!ds_plan(s, G, &plan)) return 0;
+  const int group = s.Hq / s.Hkv;
+  const double weights = 2e-6 * s.H * (2.0 * s.Hq * 128 + 2.0 * s.Hkv * 128 + 3.0 * s.I);      // MB of a layer
+  const double saved[2][DS_MAX_M] = {{31, 23, 23 - 0.06 * weights, 18, 15, 7},
+                                      {31, 23, 23 - 0.06 * weights, 24 - 32.0 / plan.splits, 15 - 22.0 / plan.splits, 3.7}};      // us
+  const double walk[DS_MAX_M] = {33.5, 38.5, 40, 47.5, 59, 56};      // ns a key
+  const double gain = 1e3 * saved[group == 4][s.M - 1];
+  const double loss = (group == 1 ? 15.0 : group == 2 ? 17.6 : walk[s.M - 1]) / plan.splits - s.M * s.Hkv * 512 / 6900.0;
+  if (gain <= 0) return 0;
+  return loss * 1e9 <= gain ? INT_MAX : (int)std::min<double>(gain / loss, INT_MAX);
+}
+
 typedef void (*DsKernel)(const DsParams);
 template <int GROUP>
 static DsKernel ds_kernel(int M) {
@@ -849,6 +872,17 @@ KD_API int kd_decode_step_state_bytes(int sequences, int hidden, int inter, int 
   }
   DsPlan plan;
   *bytes_out = ds_plan(DsShape{sequences, hidden, inter, q_heads, kv_heads, head_dim, vocab, layers}, grid, &plan) ? plan.state_bytes : 0;
+  return KD_OK;
+}
+
+KD_API int kd_decode_step_max_context(int sequences, int hidden, int inter, int q_heads, int kv_heads, int head_dim, int vocab, int layers,
+                                      int grid, int* keys_out) {
+  KD_REQUIRE(keys_out, "null argument");
+  if (grid <= 0) {
+    KD_TRY(require_init());
+    grid = ctx().sm_count;
+  }
+  *keys_out = ds_max_context(DsShape{sequences, hidden, inter, q_heads, kv_heads, head_dim, vocab, layers}, grid);
   return KD_OK;
 }
 

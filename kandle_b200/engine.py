@@ -3,13 +3,13 @@ tcgen05 flash attention, split-KV decode attention and a CUDA-graph decode step.
 
 It computes what `Qwen3ForCausalLM.forwardWithKVCache` + greedy argmax compute on the eager path
 (packages/model-utils/src/qwen3/for_causal_lm.ts:170-194,475-508), with the ~41 backend calls per
-layer collapsed into 7 (prefill) / 3 (decode, larger batches) kernels and no intermediate copies:
+layer collapsed into 7 (prefill) / 3 (decode, larger batches or long contexts) kernels and no intermediate copies:
 
   prefill, per layer     rms_norm -> QKV GEMM (epilogue: q/k-norm+RoPE+cache write) -> flash attention ->
                          o_proj GEMM (+residual) -> rms_norm -> gate/up GEMM (SiLU*up epilogue) ->
                          down GEMM (+residual)
   decode step of up to   one persistent kernel for the whole step: embedding, every layer, final norm, lm_head and
-  six sequences          the greedy next tokens (kd_decode_step; use_step_kernel has the limits)
+  six sequences          the greedy next tokens (kd_decode_step, up to the context of kd_decode_step_max_context)
   otherwise, per layer   norm+RoPE+cache write (sums the QKV split-K partials) -> split-KV attention ->
                          one persistent kernel: o_proj -> residual+rms_norm -> gate/up with SiLU*up
                          -> down -> residual+rms_norm -> the NEXT layer's QKV partials
@@ -78,6 +78,10 @@ class DecoderEngine:
         self.use_pdl = True
         self.sampler = None   # None: greedy argmax; else dict(temperature, top_k, top_p, rng), see set_sampler
 
+    def _form(self, d: dict) -> str:
+        """Which form a step at self.pos takes, for engines that have more than one; each is captured when it is first needed."""
+        return "step"
+
     def _warm_decode_step(self, d: dict) -> None:
         """The eager step before a capture (see start_decode)."""
         self._enqueue_decode_step(d)
@@ -108,19 +112,29 @@ class DecoderEngine:
 
     def start_decode(self, first_tokens: Tensor, use_graph: bool = True) -> dict:
         """Prepares the decode state after a prefill: next input ids = first_tokens (device int64 [B]),
-        write position = prompt length.  With use_graph the step is captured once (after one eager
-        warm-up step on a scratch position) and replayed by decode_step()."""
+        write position = prompt length.  With use_graph the step is captured once (see _captured) and
+        replayed by decode_step()."""
         B = first_tokens.shape[0]
         d = self._decode_state(B)
         if self.pos + 1 > self.max_seq_len:
             raise ValueError("Cache overflow: no room left for decode steps")
-        be = core._backend()
-        if use_graph and d["graph"] is None:
-            # warm-up at the current position: sizes the library's scratch and the allocator's caches
-            # (nothing may allocate while capturing); the cache row it writes is overwritten by the
-            # first real step, which runs at the same position.
-            core.copy_(d["ids"], first_tokens)
-            be.upload(d["scalars"]._handle, np.array([self.pos, self.pos + 1], np.int32))
+        core.copy_(d["ids"], first_tokens)
+        self._place(d)
+        if use_graph:
+            self._captured(d)
+        d["use_graph"] = use_graph
+        return d
+
+    def _place(self, d: dict) -> None:
+        core._backend().upload(d["scalars"]._handle, np.array([self.pos, self.pos + 1], np.int32))
+
+    def _captured(self, d: dict) -> int:
+        """The graph of a step of the form that self.pos takes.  Before it is captured one eager step at this position sizes the
+        library's scratch and the allocator's caches (nothing may allocate while capturing); the cache row that it writes is
+        overwritten by the real step, and the step's ids and position are put back."""
+        form = self._form(d)
+        if form not in d["graph"]:
+            ids = d["ids"].clone()
             self._warm_decode_step(d)
             lib.call("kd_graph_begin")
             try:
@@ -128,11 +142,11 @@ class DecoderEngine:
             finally:
                 g = ctypes.c_uint64(0)
                 lib.call("kd_graph_end", ctypes.byref(g))
-            d["graph"] = g.value
-        core.copy_(d["ids"], first_tokens)
-        be.upload(d["scalars"]._handle, np.array([self.pos, self.pos + 1], np.int32))
-        d["use_graph"] = use_graph
-        return d
+            d["graph"][form] = g.value
+            core.copy_(d["ids"], ids)
+            ids.dispose()
+            self._place(d)
+        return d["graph"][form]
 
     def decode_step(self) -> Tensor:
         """Runs one step; returns the device int64 [B] tensor holding the tokens just produced."""
@@ -142,7 +156,7 @@ class DecoderEngine:
         if self.sampler is not None:
             self._fresh_uniforms(d["uniforms"])     # read by the (replayed) sampling kernel of this step
         if d["use_graph"]:
-            lib.call("kd_graph_launch", ctypes.c_uint64(d["graph"]))
+            lib.call("kd_graph_launch", ctypes.c_uint64(self._captured(d)))
         else:
             self._enqueue_decode_step(d)
         self.pos += 1
@@ -162,8 +176,8 @@ class DecoderEngine:
         return out
 
     def dispose(self) -> None:
-        if self._decode is not None and self._decode.get("graph"):
-            lib.call("kd_graph_destroy", ctypes.c_uint64(self._decode["graph"]))
+        for g in self._decode["graph"].values() if self._decode is not None else ():
+            lib.call("kd_graph_destroy", ctypes.c_uint64(g))
         self._decode = None
 
 
@@ -458,7 +472,7 @@ class Qwen3Engine(DecoderEngine):
             return s.value
         p2p = self.tp > 1 and self.use_p2p and parallel.peer_buffers_ready()
         d = {
-            "B": B, "graph": None, "chain": self.use_chain,
+            "B": B, "graph": {}, "chain": self.use_chain,
             # (tensor parallel: fp32 partial sums of all sequences must fit one 2 MiB exchange slot)
             "fused": self.use_fused_layer and (self.tp == 1 or (p2p and B * self.H * 4 <= (2 << 20))),
             "p2p": p2p,
@@ -475,7 +489,7 @@ class Qwen3Engine(DecoderEngine):
         if self.use_chain and not self.use_fused_layer:
             d["qkv_p"].dispose()
             d["qkv_p"] = f(chain_splits(self.nqkv, self.H), B, self.nqkv)
-        d["step"] = self._step_kernel_state(B)
+        d["step"], d["step_keys"] = self._step_kernel_state(B)
         d["pos"] = d["scalars"].slice([slice(0, 1)])
         d["ctx"] = d["scalars"].slice([slice(1, 2)])
         self._decode = d
@@ -491,15 +505,20 @@ class Qwen3Engine(DecoderEngine):
         return self._refs[0]
 
     def _step_kernel_state(self, B: int):
-        """The hand-over words that kd_decode_step needs beside a step's buffers, or None where it does not take the shape.  Its attention reads the cache at two thirds of the rate of kd_attention_decode: with six
-        sequences it is ahead up to 5000 keys (step of the 0.6B model: 0.76 ms against 1.10 at 300 keys, 1.1 against 1.3 at
-        2200, 2.2 against 2.0 at 8000), with one at any length (0.71 against 1.53 at 8000)."""
-        n = ctypes.c_uint64(0)
-        if self.tp == 1 and self.use_fused_layer and self.use_step_kernel and B * self.max_seq_len <= 32768:
-            lib.call("kd_decode_step_state_bytes", B, self.H, self.I, self.Hq, self.Hkv, self.D, self.V, self.L, 0, ctypes.byref(n))
-        if not n.value:
-            return None
-        return core.zeros((n.value // 4,), "int32")
+        """The hand-over words that kd_decode_step needs beside a step's buffers and the longest context at which it is the faster
+        form (kd_decode_step_max_context), or None and 0 where it does not take the shape."""
+        n, keys = ctypes.c_uint64(0), ctypes.c_int(0)
+        if self.tp == 1 and self.use_fused_layer and self.use_step_kernel:
+            shape = (B, self.H, self.I, self.Hq, self.Hkv, self.D, self.V, self.L, 0)
+            lib.call("kd_decode_step_state_bytes", *shape, ctypes.byref(n))
+            lib.call("kd_decode_step_max_context", *shape, ctypes.byref(keys))
+        if not keys.value:
+            return None, 0
+        return core.zeros((n.value // 4,), "int32"), keys.value
+
+    def _form(self, d: dict) -> str:
+        # by the position and not by the room in the cache: most engines are built for far longer contexts than a request has
+        return "step" if d["step"] is not None and self.pos <= d["step_keys"] else "layers"
 
     def _enqueue_decode_step(self, d: dict) -> None:
         """One decode step for d['ids'] at device position d['pos']; leaves the next ids in d['ids']."""
@@ -515,7 +534,7 @@ class Qwen3Engine(DecoderEngine):
     def _decode_step_kernels(self, d: dict) -> None:
         c, B = self.cfg, d["B"]
         eps = ctypes.c_float(c.rmsNormEps)
-        if d["step"] is not None:
+        if self._form(d) == "step":
             lib.call("kd_decode_step", self._layer_refs(), self.L, _r(self.embed), _r(self.final_norm), _r(d["ids"]), _r(self.inv_freq), _r(d["pos"]),
                      _r(d["ctx"]), eps, ctypes.c_float(self.scale), _r(self.block_table), _r(d["step"]), _r(d["logits"]),
                      _r(d["ids"]) if self.sampler is None else None)

@@ -661,7 +661,7 @@ class HybridEngine(DecoderEngine):
         if self._decode is not None and self._decode["B"] == B:
             return self._decode
         self.dispose()
-        d = {"B": B, "graph": None, "scalars": core.zeros((2,), "int32"), "ids": core.zeros((B,), "int64"), "ws": _Buffers(),
+        d = {"B": B, "graph": {}, "scalars": core.zeros((2,), "int32"), "ids": core.zeros((B,), "int64"), "ws": _Buffers(),
              "logits": core.empty((B, self.V), "float32"), "uniforms": core.zeros((B,), "float32"), "at": -1}
         d["pos"] = d["scalars"].slice([slice(0, 1)])
         self._decode = d
@@ -697,7 +697,7 @@ class HybridEngine(DecoderEngine):
         """One decode step on given tokens [B, 1]; returns the step's logits [B, V] (a copy)."""
         toks = Tensor(ids.reshape(-1).astype(np.int64))
         d = self._decode
-        if d is None or d["B"] != ids.shape[0] or d["graph"] is None or d["at"] != self.pos:
+        if d is None or d["B"] != ids.shape[0] or not d["graph"] or d["at"] != self.pos:
             d = self.start_decode(toks)
         else:
             core.copy_(d["ids"], toks)

@@ -163,6 +163,7 @@ _SIGNATURES = {
     "kd_qwen3_prompt_layers": [_REFS, ctypes.c_int] + [_T] * 8 + [ctypes.c_float] * 2,
     "kd_whisper_encoder_layers": [_REFS, ctypes.c_int, ctypes.c_int, ctypes.POINTER(ctypes.c_float), ctypes.c_float, _T, _T],
     "kd_decode_step_state_bytes": [ctypes.c_int] * 9 + [ctypes.POINTER(_u64)],
+    "kd_decode_step_max_context": [ctypes.c_int] * 9 + [ctypes.POINTER(ctypes.c_int)],
     "kd_debug_decode_layer_plan": [ctypes.c_int] * 9 + [ctypes.POINTER(ctypes.c_int), ctypes.c_int],
     "kd_debug_decode_layer_trace": [ctypes.POINTER(ctypes.c_uint64), ctypes.c_int],
     "kd_decode_layer_chain_splits": [ctypes.c_int64, ctypes.c_int64, ctypes.POINTER(ctypes.c_int)],

@@ -110,6 +110,37 @@ def test_step_kernel_reports_bad_tokens_and_positions(backend):
     eng.dispose()
 
 
+def test_the_form_follows_the_position(backend):
+    """An engine with room for far more positions than its requests have takes the step kernel, and goes over to the kernels per
+    layer (and back, on the next prompt) at the context that the library names, replayed or not."""
+    c = (2, 512, 512, 4, 2, 40)
+    eng, _ = _engine(c)
+    ids = synth.token_ids("step.ids", (2, 40 + STEPS), 20011)
+    alone = _forced(eng, ids, 40, True)
+    room = Qwen3Engine(eng.cfg, _engine(c)[1], 2, 40960)
+    assert np.array_equal(_forced(room, ids, 40, True), alone)
+    d = room._decode
+    assert d["step_keys"] > 10000 and list(d["graph"]) == ["step"]
+    d["step_keys"] = 41                                                    # (the last of the three steps is beyond it)
+    for use_graph in (False, True, True):
+        got = _forced(room, ids, 40, use_graph)
+        assert np.array_equal(got[:, :2], alone[:, :2])
+        assert 0 < np.linalg.norm(got[:, 2] - alone[:, 2]) <= 1e-2 * np.linalg.norm(alone[:, 2])
+    assert list(d["graph"]) == ["step", "layers"]
+    room.dispose()                                                         # the change, and its capture, in the middle of a run
+    room.prefill(np.ascontiguousarray(ids[:, :40]))
+    d = room.start_decode(Tensor(ids[:, 40].astype(np.int64)))
+    d["step_keys"] = 41
+    for t in range(STEPS):
+        if t:
+            backend.upload(d["ids"]._handle, ids[:, 40 + t].astype(np.int64))
+        assert np.array_equal(d["ids"].dataAsync(), ids[:, 40 + t])
+        room.decode_step()
+        assert np.array_equal(d["logits"].dataAsync()[0], got[:, t])
+    room.dispose()
+    eng.dispose()
+
+
 def test_shapes_that_keep_the_kernels_per_layer(backend):
     def taken(*shape):
         n = ctypes.c_uint64(0)
