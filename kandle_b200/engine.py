@@ -250,7 +250,6 @@ class Qwen3Engine(DecoderEngine):
             self.v_cache = [core.zeros((self.B, self.Hkv, max_seq_len, self.D), "bfloat16") for _ in range(self.L)]
         self.scale = 1.0 / math.sqrt(self.D)
         self._prefill_bufs = {}
-        self._refs = None
         self.use_early_kv = os.environ.get("KD_EARLY_KV", "1") != "0"
         # decode: run o_proj .. next layer's QKV as one persistent kernel per layer (kd_decode_layer_chain);
         # tensor parallelism needs an all-reduce after o_proj and down_proj, so it keeps separate kernels
@@ -389,9 +388,11 @@ class Qwen3Engine(DecoderEngine):
         h, h1 = w["h"], w["h1"]
         table = self.block_table.slice([slice(0, B), slice(None)]) if self.paged else None
         native = self.tp == 1 and self.D == 128 and not self.paged
-        if native:
-            lib.call("kd_qwen3_prompt_layers", self._layer_refs(), self.L, _r(w["x"]), _r(h), _r(h1), _r(w["q"]), _r(w["attn"]), _r(w["act"]),
-                     _r(w["cos"]), _r(w["sin"]), ctypes.c_float(c.rmsNormEps), ctypes.c_float(self.scale))
+        # layers 0, 1 to 3, and the rest: descriptors are gathered (2.5 us a layer) while the GPU is at the layers before
+        for a, b in ((0, 1), (1, 4), (4, self.L)) if native else ():
+            if a < min(b, self.L):
+                lib.call("kd_qwen3_prompt_layers", self._layer_refs(a, b), min(b, self.L) - a, _r(w["x"]), _r(h), _r(h1), _r(w["q"]), _r(w["attn"]), _r(w["act"]),
+                         _r(w["cos"]), _r(w["sin"]), ctypes.c_float(c.rmsNormEps), ctypes.c_float(self.scale))
         for li, lw in enumerate(self.layers if not native else ()):
             if self.paged:
                 # the prompt's K/V go to a contiguous buffer that the attention reads, then into the pages
@@ -495,14 +496,12 @@ class Qwen3Engine(DecoderEngine):
         self._decode = d
         return d
 
-    def _layer_refs(self):
-        """The layers' tensors as kd_decode_step and kd_qwen3_prompt_layers take them.  Laid out once: it takes 75 us, and the GPU
-        waits for it at the start of a prompt.  (The library looks the storages up at each call.)"""
-        if self._refs is None:
-            names = ("in_norm", "wqkv", "q_norm", "k_norm", "wo", "post_norm", "wgu", "wdown")
-            kept = [t._handle.c() for i, lw in enumerate(self.layers) for t in [lw[k] for k in names] + [self.k_cache[i], self.v_cache[i]]]
-            self._refs = (ctypes.c_void_p * len(kept))(*map(ctypes.addressof, kept)), kept
-        return self._refs[0]
+    def _layer_refs(self, first: int, end: int):
+        """The tensors of layers first..end-1 as kd_decode_step and kd_qwen3_prompt_layers take them.  Laid out for every call (2.5 us a
+        layer): a program may have put another weight or cache into the engine since the last one."""
+        names = ("in_norm", "wqkv", "q_norm", "k_norm", "wo", "post_norm", "wgu", "wdown")
+        return lib.refs([t for lw, k, v in zip(self.layers[first:end], self.k_cache[first:end], self.v_cache[first:end])
+                         for t in (*(lw[n] for n in names), k, v)])
 
     def _step_kernel_state(self, B: int):
         """The hand-over words that kd_decode_step needs beside a step's buffers and the longest context at which it is the faster
@@ -535,7 +534,7 @@ class Qwen3Engine(DecoderEngine):
         c, B = self.cfg, d["B"]
         eps = ctypes.c_float(c.rmsNormEps)
         if self._form(d) == "step":
-            lib.call("kd_decode_step", self._layer_refs(), self.L, _r(self.embed), _r(self.final_norm), _r(d["ids"]), _r(self.inv_freq), _r(d["pos"]),
+            lib.call("kd_decode_step", self._layer_refs(0, self.L), self.L, _r(self.embed), _r(self.final_norm), _r(d["ids"]), _r(self.inv_freq), _r(d["pos"]),
                      _r(d["ctx"]), eps, ctypes.c_float(self.scale), _r(self.block_table), _r(d["step"]), _r(d["logits"]),
                      _r(d["ids"]) if self.sampler is None else None)
             if self.sampler is not None:

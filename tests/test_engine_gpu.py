@@ -203,3 +203,29 @@ def test_early_kv_prefetch_gives_the_same_tokens(backend, oracle):
         eng.dispose()
         assert np.array_equal(want, plain)
         assert np.array_equal(got, want) and np.array_equal(got_eager, want)
+
+
+def test_an_engine_uses_the_weights_and_caches_that_it_has_now(backend):
+    """A program may put other tensors into an engine between two prompts."""
+    dims = dict(vocab=512, hidden=512, inter=512, layers=3, heads=4, kv_heads=2, head_dim=128)
+    cfg = Qwen3Config(vocabSize=512, hiddenSize=512, intermediateSize=512, numHiddenLayers=3, numAttentionHeads=4, numKeyValueHeads=2, headDim=128,
+                      dtype="bfloat16")
+    one, other = (Qwen3Engine(cfg, synth.qwen3_weights(std=std, **dims), 2, 64) for std in (0.03, 0.06))
+    ids = synth.token_ids("swap.ids", (2, 20), 512)
+    want = [e.prefill(ids, all_logits=True)[1].dataAsync() for e in (one, other)]
+    first = one.generate(ids, 3)
+    assert not np.array_equal(*want)
+    before = one.layers, one.k_cache, one.v_cache, one.embed       # (kept, so that nothing takes their place)
+    one.layers, one.embed, one.final_norm = list(other.layers), other.embed, other.final_norm
+    one.k_cache, one.v_cache = ([core.zeros((2, 2, 64, 128), "bfloat16") for _ in range(3)] for _ in range(2))
+    one.dispose()                                                  # (the captured step holds the old ones)
+    tokens = [one.generate(ids, 3, use_graph=False), other.generate(ids, 3)]
+    assert np.array_equal(*tokens) and not np.array_equal(tokens[0], first)
+    for a, b in zip(one.k_cache + one.v_cache, other.k_cache + other.v_cache):
+        assert np.array_equal(a.dataAsync(), b.dataAsync())
+    assert np.array_equal(one.prefill(ids, all_logits=True)[1].dataAsync(), want[1])
+    one.layers, one.k_cache, one.v_cache, one.embed = before
+    one.layers[1] = dict(one.layers[1], wo=other.layers[1]["wo"])
+    assert not np.array_equal(one.prefill(ids, all_logits=True)[1].dataAsync(), want[0])
+    one.dispose()
+    other.dispose()
