@@ -223,22 +223,37 @@ __global__ void __launch_bounds__(LF_THREADS, 1) linear_few_kernel(const FewPara
 struct FewPlan { int S, R, smem; };
 
 // How the call is split: the fewest CTAs a cluster that fill the SMs and leave a CTA at most 32 KB of x to read (all of x passes through
-// every cluster).  S = 0: not taken.  Taken are the sizes at which this kernel is the faster one in a chain of linears (us, tcgen05 kernels
-// before, with kd_set_pdl(3) now; rows x N x K).  Up to 16 rows: 1 x 2048 x 2048 10.7, 4.4; 1 x 1024 x 1024 7.5, 3.2; 1 x 64 x 2048
-// 8.1, 2.8; 8 x 4096 x 2048 12.7, 8.1; 8 x 8448 x 2048 17.9, 14.2; 8 x 2048 x 6144 14.6, 11.8; 8 x 12288 x 2048 13.8, 21.0 (registers
-// hold too little of a long stream: left to the kernel with a ring).  More: 32 x 2048 x 2048 9.7, 6.7; 32 x 1024 x 1024 7.5, 4.2; 32 x
-// 4096 x 2048 10.6, 10.0; 32 x 8448 x 2048 12.6, 17.4; 32 x 2048 x 6144 14.6, 27.2 (x itself is the traffic).
+// every cluster).  With more than 16 rows an SM holds one CTA (registers), and clusters of four and eight leave SMs over: 33 and 15 of
+// them fit 148 SMs.  A cluster is not doubled there where that many more do not fit, as long as x allows it (32 x 1024 x 3072, rows
+// x N x K: 16 clusters of eight 12.5 us, 32 of four 5.9; 32 x 2560 x 512: 40 of two 4.7, 80 CTAs alone 3.5).
+// S = 0: not taken.  Taken are the sizes at which this kernel is the faster one (us in a chain with kd_set_pdl(3): tcgen05
+// kernels, this one).  Up to 16 rows: 1 x 2048 x 2048 9.0, 4.4; 1 x 64 x 2048 7.5, 2.8; 8 x 4096 x 2048 10.9, 8.3; 8 x 8192 x 2048 15.7, 14.8;
+// 8 x 2048 x 6144 17.9, 12.2; 8 x 5120 x 2560 17.5, 14.1; 1 x 10240 x 1024 10.5, 10.2; not: 16 x 10240 x 768 8.4, 9.1; 8 x 10240 x 1536 13.4, 15.6; 16 x 4096 x 4096 13.0, 15.7; 16 x 2048 x 6144
+// 12.6, 13.5; 1 x 5120 x 2560 16.2, 19.1 (registers hold too little of a long stream).  More: 32 x 2048 x 2048 8.6, 6.7; 32 x 1024 x 3072 9.0,
+// 5.9; 32 x 2048 x 3072 9.5, 8.9; 32 x 6144 x 1024 8.5, 8.5; 20 x 4096 x 2048 10.6, 9.8; not: 32 x 4096 x 2048 9.3, 10.2; 32 x 8192 x 1024 8.6,
+// 9.1; 32 x 2560 x 3072 10.4, 11.1; 24 x 6144 x 768 7.3, 8.0.
 static FewPlan lf_plan(int64_t M, int64_t N, int64_t K, int sms) {
   FewPlan f{0, 0, 0};
   if (M < 1 || M > 32 || N < 32 || N % 8 || K < 256 || K % 32) return f;
-  if (M <= 16 ? N * K > (18ll << 20) : N * K > (8ll << 20) || K > 4096) return f;
-  const int tiles = (int)((N + LF_ROWS - 1) / LF_ROWS);
+  const int64_t weights = N * K, x = M * K * 2, mega = 1ll << 20, kb = 1024;
+  if (M <= 16) {
+    if (weights > (N > 8192 ? (M <= 8 ? 12 : 6) : x > 128 * kb ? 9 : 18) * mega) return f;
+    if (weights > 12 * mega && K > 2048 && ((x < 32 * kb && (N > 4096 || K > 4096)) || x > 96 * kb)) return f;
+  } else {
+    if (K > 4096 || N > 8192 || weights > (x > 128 * kb ? 6 : 8) * mega || M * weights > 192 * mega) return f;
+    if (N > 4096 && K > 512 && K < 1024 && M > 20) return f;
+  }
+  const int tiles = (int)((N + LF_ROWS - 1) / LF_ROWS), mt = M <= 16 ? 1 : 2;
+  const auto fit = [&](int S) { return std::max(1, sms / S - (mt == 1 || S < 4 ? 0 : S == 4 ? 4 : 3)); };      // clusters at a time
+  const auto rounds = [&](int S) { return (tiles + fit(S) - 1) / fit(S); };
   int S = 1;
-  while (S < 8 && K / 32 >= 16 * S && (tiles * S < sms * 2 / 3 || M * K * 2 / S > 32 * 1024)) S *= 2;
-  const int clusters = std::max(1, sms / S);
-  const int R = LF_ROWS * ((tiles + clusters - 1) / clusters), mt = M <= 16 ? 1 : 2;
+  while (S < 8 && K / 32 >= 16 * S && (tiles * S < sms * 2 / 3 || x / S > 32 * kb)) {
+    if (mt == 2 && rounds(2 * S) >= 2 * rounds(S) && x / S <= (S == 2 ? 48 : 64) * kb) break;
+    S *= 2;
+  }
+  const int R = LF_ROWS * rounds(S);
   const int64_t smem = 16 * mt * (((((K / 32 + S - 1) / S) | 1) * 64) + LF_WARPS * (LF_ROWS + 4) * 4 + (R + 4) * 4);
-  if (smem > 200 * 1024) return f;
+  if (smem > 200 * kb) return f;
   return FewPlan{S, R, (int)smem};
 }
 

@@ -373,10 +373,11 @@ KD_API int kd_linear_glu(const kd_tensor* x, const kd_tensor* weight, int epilog
   KD_TRY(tensor_ptr(weight, &pw));
   KD_TRY(tensor_ptr(out, &po));
   if (x->dtype == KD_BF16 && K % 8 == 0 && ((reinterpret_cast<uintptr_t>(px) | reinterpret_cast<uintptr_t>(pw) | reinterpret_cast<uintptr_t>(po)) & 15) == 0) {
-    if (linear_few_rows(M, N, K)) return linear_few(px, K, pw, po, N / 2, 0, nullptr, 0, (int)M, (int)N, (int)K, epilogue);
-    // a handful of rows: the kernel that streams the weights, where its 128-row tiles are enough to fill the GPU
+    // a handful of rows: the kernel that streams the weights, where its 128-row tiles are enough to fill the GPU (8 x 10240 x 512, rows x N x K:
+    // 4.9 us, linear_few 5.7)
     if (M <= 64 && N >= 128ll * (ctx().sm_count / 2))
       return gemm_bf16_skinny(px, K, pw, K, (int)M, (int)N, (int)K, 1, nullptr, po, epilogue == KD_EPI_GEGLU ? 2 : 1);
+    if (linear_few_rows(M, N, K)) return linear_few(px, K, pw, po, N / 2, 0, nullptr, 0, (int)M, (int)N, (int)K, epilogue);
     return gemm_bf16(px, K, pw, K, po, N / 2, 0, nullptr, 0, (int)M, (int)N, (int)K, epilogue);
   }
   return grouped_linear(x->dtype, px, pw, nullptr, M, 1, N, K, epilogue, 0.f, po);
