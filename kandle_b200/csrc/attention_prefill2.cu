@@ -173,13 +173,21 @@ flash_attention_prefill2_kernel(const __grid_constant__ CUtensorMap tmap_q, cons
   pdl_trigger();   // after the TMEM allocation (see common.cuh)
   if (warp >= 8) {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 72;");
-  // Whole warps wait and an elected lane issues, which keeps addresses and descriptors in uniform registers (an MMA issued from
-  // inside `if (lane == 0)` took its warp about 70 cycles, now 13).  One clip of Whisper's encoder: 1014 -> 960 us, with the GEMMs' loops likewise; 32 prompts of 2048: 2 % less.
-  auto wait = [&](uint64_t* bar, uint32_t parity, int code) { return (bool)__all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, p.err, code)); };
+  // Heads of 128: whole warps wait and an elected lane issues, which keeps addresses and descriptors in uniform registers (an MMA
+  // issued from inside `if (lane == 0)` took its warp about 70 cycles, now 13).  With heads of 64 there are half as many MMAs to a
+  // wait, and one lane by itself is through sooner.  us, one lane and whole warps: 16 heads of 128, causal, 4 x 2048 102, 95; 3 x 701
+  // 18.5, 17.1; 12 heads of 64, 2 x 1500 29.0, 32.5; 8 x 1500 104, 112; 64 x 1500 799, 826.
+  constexpr bool WHOLE = D > 64;
+  auto wait = [&](uint64_t* bar, uint32_t parity, int code) {
+    const bool ok = mbar_wait(bar, parity, abort_flag, p.err, code);
+    return WHOLE ? (bool)__all_sync(0xffffffffu, ok) : ok;
+  };
+  auto issues = [] { return WHOLE ? elect_one() : true; };
+  auto together = [] { if (WHOLE) __syncwarp(); };
   if (warp == 8) {
-    {
+    if (WHOLE || lane == 0) {
       // an absent second sub-tile still gets a (zero-filled, out-of-range) load so that the byte count is fixed
-      if (elect_one()) {
+      if (issues()) {
         mbar_arrive_expect_tx(q_full, 2 * Q_BYTES);
 #pragma unroll
         for (int t = 0; t < 2; ++t)
@@ -187,11 +195,11 @@ flash_attention_prefill2_kernel(const __grid_constant__ CUtensorMap tmap_q, cons
           for (int s = 0; s < QK_SLABS; ++s)
             tma_load_4d(q_smem + t * Q_BYTES + s * SLAB_BYTES, &tmap_q, q_full, s * 64, q0[t], head[t], b);
       }
-      __syncwarp();
+      together();
       for (int j = 0; j < n_blocks; ++j) {
         const int sk = j % NK, sv = j % NV;
         if (!wait(&t_empty[sk], (uint32_t)(((j / NK) & 1) ^ 1), 401)) break;
-        if (elect_one()) {
+        if (issues()) {
           mbar_arrive_expect_tx(&t_full[sk], K_BYTES);
 #pragma unroll
           for (int s = 0; s < SLABS; ++s)
@@ -200,19 +208,19 @@ flash_attention_prefill2_kernel(const __grid_constant__ CUtensorMap tmap_q, cons
           for (int s = SLABS; s < QK_SLABS; ++s)
             tma_load_4d(k_ring + sk * K_BYTES + s * SLAB_BYTES, &tmap_kr, &t_full[sk], (s - SLABS) * 64, (j0 + j) * FA2_BKV, 0, b);
         }
-        __syncwarp();
+        together();
         if (!wait(&t_empty[NK + sv], (uint32_t)(((j / NV) & 1) ^ 1), 402)) break;
-        if (elect_one()) {
+        if (issues()) {
           mbar_arrive_expect_tx(&t_full[NK + sv], V_BYTES);
 #pragma unroll
           for (int s = 0; s < SLABS; ++s)
             tma_load_4d(v_ring + sv * V_BYTES + s * SLAB_BYTES, &tmap_v, &t_full[NK + sv], s * 64, (j0 + j) * FA2_BKV, hk, b);
         }
-        __syncwarp();
+        together();
       }
     }
   } else if (warp == 9) {
-    {
+    if (WHOLE || lane == 0) {
       bool ok = wait(q_full, 0, 403);
       // S_t(j) = Q_t K(j)^T.  The K tile is waited for once per block (by whichever sub-tile comes first).
       auto issue_qk = [&](int t, int j, bool wait_k) -> bool {
@@ -222,7 +230,7 @@ flash_attention_prefill2_kernel(const __grid_constant__ CUtensorMap tmap_q, cons
         const uint32_t q_addr = smem_u32(q_smem + t * Q_BYTES);
         const uint32_t k_addr = smem_u32(k_ring + stage * K_BYTES);
         const uint32_t d_tmem = tmem_base + (uint32_t)(t * 128);
-        if (elect_one()) {
+        if (issues()) {
           const uint64_t qdesc = make_smem_desc_sw128(q_addr, 16, 1024), kdesc = make_smem_desc_sw128(k_addr, 16, 1024);
 #pragma unroll
           for (int k = 0; k < (D + DR) / 16; ++k) {
@@ -231,13 +239,13 @@ flash_attention_prefill2_kernel(const __grid_constant__ CUtensorMap tmap_q, cons
           }
           umma_commit(&s_full[t]);
         }
-        __syncwarp();
+        together();
         return true;
       };
       // the K slot of block j is released after the last QK^T that reads it
       auto commit = [&](uint64_t* bar) {
-        if (elect_one()) umma_commit(bar);
-        __syncwarp();
+        if (issues()) umma_commit(bar);
+        together();
       };
       auto release_k = [&](int j) { commit(&t_empty[j % NK]); };
       auto issue_pv = [&](int t, int j, bool wait_v) -> bool {
@@ -248,14 +256,14 @@ flash_attention_prefill2_kernel(const __grid_constant__ CUtensorMap tmap_q, cons
         for (int half = 0; half < 2; ++half) {
           if (!wait(&p_ready[2 * t + half], (uint32_t)(j & 1), 405)) return false;
           tc_fence_after();
-          if (elect_one()) {
+          if (issues()) {
             const uint64_t vdesc = make_smem_desc_sw128(v_addr, SLAB_BYTES, 1024);
 #pragma unroll
             for (int k = 4 * half; k < 4 * half + 4; ++k)
               umma_ts(tmem_base + (uint32_t)(256 + t * D), tmem_base + (uint32_t)(t * 128 + k * 8), vdesc + (uint32_t)(k * 128), IDESC_PV, (j | k) != 0 ? 1u : 0u);
             if (half == 1) umma_commit(&o_done[t]);
           }
-          __syncwarp();
+          together();
         }
         return true;
       };
