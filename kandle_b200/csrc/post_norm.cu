@@ -81,11 +81,12 @@ __device__ __forceinline__ float block_total(float v, float* red) {
   return t;
 }
 
-// NV chunks of four columns a thread.  Bound: the latency of its loads, so all of them are on their way at once (the weights, and up
+// NV chunks of four columns a thread; SPLIT: more than one partial sum and few rows.  Bound: the latency of its loads, so all of them are on their way at once (the weights, and up
 // to AHEAD partial sums beside the first): a decode step of the hybrid in 6 layers, 12 such kernels: 32 sequences of 2048
 // columns 502 -> 491 us, 4 of 1024 243 -> 237, against one partial sum after the other and the weights behind the sum.
-// With one partial sum (prompts: many rows, bound by HBM) the registers for that would only cost warps: a prompt of 8192 tokens
-// of the hybrid in 6 layers took 10.1 ms before there was this form, 10.9 when it served prompts too.
+// With one partial sum (prompts) or more rows than SMs the registers for that only cost warps: a prompt of 8192 tokens of the hybrid in 6
+// layers took 10.1 ms before there was this form, 10.9 when it served prompts too; two partial sums of 2048 columns, one after the other
+// and ahead: 148 rows 2.4 us, 2.5; 200 rows 2.7, 4.1; 1500 rows 6.7, 19.3; eight: 148 rows 4.9, 2.8; 400 rows 5.6, 6.9.
 template <int NV, bool SPLIT>
 __global__ void __launch_bounds__(256) residual_post_norm_kernel(PostNormParams p) {
   __shared__ float red[2][32];
@@ -124,6 +125,18 @@ __global__ void __launch_bounds__(256) residual_post_norm_kernel(PostNormParams 
 #pragma unroll
             for (int e = 0; e < 4; ++e) y[i][e] += t[u][i][e];
     }
+  else
+    for (int s = 1; s < p.splits; ++s)
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const int col = (i * blockDim.x + threadIdx.x) * 4;
+        if (col < p.width) {
+          float t[4];
+          load4(p.y, p.dt_y, ((int64_t)s * p.rows + row) * p.width + col, t);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) y[i][e] += t[e];
+        }
+      }
 #pragma unroll
   for (int i = 0; i < NV; ++i)
 #pragma unroll
@@ -248,7 +261,7 @@ KD_API int kd_residual_post_norm(const kd_tensor* x, const kd_tensor* y, const k
   if (W % 4 == 0 && (all & 15) == 0 && W <= 8192) {
     threads = W >= 1024 ? 256 : W >= 512 ? 128 : 64;
     const int64_t chunks = (W / 4 + threads - 1) / threads;
-    if (p.splits > 1) kernel = chunks <= 1 ? residual_post_norm_kernel<1, true> : chunks <= 2 ? residual_post_norm_kernel<2, true> : chunks <= 4 ? residual_post_norm_kernel<4, true> : residual_post_norm_kernel<8, true>;
+    if (p.splits > 1 && rows <= ctx().sm_count) kernel = chunks <= 1 ? residual_post_norm_kernel<1, true> : chunks <= 2 ? residual_post_norm_kernel<2, true> : chunks <= 4 ? residual_post_norm_kernel<4, true> : residual_post_norm_kernel<8, true>;
     else kernel = chunks <= 1 ? residual_post_norm_kernel<1, false> : chunks <= 2 ? residual_post_norm_kernel<2, false> : chunks <= 4 ? residual_post_norm_kernel<4, false> : residual_post_norm_kernel<8, false>;
   }
   KD_CUDA_CHECK(launch_ex(kernel, dim3((unsigned)rows), dim3(threads), 0, p));

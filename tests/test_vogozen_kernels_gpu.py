@@ -68,6 +68,19 @@ def test_embedding_and_output_norm(backend, width, dtype):
         _close(_get(h), hybrid.rms_norm(want, fw, 1e-3), 2e-6 if dtype == "float32" else 5e-3, "final norm")
 
 
+@pytest.mark.parametrize("rows", [147, 148, 149, 300])
+@pytest.mark.parametrize("width, splits", [(1024, 2), (2048, 9), (3000, 3), (8192, 5)])
+def test_output_norm_of_partial_sums(backend, rows, width, splits):
+    """On both sides of one row per multiprocessor, where the partial sums are fetched ahead and one after the other."""
+    rng = _rng(rows + width)
+    x, y, w = _bf(rng.standard_normal((rows, width))), _bf(rng.standard_normal((splits, rows, width))), _bf(1 + 0.3 * rng.standard_normal(width))
+    tx, ty, tw, h = _put(x), _put(y), _put(w), core.full((rows, width), float("nan"))
+    lib.call("kd_residual_post_norm", _r(tx), _r(ty), _r(tw), F(1e-3), None, _r(tx), _r(h))
+    want = x.astype(np.float64) + hybrid.rms_norm(y.astype(np.float64).sum(0), w.astype(np.float64), 1e-3)
+    _close(_get(tx), want, 2e-6, "residual")
+    _close(_get(h), want, 2e-6, "copy")
+
+
 def test_embedding_reports_a_bad_id(backend):
     x, h = core.empty((1, 8)), core.empty((1, 8))
     lib.call("kd_embed_rows", _r(_put(np.ones((3, 8)))), _r(Tensor(np.array([3], np.int32))), _r(x), _r(h))
