@@ -714,12 +714,12 @@ int attention_prefill2(const CUtensorMap& tq, const CUtensorMap& tk, const CUten
 
 // Whether the kernel that shares K/V tiles between two query sub-tiles of a CTA takes the call: it reads K and V half as often and
 // keeps the tensor pipe busy during a softmax, but leaves SMs idle where one tile a CTA is a single wave (us, two tiles and one: 16 heads of
-// 128, causal, 1 x 300 12.5, 10.5; 1 x 1024 24.1, 16.8; 2 x 700 18.7, 20.8; 3 x 701 20.7, 24.9; 12 heads of 64, 1 x 1500 28.5, 20.6;
-// 2 x 750 17.9, 14.5; 2 x 1500 28.9, 37.1).  Single query tiles gain nothing from the other kernel (1 x 20 8.5, 9.1; 8 x 97 9.2, 9.5).
+// 128, causal, 1 x 97 6.3, 5.0; 9 x 128 7.5, 5.8; 10 x 97 7.3, 10.1; 1 x 300 9.4, 6.6; 1 x 1024 19.5, 13.0; 2 x 700 15.4, 16.6; 3 x 701 15.6,
+// 20.1; 12 heads of 64, 1 x 1500 26.9, 17.5; 2 x 750 15.8, 10.8; 2 x 800 17.9, 21.6; 2 x 1500 27.5, 33.3).
 static bool attention_two_tiles(const AttnParams& a, int sms) {
   const int64_t tiles = (a.Sq + FA_BQ - 1) / FA_BQ;
   if ((a.Hq / a.Hkv) % 2 != 0 && tiles == 1) return false;      // one query tile per KV head
-  return tiles == 1 || tiles * a.Hq * a.B > sms;
+  return tiles * a.Hq * a.B > sms;
 }
 
 int attention_tc_try(const kd_tensor* q, const kd_tensor* k, const kd_tensor* v, const kd_tensor* out,

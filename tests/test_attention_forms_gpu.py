@@ -15,7 +15,8 @@ pytestmark = pytest.mark.gpu
     (6, 12, 12, 200, 200, 64), (7, 12, 12, 257, 257, 64),            # 144, and 252 with three tiles a head: the last one alone
     (37, 2, 1, 129, 129, 64), (38, 2, 1, 129, 129, 64),              # 148 and 152
     (3, 24, 8, 300, 300, 128), (1, 48, 48, 300, 412, 128),           # odd groups: consecutive tiles of a head; more keys than queries
-    (40, 4, 2, 100, 100, 128), (40, 4, 4, 100, 100, 128)])           # one tile a head
+    (40, 4, 2, 100, 100, 128), (40, 4, 4, 100, 100, 128),            # one tile a head
+    (9, 16, 8, 128, 128, 128), (10, 16, 8, 97, 97, 128), (12, 12, 6, 33, 33, 64), (1, 8, 2, 16, 16, 64)])     # ... of pairs of heads, 144, 160, 144 and 8 tiles
 def test_one_and_two_query_tiles(backend, oracle, causal, b, hq, hkv, sq, skv, d):
     if causal and sq != skv:
         pytest.skip("the oracle aligns the mask at the first key")
