@@ -818,12 +818,12 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams&
 }
 
 // Tile width and number of CTAs that share a tile; widths from `narrowest` on.  256 columns where such tiles occupy more than
-// half of the SMs; else the shortest estimate.  An SM takes a k-block in the time of its copies from L2 (about 83 GB/s: 0.28,
-// 0.38, 0.57 us for 64-, 128- and 256-wide tiles); a shared tile costs two barriers of the cluster and the others' sums.
-// One CTA and the chosen number a tile, 97 rows: N = 1024, K = 2048 12.4, 9.5 us; N = 1024, K = 3072 16.9, 10.6; N = 2560,
-// K = 9728 46.2, 22.7; N = K = 768 8.4, 10.4 (not shared).  Measured for 1 to 2103 rows and 15 shapes of weights, none above
-// the time of one CTA a tile by more than its runs differ.  Above two rows of tiles it gave little or nothing (700 rows,
-// N = 1024, K = 2048: 16.5, 18.5).
+// half of the SMs; else the shortest estimate.  In it a k-block costs a CTA 0.28, 0.38 and 0.57 us for 64-, 128- and 256-wide tiles
+// (the loops alone take 0.22 whatever the width), and a shared tile two barriers of the cluster and the others' sums.
+// One CTA and the chosen number a tile, 97 rows: N = 1024, K = 2048 9.2, 8.1 us; N = 1024, K = 3072 12.5, 9.2; N = 2560,
+// K = 9728 34.4, 20.9; N = K = 768 5.1, 6.2 (not shared).  Measured for 40 to 2103 rows and 16 shapes of weights: up to two rows of tiles
+// the choice is the fastest form or within 4 % of it (40 rows, N = 6144, K = 1024: 8 %).  More rows of tiles are not
+// shared: 701 rows and more gain nothing by it; 300 rows with a long K would (N = 2560, K = 9728: 36.4 us, shared 26.4).
 static int linear_tile(int64_t M, int64_t N, int64_t K, int narrowest, int64_t sms, int* splits) {
   const int64_t m_tiles = (M + GEMM_BM - 1) / GEMM_BM, kbs = (K + GEMM_BK - 1) / GEMM_BK;
   *splits = 1;
@@ -844,11 +844,11 @@ static int linear_tile(int64_t M, int64_t N, int64_t K, int narrowest, int64_t s
 }
 
 // Whether 256-wide tiles are worked on by pairs of CTAs.  A launch of pairs costs 1 to 2 us more (two cluster barriers, tensor memory
-// for both); it gains where the SMs multiply long enough: by K (less copied and read per k-block: N = 2560, K = 9728, 2103 rows
-// 128 -> 111 us; N = 1024, K = 3072, 8192 rows 56 -> 49, 4096 rows 29 -> 31) and where the chip runs at its power limit (65536 rows:
-// N = 4096, K = 1024 475 -> 395 to 458 us, N = 6144 630 -> 572; 96000 rows, K = 768: N = 2304 319 -> 300, N = 3072 427 -> 382).
-// Between, at K = 1024, it is even (16384 rows: N = 4096 113 -> 111, N = 6144 153 -> 159); N = 768 loses up to 24576 rows (16384 rows,
-// K = 3072 67 -> 72).
+// for both); it gains where the SMs multiply long enough (less is copied and read per k-block) and where the chip runs at its power
+// limit.  One CTA -> a pair, us: N = 2560, K = 9728, 2103 rows 153 -> 143; N = 1024, K = 3072, 8192 rows 54 -> 53, 4096 rows 23 -> 25;
+// N = 6144, K = 1024, 4096 rows 45 -> 39, 16384 rows 181 -> 147, 65536 rows 727 -> 588; N = 2304, K = 768, 8192 rows 29.7 -> 30.3, 96000 rows
+// 311 -> 291; N = K = 768, 24576 rows 34.6 -> 35.3, 65536 rows 90 -> 85.  The line is on the safe side of where it gains since the loops
+// were shortened: N = 4096, K = 1024, 4096 rows would take 34.6 instead of 37.7, N = 768, K = 3072, 16384 rows 69 instead of 74.
 static bool linear_pair(int64_t M, int64_t N, int64_t K, int64_t sms) {
   const int64_t n_tiles = (N + 255) / 256, kbs = (K + GEMM_BK - 1) / GEMM_BK;
   const int64_t waves = ((M + 127) / 128 * n_tiles + sms - 1) / sms, pair_waves = ((M + 255) / 256 * n_tiles + sms / 2 - 1) / (sms / 2);
@@ -969,7 +969,8 @@ int gemm_bf16_qkv_rope(const void* A, int64_t lda, const void* W, int64_t ldw, i
 // Microseconds, one k-block a step and a loop of one lane before / now (weights from HBM, in a programmatic chain):
 // 4 x 6144 x 4096 (rows x N x K) 22.3, 14.6; 32 x 6144 x 4096 24.5, 16.8; 32 x 12288 x 2048 16.2, 13.8; 32 x 6144 x 1024 10.3, 8.4;
 // 32 x 32768 x 2048 32.8, 26.0; 4 x 32768 x 1024 18.4, 14.1; 32 x 19456 x 2560 36.1, 23.4 (21.9 with one k-block a step);
-// 128 x 12288 x 2048 24.6, 23.1 (one k-block a step); 32 x 151936 x 1024 62.9, 60.9.
+// 128 x 12288 x 2048 24.6, 23.1 (one k-block a step); 32 x 151936 x 1024 62.9, 60.9.  33 to 128 rows with more tiles than SMs: 64 x 19456
+// x 2560 40.0, 26.6; 128 x 24576 x 1024 34.0, 22.5; 128 x 37888 x 2048 39.3, 38.9.
 //
 // When N/128 gives too few CTAs the K range is split across CTAs; every split writes fp32 partial sums [split][m][n],
 // which the consumer kernels
@@ -1137,6 +1138,8 @@ gemm_skinny_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_w, const __g
 // Picks the split-K factor for a skinny GEMM: up to half as many CTAs as SMs, each with at least four k-blocks and an even
 // number of them (a step of the ring takes two).  A decode step of the hybrid in 6 layers, 32 sequences, widths 2048 / 1024:
 // 446 / 284 us with 40 CTAs of at least 8 k-blocks, 436 / 281 with 74 of 4, 440 / 281 with 148 of 4; 2 k-blocks: 458 and 307.
+// With the norm that adds the partial sums up (add_rmsnorm_kernel), 40 CTAs of 8 and the loops of one lane / now: 8 x 2560 x 9728
+// 29.8, 18.1; 128 x 2560 x 9728 38.4, 30.7; 8 x 1024 x 3072 8.6, 7.3; 128 x 1024 x 2048 15.9, 15.3.
 int gemm_skinny_auto_splits(int N, int K) {
   const int tiles = (N + 127) / 128, total_kb = (K + GEMM_BK - 1) / GEMM_BK;
   const int splits = std::max(1, std::min(ctx().sm_count / 2 / tiles, total_kb / 4));

@@ -47,9 +47,11 @@ def _close(got, want, rel):
 
 
 # microseconds of one CTA and of a pair a tile, from measuring both
-@pytest.mark.parametrize("M, N, K, one, two", [(700, 4096, 1024, 12.8, 14.9), (4096, 1024, 2048, 22.9, 24.9), (8192, 4096, 1024, 55.2, 51.5), (65536, 6144, 1024, 630, 572),
-                                               (2103, 2560, 9728, 128, 111), (2103, 10240, 2560, 89, 81), (16384, 768, 3072, 67, 72), (96000, 768, 3072, 369, 362),
-                                               (12000, 768, 768, 18.2, 21.7), (96000, 2304, 768, 323, 300), (32768, 1024, 3072, 193, 167)])
+@pytest.mark.parametrize("M, N, K, one, two", [(700, 4096, 1024, 10.3, 11.5), (4096, 1024, 2048, 17.3, 19.4), (4096, 1024, 3072, 23.2, 25.0), (8192, 4096, 1024, 68.2, 61.5),
+                                               (16384, 6144, 1024, 181, 147), (65536, 6144, 1024, 727, 588), (2103, 2560, 9728, 153, 143), (2103, 6144, 2560, 51.9, 47.9),
+                                               (6000, 2048, 2048, 46.9, 44.1), (2103, 8448, 2048, 66.2, 68.6), (8192, 1024, 2048, 39.1, 39.8), (8192, 1024, 3072, 54.2, 53.3),
+                                               (8192, 2304, 768, 29.7, 30.3), (12288, 768, 768, 18.0, 19.5), (96000, 768, 3072, 355, 317), (96000, 2304, 768, 311, 291),
+                                               (32768, 1024, 3072, 170, 155), (65536, 768, 768, 90.1, 84.5)])
 def test_pairs_where_they_are_the_faster_form(M, N, K, one, two):
     assert _pair(M, N, K) == (two < one)
 
