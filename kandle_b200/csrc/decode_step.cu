@@ -147,6 +147,12 @@ __device__ __forceinline__ u64 ds_key(float v, int column) {
   const uint32_t b = __float_as_uint(v + 0.0f);          // (-0 is 0)
   return (u64)(b & 0x80000000u ? ~b : b | 0x80000000u) << 32 | (0xffffffffu - (uint32_t)column);
 }
+// 1 / sqrt(s), with a Newton step: as exact as the division; 0 for squares beyond the range of fp32, as the division gives (the
+// larger of no number and 0 is 0).
+__device__ __forceinline__ float ds_inv_sqrt(float s) {
+  const float y = rsqrtf(s);
+  return y * (1.5f - fmaxf(0.5f * s * y * y, 0.f));
+}
 template <int LANES>
 __device__ __forceinline__ float ds_sum(float v) {        // over groups of lanes
 #pragma unroll
@@ -487,8 +493,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
     // Sum of a row over the warps, in half a warp (lane % 16 = warp whose share it reads).
     auto total = [&](int m, int row) { return ds_sum<16>(red[(flip * DS_WARPS + (lane & 15)) * red_warp + m * DS_ROWS + row]); };
     auto inv_rms = [&](int at_flip, int m) {
-      const float s = ds_sum<16>(ssq[(at_flip * M + m) * DS_WARPS + (lane & 15)]) * inv_h + p.eps, y = rsqrtf(s);
-      return y * (1.5f - 0.5f * s * y * y);                  // (a Newton step: as exact as the division)
+      return ds_inv_sqrt(ds_sum<16>(ssq[(at_flip * M + m) * DS_WARPS + (lane & 15)]) * inv_h + p.eps);
     };
 
     for (int l = 0, phase = DS_QKV; phase != DS_DONE; ds_next(l, phase, p.L)) {
@@ -506,8 +511,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
           ds_take(v, [&](int i) { return src + 2 * i; }, [](int) { return true; }, tag, abort_flag, p.err, 543);
           float y[4] = {ds_f(v[0].x), ds_f(v[0].y), ds_f(v[1].x), ds_f(v[1].y)};
           if (warp <= GROUP) {
-            const float ss = warp_sum(y[0] * y[0] + y[1] * y[1] + y[2] * y[2] + y[3] * y[3]) * (1.f / 128.f) + p.eps, r = rsqrtf(ss);
-            const float sc = r * (1.5f - 0.5f * ss * r * r);
+            const float sc = ds_inv_sqrt(warp_sum(y[0] * y[0] + y[1] * y[1] + y[2] * y[2] + y[3] * y[3]) * (1.f / 128.f) + p.eps);
             y[0] = (y[0] * sc) * ds_lo(nw.x);
             y[1] = (y[1] * sc) * ds_hi(nw.x);
             y[2] = (y[2] * sc) * ds_lo(nw.y);

@@ -94,6 +94,25 @@ def test_the_lowest_of_equal_logits_is_the_next_token(backend):
     eng.dispose()
 
 
+def test_squares_beyond_fp32_count_as_the_kernels_per_layer_have_them(backend):
+    """A row whose sum of squares overflows is scaled by 1 / infinity, in either form."""
+    eng, w = _engine((2, 512, 512, 4, 2, 9))
+    rows = w["model.embed_tokens.weight"].copy()
+    rows[7] = np.where(rows[7] < 0, -1e25, 1e25)
+    eng.embed = Tensor(rows, dtype="bfloat16")
+    got = []
+    for eng.use_step_kernel in (True, False):
+        eng.prefill(synth.token_ids("step.ids", (2, 9), 6))
+        eng.start_decode(Tensor(np.array([7, 3], np.int64)), False)
+        assert (eng._decode["step"] is not None) == eng.use_step_kernel
+        eng.decode_step()
+        got.append(eng._decode["logits"].dataAsync()[0])
+        eng.dispose()
+    one, other = (g[:, np.arange(1000) != 7] for g in got)                 # (the products of row 7 with itself overflow as well)
+    assert not one[0].any() and not other[0].any()
+    assert np.linalg.norm(one[1] - other[1]) <= 1e-2 * np.linalg.norm(other[1])
+
+
 def test_step_kernel_reports_bad_tokens_and_positions(backend):
     eng, _ = _engine((1, 512, 512, 4, 2, 5))
     eng.prefill(synth.token_ids("step.ids", (1, 5), 1000))
