@@ -510,7 +510,8 @@ int kd_whisper_encoder_layers(const kd_tensor* const* layer_tensors, int n_layer
  * kd_decode_step_state_bytes gives 0 for shapes that this form does not take: it takes 1 to 6 sequences whose activations
  * fit shared memory beside the weights on their way, head_dim 128, 1, 2 or 4 query heads to a KV head, up to 64 layers, and
  * widths that are multiples of 512 with at least one row per CTA (`grid` CTAs; 0: this device's).  A token outside the table is taken as zeros (code 101), a
- * cache row outside [0, maxS) is not written (code 102), a wait that runs out reports 541-545.  Results are bit-identical from
+ * cache row outside [0, maxS) is not written (code 102), a page outside the pools is read as the last one and not written (code 103), a
+ * wait that runs out reports 541-545.  Results are bit-identical from
  * launch to launch; the order of the sums over keys follows the number of sequences and the position. */
 int kd_decode_step_state_bytes(int sequences, int hidden, int inter, int q_heads, int kv_heads, int head_dim, int vocab, int layers,
                                int grid, uint64_t* bytes_out);

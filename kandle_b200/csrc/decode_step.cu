@@ -82,6 +82,7 @@ struct DsParams {
   int64_t kc_b, kc_h, kc_s;
   float eps, scale_log2;
   int M, H, I, Hq, Hkv, L, V, max_s, max_pages, splits, units;
+  unsigned last_page;         // of the pools
   int x_stride, h_rows;       // bytes of a sequence's activations; rows of the residual that a CTA may own
 };
 
@@ -147,11 +148,10 @@ __device__ __forceinline__ u64 ds_key(float v, int column) {
   const uint32_t b = __float_as_uint(v + 0.0f);          // (-0 is 0)
   return (u64)(b & 0x80000000u ? ~b : b | 0x80000000u) << 32 | (0xffffffffu - (uint32_t)column);
 }
-// 1 / sqrt(s), with a Newton step: as exact as the division; 0 for squares beyond the range of fp32, as the division gives (the
-// larger of no number and 0 is 0).
+// 1 / sqrt(s), with a Newton step: as exact as the division; 0 for squares beyond the range of fp32, as the division gives.
 __device__ __forceinline__ float ds_inv_sqrt(float s) {
   const float y = rsqrtf(s);
-  return y * (1.5f - fmaxf(0.5f * s * y * y, 0.f));
+  return y == 0.f ? 0.f : y * (1.5f - 0.5f * s * y * y);
 }
 template <int LANES>
 __device__ __forceinline__ float ds_sum(float v) {        // over groups of lanes
@@ -193,8 +193,9 @@ __device__ __forceinline__ void ds_next(int& l, int& phase, int L) {
     ++phase;
   }
 }
+// A page outside the pool (reported at the start of the step) is taken for the last one.
 __device__ __forceinline__ int64_t ds_cache_row(const DsParams& p, int b, int g, int key) {
-  if (p.table) return (int64_t)p.table[(int64_t)b * p.max_pages + key / 128] * p.kc_b + g * p.kc_h + (key % 128) * p.kc_s;
+  if (p.table) return (int64_t)min((unsigned)p.table[(int64_t)b * p.max_pages + key / 128], p.last_page) * p.kc_b + g * p.kc_h + (key % 128) * p.kc_s;
   return b * p.kc_b + g * p.kc_h + key * p.kc_s;
 }
 
@@ -253,6 +254,11 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
     fence_mbar_init();
     if (!pos_ok && cta == 0 && atomicCAS(p.err, 0, 102) == 0) { p.err[1] = pos_given; p.err[2] = p.max_s; }
   }
+  if (p.table && cta < M)                                    // the step's pages of a sequence
+    for (int i = t; i <= pos / 128; i += DS_THREADS) {
+      const int page = p.table[(int64_t)cta * p.max_pages + i];
+      if ((unsigned)page > p.last_page && atomicCAS(p.err, 0, 103) == 0) { p.err[1] = cta; p.err[2] = page; }
+    }
   __syncthreads();
 
   // attention: (sequence, KV head), share of its keys
@@ -526,7 +532,7 @@ __global__ void __launch_bounds__(DS_THREADS, 1) decode_step_kernel(const __grid
             }
           }
           const uint32_t lo = ds_pack(y[0], y[1]), hi = ds_pack(y[2], y[3]);
-          if (warp >= GROUP && pos_ok)
+          if (warp >= GROUP && pos_ok && (!p.table || (unsigned)p.table[(int64_t)b * p.max_pages + pos / 128] <= p.last_page))
             *reinterpret_cast<uint2*>((warp == GROUP ? w.kc : w.vc) + ds_cache_row(p, b, g, pos) + 4 * lane) = make_uint2(lo, hi);
           *reinterpret_cast<float4*>(q_s + warp * 128 + 4 * lane) = make_float4(ds_lo(lo), ds_hi(lo), ds_lo(hi), ds_hi(hi));
         }
@@ -901,7 +907,7 @@ KD_API int kd_decode_step(const kd_tensor* const* layer_tensors, int n_layers, c
              "decode step: embedding and matrices must be 2-D, ids 1-D");
   Context& c = ctx();
   const kd_tensor* kc0 = layer_tensors[8];
-  KD_REQUIRE(kc0->ndim == 4, "decode step: caches must be 4-D");
+  KD_REQUIRE(kc0->ndim == 4 && kc0->shape[0] >= 1, "decode step: caches must be 4-D, with rows");
   DsShape s;
   s.M = (int)ids->shape[0];
   s.V = (int)embed->shape[0];
@@ -970,6 +976,7 @@ KD_API int kd_decode_step(const kd_tensor* const* layer_tensors, int n_layers, c
   p.logits = static_cast<float*>(pl);
   p.table = static_cast<const int*>(pt);
   p.max_pages = block_table ? (int)block_table->shape[1] : 0;
+  p.last_page = (unsigned)(kc0->shape[0] - 1);
   p.max_s = block_table ? p.max_pages * 128 : (int)kc0->shape[2];
   p.err = c.error_flag;
   p.state = static_cast<unsigned*>(ps);

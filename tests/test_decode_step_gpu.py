@@ -160,6 +160,28 @@ def test_the_form_follows_the_position(backend):
     eng.dispose()
 
 
+def test_pages_outside_the_pool_are_reported(backend):
+    eng, _ = _engine((2, 512, 512, 4, 2, 150), paged=True)
+    ids = synth.token_ids("step.ids", (2, 150), 1000)
+    table = eng.block_table.dataAsync().astype(np.int32)
+    eng.prefill(ids)
+    first = Tensor(np.array([1, 2], np.int64))
+    for b, place, page in ((0, 1, int(table.max()) + 1), (1, 0, -1), (1, 1, 1 << 30)):
+        bad = table.copy()
+        bad[b, place] = page
+        eng.start_decode(first, False)
+        backend.upload(eng.block_table._handle, bad)
+        eng.decode_step()
+        with pytest.raises(lib.KandleCudaError, match="code 103"):
+            backend.synchronize()
+        eng.pos = 150
+    backend.upload(eng.block_table._handle, table)
+    eng.start_decode(first, False)                                         # and goes on
+    eng.decode_step()
+    backend.synchronize()
+    eng.dispose()
+
+
 def test_shapes_that_keep_the_kernels_per_layer(backend):
     def taken(*shape):
         n = ctypes.c_uint64(0)
