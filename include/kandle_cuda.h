@@ -484,7 +484,7 @@ int kd_decode_layer_fused(const kd_tensor* attn, const kd_tensor* w_o, const kd_
                           const kd_tensor* sin, const kd_tensor* pos, const kd_tensor* k_cache_next,
                           const kd_tensor* v_cache_next, const kd_tensor* block_table, const kd_tensor* q_out,
                           const kd_tensor* resid_out, const kd_tensor* x_final);
-/* All layers of a prompt (packages/model-utils/src/qwen3/decoder_layer.ts:191-241), enqueued by one call: per layer kd_add_rmsnorm,
+/* Consecutive layers of a prompt (packages/model-utils/src/qwen3/decoder_layer.ts:191-241), enqueued by one call: per layer kd_add_rmsnorm,
  * kd_qkv_linear_norm_rope_cachewrite, kd_flash_attention, kd_linear_bf16 (+ residual), kd_add_rmsnorm, kd_linear_bf16 (SwiGLU) and
  * kd_linear_bf16 (+ residual).  layer_tensors as in kd_decode_step (contiguous caches [>=B,Hkv,>=S,128]); x [B*S,H] bf16, h (the
  * residual stream, in and out) and h1 [B*S,H] fp32, q and attn [B,S,Hq,128], act [B*S,I], cos and sin [S,64]. */

@@ -366,7 +366,8 @@ class Qwen3Engine(DecoderEngine):
             core._backend().upload(w["ids"]._handle, ids.reshape(-1))
             ids_t = w["ids"]
         # every kernel starts while the one before it drains, and the linears fetch their first weights meanwhile
-        # (0.6B: 97 tokens 2.07 -> 1.79 ms, 2103 3.87 -> 3.38, 8192 11.4 -> 10.9, 16384 and 32768 the same, 65536 81.0 -> 83.1)
+        # (ms without and with: 0.6B, 97 tokens 1.96, 1.63; 3 x 701 3.62, 3.18; 4 x 2048 9.9, 9.5; 8 x 2048 even; beyond, nothing is gained.
+        # 2560 wide, 9 layers: 1024 2.62, 2.49; 3 x 701 4.52, 4.46)
         lib.call("kd_set_pdl", 3 if self.use_pdl and self.tp == 1 and B * S <= 16384 else 0)
         try:
             full = self._prefill_kernels(w, ids_t, B, S, all_logits)
