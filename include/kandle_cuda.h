@@ -121,7 +121,7 @@ int kd_debug_fill_scratch(int byte_value);
  * multiprocessors.  Touch no device.
  *   linear       width of the output tiles of kd_linear_bf16 and its relatives (heads_of_128: of
  *                kd_qkv_linear_norm_rope_cachewrite) and the CTAs that share a tile's K
- *   pair         whether pairs of CTAs work on its 256-wide tiles
+ *   pair         whether pairs of CTAs work on its 256-wide tiles (with K <= 1024: of linears whose epilogue is light, see heavy_epilogue)
  *   linear_few   CTAs of a cluster and its weight rows where linears of up to 32 rows take the kernel for a few rows, else 0
  *   matmul_f32   as linear, for kd_matmul with K-major fp32 operands
  *   recurrence   whether kd_delta_rule (delta = 1) or kd_wkv takes a call of `tokens` tokens and `heads` heads (of all

@@ -205,7 +205,7 @@ __device__ __forceinline__ float4 ld_peer_f4(uint32_t addr, uint32_t rank) {
 // PAIR: a cluster of two CTAs works on tiles of 256 rows with MMAs across both SMs (cta_group::2).  Each brings in its 128 rows of
 // A and half of the W tile, so a k-block costs an SM 32 KB of copies and of operand reads instead of 48, and six stages
 // fit instead of four.
-template <int BLOCK_N, int STAGES, bool SHARED, bool PAIR = false>
+template <int BLOCK_N, int STAGES, bool SHARED, bool PAIR = false, bool LONE = false>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b, GemmParams p) {
   constexpr int A_BYTES = GEMM_BM * GEMM_BK * 2;
@@ -317,8 +317,14 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
   // Warps 0 and 1 walk through the k-blocks as whole warps and an elected lane issues copies and MMAs, so that addresses and
   // descriptors stay in uniform registers: with a loop inside `if (lane == 0)` a k-block took its warp 0.29 us whatever the
   // width of the tile, now 0.22.  Prompts of 97 and 3 x 701 tokens: 1774 and 3384 us before, 1650 and 3232 now; 32 x 2048: 0.8 % less.
-  if (warp == 0) {
-    early = __shfl_sync(0xffffffffu, early, 0);
+  // LONE: loops of one lane, where the epilogue is what takes the time (heavy_epilogue).
+  auto all = [](bool ok) { return LONE ? ok : (bool)__all_sync(0xffffffffu, ok); };
+  auto issues = [] { return LONE ? true : elect_one(); };
+  auto together = [] { if (!LONE) __syncwarp(); };
+  if (LONE && warp < 2 && lane != 0) {
+    // (the other lanes have nothing to do)
+  } else if (warp == 0) {
+    if (!LONE) early = __shfl_sync(0xffffffffu, early, 0);
     int stage = 0;
     uint32_t phase = 0;
     bool ok = true;
@@ -330,14 +336,14 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
         uint8_t* sa = smem + stage * STAGE_BYTES;
         const bool w_here = early > 0;                   // (the first stages: W is on its way)
         if (w_here) --early;
-        else ok = __all_sync(0xffffffffu, mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.err, 201));
+        else ok = all(mbar_wait(&empty[stage], phase ^ 1, abort_flag, p.err, 201));
         if (!ok) break;
-        if (elect_one()) {
+        if (issues()) {
           if (!w_here) expect(stage);
           load(sa, &tmap_a, stage, kb * GEMM_BK, row0);
           if (!w_here) load(sa + A_BYTES, &tmap_b, stage, kb * GEMM_BK, w_row + n_tile * BLOCK_N + (int)pair_rank * (BLOCK_N / 2));
         }
-        __syncwarp();
+        together();
         if (++stage == STAGES) { stage = 0; phase ^= 1; }
       }
     }
@@ -350,15 +356,15 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
       uint32_t acc_phase = 0;
       bool ok = true;
       for (int tile = first; ok && tile < total_tiles; tile += step) {
-        ok = __all_sync(0xffffffffu, mbar_wait(&tmem_empty[acc], acc_phase ^ 1, abort_flag, p.err, 202));
+        ok = all(mbar_wait(&tmem_empty[acc], acc_phase ^ 1, abort_flag, p.err, 202));
         if (!ok) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + (uint32_t)(acc * BLOCK_N);
         for (int kb = kb_begin; kb < kb_end; ++kb) {
-          ok = __all_sync(0xffffffffu, mbar_wait(&full[stage], phase, abort_flag, p.err, 203));
+          ok = all(mbar_wait(&full[stage], phase, abort_flag, p.err, 203));
           if (!ok) break;
           tc_fence_after();
-          if (elect_one()) {
+          if (issues()) {
             const uint64_t adesc = adesc0 + (uint32_t)(stage * (STAGE_BYTES >> 4)), bdesc = bdesc0 + (uint32_t)(stage * (STAGE_BYTES >> 4));
 #pragma unroll
             for (int k = 0; k < GEMM_BK / 16; ++k) {
@@ -368,15 +374,15 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
             if constexpr (PAIR) umma_commit_pair(&empty[stage]);
             else umma_commit(&empty[stage]);
           }
-          __syncwarp();
+          together();
           if (++stage == STAGES) { stage = 0; phase ^= 1; }
         }
         if (!ok) break;
-        if (elect_one()) {
+        if (issues()) {
           if constexpr (PAIR) umma_commit_pair(&tmem_full[acc]);
           else umma_commit(&tmem_full[acc]);
         }
-        __syncwarp();
+        together();
         acc ^= 1;
         if (acc == 0) acc_phase ^= 1;
       }
@@ -745,6 +751,10 @@ gemm_bf16_tcgen05_kernel(const __grid_constant__ CUtensorMap tmap_a, const __gri
   }
 }
 
+// Whether the epilogue takes longer than the k-blocks of a 256-wide tile: an activation or a residual than 16 of them, a bias alone
+// than 15.
+static bool heavy_epilogue(const GemmParams& p) { return p.K <= (p.epi == KD_EPI_RESIDUAL || p.act ? 16 : p.bias ? 15 : 0) * GEMM_BK; }
+
 // Tiles of 256 x 256 by pairs of CTAs.
 static int launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams& p) {
   constexpr int BLOCK_N = 256, STAGES = 6, SMEM = STAGES * (GEMM_BM + BLOCK_N / 2) * GEMM_BK * 2 + 1024 + 256;
@@ -786,6 +796,8 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams&
     KD_CUDA_CHECK(cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<BLOCK_N, STAGES, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
     if (BLOCK_N < 256)
       KD_CUDA_CHECK(cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<BLOCK_N, STAGES, BLOCK_N < 256>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
+    if constexpr (BLOCK_N == 256)
+      KD_CUDA_CHECK(cudaFuncSetAttribute(gemm_bf16_tcgen05_kernel<BLOCK_N, STAGES, false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM));
     configured[ctx().device & 63] = true;
   }
   // (grouped: every group may end in a partial tile, and groups without rows have none)
@@ -813,6 +825,13 @@ static int launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, GemmParams&
   }
   p.splits = 1;
   const int grid = total < ctx().sm_count ? (int)total : ctx().sm_count;
+  if constexpr (BLOCK_N == 256)
+    // There the warps that wait as a whole take issue slots from the epilogue: 96000 rows, N = K = 768, bias and residual 171 us with
+    // one lane, 178 with whole warps, bias and GELU 146, 147; without an epilogue 97.5, 96.8 (N = 3072: 372, 363).
+    if (heavy_epilogue(p)) {
+      KD_CUDA_CHECK(launch_ex(gemm_bf16_tcgen05_kernel<BLOCK_N, STAGES, false, false, true>, dim3(grid), dim3(GEMM_THREADS), (size_t)SMEM, ta, tb, p));
+      return after_launch("gemm_bf16_tcgen05_kernel");
+    }
   KD_CUDA_CHECK(launch_ex(gemm_bf16_tcgen05_kernel<BLOCK_N, STAGES, false>, dim3(grid), dim3(GEMM_THREADS), (size_t)SMEM, ta, tb, p));
   return after_launch("gemm_bf16_tcgen05_kernel");
 }
@@ -845,14 +864,17 @@ static int linear_tile(int64_t M, int64_t N, int64_t K, int narrowest, int64_t s
 
 // Whether 256-wide tiles are worked on by pairs of CTAs.  A launch of pairs costs 1 to 2 us more (two cluster barriers, tensor memory
 // for both); it gains where the SMs multiply long enough (less is copied and read per k-block) and where the chip runs at its power
-// limit.  One CTA -> a pair, us: N = 2560, K = 9728, 2103 rows 153 -> 143; N = 1024, K = 3072, 8192 rows 54 -> 53, 4096 rows 23 -> 25;
-// N = 6144, K = 1024, 4096 rows 45 -> 39, 16384 rows 181 -> 147, 65536 rows 727 -> 588; N = 2304, K = 768, 8192 rows 29.7 -> 30.3, 96000 rows
-// 311 -> 291; N = K = 768, 24576 rows 34.6 -> 35.3, 65536 rows 90 -> 85.  The line is on the safe side of where it gains since the loops
-// were shortened: N = 4096, K = 1024, 4096 rows would take 34.6 instead of 37.7, N = 768, K = 3072, 16384 rows 69 instead of 74.
+// limit.  One CTA -> a pair, us, with the epilogue that the size has in a model: gate/up, N = 6144, K = 1024, 700 rows 10.8 -> 12.0, 4096
+// 40 -> 36, 16384 145 -> 128, 65536 698 -> 604; o_proj, N = 1024, K = 2048, 4096 rows 40.8 -> 41.5, 36000 177 -> 168; down, N = 1024,
+// K = 3072, 4096 rows 43.6 -> 45.3, 8192 91 -> 85; N = 2560, K = 9728, 2103 rows 153 -> 135; bias and residual, N = 768, K = 3072, 96000
+// rows 355 -> 319.  Below 12 k-blocks a pair loses at any number of rows (65536 rows, N = K = 512: 34.9 -> 37.8), and so it does with
+// a heavy epilogue (96000 rows, K = 768: bias, N = 2304 426 -> 439, bias and GELU, N = 3072 531 -> 546; K = 240, 195 -> 205; 36000 rows,
+// N = 2048, K = 1024: bias 128 -> 123, bias and residual 175 -> 184).
+// The line is on the safe side of where pairs gain (4096 rows, N = 4096, K = 1024, no epilogue: 29.5 -> 26.7).
 static bool linear_pair(int64_t M, int64_t N, int64_t K, int64_t sms) {
   const int64_t n_tiles = (N + 255) / 256, kbs = (K + GEMM_BK - 1) / GEMM_BK;
   const int64_t waves = ((M + 127) / 128 * n_tiles + sms - 1) / sms, pair_waves = ((M + 255) / 256 * n_tiles + sms / 2 - 1) / (sms / 2);
-  return pair_waves <= waves && (M >= 24576 || (N >= 1024 && waves * kbs >= (K >= 1024 ? 96 : 132)));
+  return kbs >= 12 && pair_waves <= waves && (M >= 24576 || (N >= 1024 && waves * kbs >= (K >= 1024 ? 96 : 132)));
 }
 
 // out[M, N or N/2] = epilogue(A[M,K] * W[N,K]^T).  Pointers are device pointers; ld* in elements.
@@ -894,7 +916,7 @@ int gemm_bf16_bias_act(const void* A, int64_t lda, const void* W, int64_t ldw, v
   CUtensorMap ta, tb;
   KD_TRY(make_tmap_bf16_2d(&ta, A, (uint64_t)M, (uint64_t)K, (uint64_t)lda, GEMM_BM, GEMM_BK));
   const int bn = linear_tile(M, N, K, 64, ctx().sm_count, &p.splits);
-  const bool pair = bn == 256 && linear_pair(M, N, K, ctx().sm_count);
+  const bool pair = bn == 256 && !heavy_epilogue(p) && linear_pair(M, N, K, ctx().sm_count);
   KD_TRY(make_tmap_bf16_2d(&tb, W, (uint64_t)N, (uint64_t)K, (uint64_t)ldw, pair ? 128 : bn, GEMM_BK));
   if (pair) return launch_gemm_pair(ta, tb, p);
   if (bn == 256) return launch_gemm<256, 4>(ta, tb, p);

@@ -46,18 +46,18 @@ def _close(got, want, rel):
     assert (np.abs(got - want) <= rel * np.abs(want) + 1e-5 * np.abs(want).max()).all()
 
 
-# microseconds of one CTA and of a pair a tile, from measuring both
-@pytest.mark.parametrize("M, N, K, one, two", [(700, 4096, 1024, 10.3, 11.5), (4096, 1024, 2048, 17.3, 19.4), (4096, 1024, 3072, 23.2, 25.0), (8192, 4096, 1024, 68.2, 61.5),
-                                               (16384, 6144, 1024, 181, 147), (65536, 6144, 1024, 727, 588), (2103, 2560, 9728, 153, 143), (2103, 6144, 2560, 51.9, 47.9),
-                                               (6000, 2048, 2048, 46.9, 44.1), (2103, 8448, 2048, 66.2, 68.6), (8192, 1024, 2048, 39.1, 39.8), (8192, 1024, 3072, 54.2, 53.3),
-                                               (8192, 2304, 768, 29.7, 30.3), (12288, 768, 768, 18.0, 19.5), (96000, 768, 3072, 355, 317), (96000, 2304, 768, 311, 291),
-                                               (32768, 1024, 3072, 170, 155), (65536, 768, 768, 90.1, 84.5)])
+# microseconds of one CTA and of a pair a tile, from measuring both with the epilogue that the size has in a model
+@pytest.mark.parametrize("M, N, K, one, two", [(700, 6144, 1024, 10.8, 12.0), (700, 19456, 2560, 77.7, 64.1), (4096, 6144, 1024, 40.4, 36.2), (16384, 6144, 1024, 145, 128),
+                                               (65536, 6144, 1024, 698, 604), (4096, 1024, 2048, 40.8, 41.5), (36000, 1024, 2048, 177, 168), (4096, 1024, 3072, 43.6, 45.3),
+                                               (8192, 1024, 3072, 90.6, 85.3), (2103, 2560, 4096, 74.1, 67.8), (2103, 2560, 9728, 153, 135), (2103, 6144, 2560, 57.6, 52.9),
+                                               (6000, 2048, 2048, 68.3, 67.1), (8192, 2304, 768, 37.7, 38.4), (36000, 768, 768, 38.3, 36.9), (96000, 768, 3072, 355, 319),
+                                               (65536, 512, 512, 34.9, 37.8), (96000, 768, 240, 195, 205), (65536, 4096, 1024, 467, 385), (2103, 4096, 1024, 16.6, 17.0)])
 def test_pairs_where_they_are_the_faster_form(M, N, K, one, two):
     assert _pair(M, N, K) == (two < one)
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("M, N, K", [(24577, 264, 72), (24800, 512, 200), (37900, 776, 64), (1409, 2312, 6152)])
+@pytest.mark.parametrize("M, N, K", [(24577, 264, 1096), (24800, 512, 1160), (29000, 776, 1032), (1409, 2312, 6152)])
 def test_epilogues_of_pairs(backend, M, N, K):
     assert _pair(M, N, K)
     x, w = _bf((M, K), 1), _bf((N, K), 2, K ** -0.5)
@@ -84,9 +84,27 @@ def test_epilogues_of_pairs(backend, M, N, K):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("M, N, K", [(24577, 264, 1032), (5000, 1032, 1024), (5000, 1032, 200), (700, 6152, 72)])
+def test_epilogues_that_take_longer_than_the_products(backend, M, N, K):
+    """Bias, activation and residual with few k-blocks: 256-wide tiles whose loops are one lane's (K <= 1024), and the sizes beside them."""
+    x, w, r, b = _bf((M, K), 1), _bf((N, K), 2, K ** -0.5), _bf((M, N), 3), _bf((N,), 4, 0.5)
+    tx, tw, tb, tr = _put(x), _put(w), _put(b), _put(r)
+    y = x.astype(np.float64) @ w.T.astype(np.float64)
+    for bias, act, res in ((tb, 0, None), (tb, 1, None), (tb, 0, tr), (None, 0, tr), (None, 1, tr)):
+        out = core.full((M, N), float("nan"), "bfloat16")
+        lib.call("kd_linear_bf16_bias", _r(tx), _r(tw), _r(bias), _r(res), act, _r(out))
+        want = y + b if bias is not None else y
+        want = (vogozen.gelu_tanh(want) if act else want) + (r if res is not None else 0)
+        _close(out.dataAsync(), want, 2.0 ** -8)
+    res32 = core.full((M, N), float("nan"), "float32")
+    lib.call("kd_linear_bf16", _r(tx), _r(tw), _r(Tensor(r)), 1, _r(res32))
+    _close(res32.dataAsync(), y + r, 0)
+
+
+@pytest.mark.gpu
 @pytest.mark.parametrize("epilogue", [2, 5])
 def test_gated_epilogues_of_pairs(backend, epilogue):
-    M, ff, K = 24800, 144, 200
+    M, ff, K = 24800, 144, 840
     assert _pair(M, 2 * ff, K)
     x, g, u = _bf((M, K), 5), _bf((ff, K), 6, 2 * K ** -0.5), _bf((ff, K), 7, K ** -0.5)
     out = core.full((M, ff), float("nan"), "bfloat16")
@@ -99,7 +117,7 @@ def test_gated_epilogues_of_pairs(backend, epilogue):
 @pytest.mark.gpu
 def test_heads_of_pairs(backend, oracle):
     """Query/key norm, rotation and cache rows: the fused epilogue against the linear and the kernel that does the same."""
-    B, S, Hq, Hkv, K, d, max_s = 96, 257, 2, 1, 72, 128, 264
+    B, S, Hq, Hkv, K, d, max_s = 96, 257, 2, 1, 776, 128, 264
     n = (Hq + 2 * Hkv) * d
     assert _pair(B * S, n, K, 1)
     x, w = _bf((B * S, K), 8), _bf((n, K), 9, K ** -0.5)
